@@ -513,8 +513,195 @@ size_t attention_smem_bytes(int BQ, int G, int hd, int hdv) {
     return floats * sizeof(float);
 }
 
+// ---- tiles of rows in 32 bits --------------------------------------------------------------------------------------
+// The same for float caches with heads of 64 or 128: a block takes up to 32 of a tile's query vectors (row, head) of one
+// kv head and walks their keys 64 at a time.  Scores and P V are register tiles (4 queries x 4 keys, 4 queries x 4
+// dimensions a thread, 16-byte shared loads), so the FFMA pipe and not the shared memory paces it; the kernel above spends a
+// shared load on every product (24 layers of a 389-token prompt at 14 / 2 heads of 64: 890 -> 62 us a layer).  Row maxima and sums are exchanged between the 16 threads that share a query row.
+constexpr int TQ = 32, TKEYS = 64, TP = TKEYS + 4;
+template <int HD> constexpr size_t tile_f32_smem() { return sizeof(float) * ((size_t)TQ * (HD + 4) + TKEYS * (HD + 4) + TKEYS * HD + TQ * TP); }
+
+template <int HD>
+__global__ void __launch_bounds__(128) paged_attention_tile_f32_kernel(AttnParams p, int chunks, int per) {
+    extern __shared__ __align__(16) float smem[];
+    constexpr int LD = HD + 4, ND = HD / 64;
+    float* Qs = smem;                        // [TQ][LD]
+    float* Ks = Qs + TQ * LD;                // [TKEYS][LD]
+    float* Vs = Ks + TKEYS * LD;             // [TKEYS][HD]
+    float* Ps = Vs + TKEYS * HD;             // [TQ][TP]
+    const int tile = gridDim.x - 1 - blockIdx.x;          // later tiles of a span have more keys: they start first
+    const int kvh = blockIdx.y / chunks, chunk = blockIdx.y % chunks;
+    const int G = p.Hq / p.Hkv;
+    const int span = p.tile_span[tile], q0 = p.tile_q0[tile];
+    const int row0 = p.span_row[span] + q0, pos0 = p.span_pos[span] + q0;
+    const int nrows = min(p.BQ, p.span_len[span] - q0);
+    const int v_lo = chunk * per, nv = min(per, nrows * G - v_lo);          // this block's vectors: v = row * G + head
+    if (nv <= 0) return;
+    const int* bt = p.block_table + (size_t)span * p.max_pages;
+    const float* q = (const float*)p.q;
+    const float* kc = (const float*)p.k_cache;
+    const float* vc = (const float*)p.v_cache;
+    const int r_lo = v_lo / G, r_hi = (v_lo + nv - 1) / G;
+    const LlbKeys keys = llb_keys(llb_first_visible(pos0 + r_lo, p.window), pos0 + r_hi + 1, p.keep);
+
+    const int tid = threadIdx.x, tq = tid >> 4, tl = tid & 15;
+    for (int i = tid; i < TQ * (HD / 4); i += 128) {
+        const int v = i / (HD / 4), d = (i % (HD / 4)) * 4;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (v < nv) {
+            const int r = (v_lo + v) / G, g = (v_lo + v) - r * G;
+            x = *reinterpret_cast<const float4*>(q + ((size_t)(row0 + r) * p.Hq + kvh * G + g) * HD + d);
+        }
+        *reinterpret_cast<float4*>(Qs + v * LD + d) = x;
+    }
+    int qpos[4];
+    float slope[4], m[4], l[4], o[4][4 * ND];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int v = v_lo + min(tq + 8 * i, nv - 1), r = v / G;
+        qpos[i] = pos0 + r;
+        slope[i] = p.slopes ? p.slopes[kvh * G + v - r * G] : 0.0f;
+        m[i] = -INFINITY;
+        l[i] = 0.0f;
+#pragma unroll
+        for (int d = 0; d < 4 * ND; ++d) o[i][d] = 0.0f;
+    }
+    for (int kb = 0; kb < keys.count; kb += TKEYS) {
+        __syncthreads();          // the last tile has been read (and the queries are there)
+        for (int i = tid; i < TKEYS * (HD / 4); i += 128) {
+            const int j = i / (HD / 4), d = (i % (HD / 4)) * 4;
+            float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f), v4 = k4;
+            if (kb + j < keys.count) {
+                const int kpos = keys.pos(kb + j);
+                const size_t slot = (size_t)bt[kpos / p.page_size] * p.page_size + (kpos % p.page_size);
+                k4 = *reinterpret_cast<const float4*>(kc + key_row(p, slot, kvh) + d);
+                v4 = *reinterpret_cast<const float4*>(vc + value_row(p, slot, kvh) + d);
+            }
+            *reinterpret_cast<float4*>(Ks + j * LD + d) = k4;
+            *reinterpret_cast<float4*>(Vs + j * HD + d) = v4;
+        }
+        __syncthreads();
+        float s[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
+#pragma unroll 4
+        for (int d = 0; d < HD; d += 4) {
+            float4 a[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(Qs + (tq + 8 * i) * LD + d);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 b = *reinterpret_cast<const float4*>(Ks + (tl + 16 * j) * LD + d);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    s[i][j] = fmaf(a[i].x, b.x, s[i][j]);
+                    s[i][j] = fmaf(a[i].y, b.y, s[i][j]);
+                    s[i][j] = fmaf(a[i].z, b.z, s[i][j]);
+                    s[i][j] = fmaf(a[i].w, b.w, s[i][j]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float top = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int n = kb + tl + 16 * j, kpos = keys.pos(n);
+                const bool visible = n < keys.count && kpos <= qpos[i] && (kpos >= llb_first_visible(qpos[i], p.window) || kpos < p.keep);
+                float x = s[i][j] * p.scale;
+                if (p.softcap > 0.0f) x = p.softcap * tanhf(x / p.softcap);
+                x -= slope[i] * (float)(qpos[i] - kpos);
+                s[i][j] = visible ? x : -INFINITY;
+                top = fmaxf(top, s[i][j]);
+            }
+#pragma unroll
+            for (int w = 8; w > 0; w >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, w));
+            const float m_new = fmaxf(m[i], top);
+            const float base = m_new == -INFINITY ? 0.0f : m_new;          // nothing visible yet: every weight is zero
+            const float corr = expf(m[i] - base);
+            float sum = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float e = expf(s[i][j] - base);
+                sum += e;
+                Ps[(tq + 8 * i) * TP + tl + 16 * j] = e;
+            }
+#pragma unroll
+            for (int w = 8; w > 0; w >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+            l[i] = l[i] * corr + sum;
+            m[i] = m_new;
+#pragma unroll
+            for (int d = 0; d < 4 * ND; ++d) o[i][d] *= corr;
+        }
+        __syncwarp();          // a query row's weights are written and read by the same half warp
+#pragma unroll 4
+        for (int j = 0; j < TKEYS; j += 4) {
+            float4 w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(Ps + (tq + 8 * i) * TP + j);
+#pragma unroll
+            for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+                for (int n = 0; n < ND; ++n) {
+                    const float4 v4 = *reinterpret_cast<const float4*>(Vs + (j + jj) * HD + n * 64 + tl * 4);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float e = jj == 0 ? w[i].x : jj == 1 ? w[i].y : jj == 2 ? w[i].z : w[i].w;
+                        o[i][4 * n] = fmaf(e, v4.x, o[i][4 * n]);
+                        o[i][4 * n + 1] = fmaf(e, v4.y, o[i][4 * n + 1]);
+                        o[i][4 * n + 2] = fmaf(e, v4.z, o[i][4 * n + 2]);
+                        o[i][4 * n + 3] = fmaf(e, v4.w, o[i][4 * n + 3]);
+                    }
+                }
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int v = tq + 8 * i;
+        if (v >= nv) continue;
+        const int r = (v_lo + v) / G, g = v_lo + v - r * G;
+        float den = l[i];
+        if (p.sinks) den += expf(p.sinks[kvh * G + g] - m[i]);
+        const float inv = 1.0f / den;
+#pragma unroll
+        for (int n = 0; n < ND; ++n)
+            *reinterpret_cast<float4*>((float*)p.out + ((size_t)(row0 + r) * p.Hq + kvh * G + g) * HD + n * 64 + tl * 4) =
+                make_float4(o[i][4 * n] * inv, o[i][4 * n + 1] * inv, o[i][4 * n + 2] * inv, o[i][4 * n + 3] * inv);
+    }
+}
+
+// Whether a call is one for the kernel above: floats, ordinary value rows, addresses in 16-byte steps.
+template <typename T>
+bool tile_f32_eligible(const AttnParams& p) {
+    return sizeof(T) == 4 && p.nsplit == 1 && (p.hd == 64 || p.hd == 128) && p.hdv == p.hd && p.vrow % 4 == 0 && !p.v_shared &&
+           (((uintptr_t)p.q | (uintptr_t)p.k_cache | (uintptr_t)p.v_cache | (uintptr_t)p.out) % 16) == 0;
+}
+
+template <int HD>
+int launch_tile_f32(const AttnParams& p, int num_tiles, cudaStream_t stream) {
+    static bool configured[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(paged_attention_tile_f32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)tile_f32_smem<HD>());
+        if (e != cudaSuccess) return llb_fail("attention: cannot opt in to shared memory: %s", cudaGetErrorString(e));
+        if (dev >= 0 && dev < 64) configured[dev] = true;
+    }
+    const int vectors = p.BQ * (p.Hq / p.Hkv), chunks = llb_ceil_div(vectors, TQ);
+    LLB_REQUIRE((long long)p.Hkv * chunks <= 65535, "attention: too many heads for tiles of %d rows", p.BQ);
+    paged_attention_tile_f32_kernel<HD><<<dim3(num_tiles, p.Hkv * chunks), 128, tile_f32_smem<HD>(), stream>>>(
+        p, chunks, llb_ceil_div(vectors, chunks));
+    return llb_check_launch("paged_attention_tile_f32");
+}
+
 template <typename T>
 int launch_attention(AttnParams p, int num_tiles, cudaStream_t stream) {
+    if (tile_f32_eligible<T>(p) && !decode_eligible<T>(p))
+        return p.hd == 64 ? launch_tile_f32<64>(p, num_tiles, stream) : launch_tile_f32<128>(p, num_tiles, stream);
     // many heads over wide rows: as many blocks share a kv head as it takes for one block's heads to fit
     const int heads = p.Hq / p.Hkv;
     while (p.share < heads && attention_smem_bytes(p.BQ, heads / p.share, p.hd, p.hdv) > 200 * 1024)

@@ -1,0 +1,47 @@
+"""The register-tiled 32-bit kernels (contraction and paged attention) at the edges of their tiles, against float64."""
+import pytest
+import torch
+
+from tests.test_kernels_gpu import attention_reference, dev, gemm_reference, ops, paged_setup, rnd, tiles_for  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+# rows around the heights of 16, 32 and 64; columns around 64 (odd ones too); K from one 16-byte step over ends of a slice
+# of 32 to sums that are cut among the blocks of a cluster (few tiles over a long K)
+SHAPES = [(4, 66, 36), (5, 66, 36), (9, 64, 4), (16, 63, 28), (17, 65, 32), (32, 2, 36), (33, 129, 100), (64, 128, 896), (65, 66, 4864), (389, 896, 1536)]
+
+
+@pytest.mark.parametrize("M,N,K", SHAPES)
+@pytest.mark.parametrize("epi", [0, 1, 2, 3])
+def test_float_contraction(ops, M, N, K, epi):  # noqa: F811
+    if epi == 3 and N % 2:
+        N += 1
+    a, w, bias = rnd((M, K), torch.float32, 1), rnd((N, K), torch.float32, 2, 0.2), rnd((N,), torch.float32, 3)
+    residual = rnd((M, N), torch.float32, 4)
+    out = None if epi == 2 else torch.full((M, N // 2 if epi == 3 else N), float("nan"), device=dev())
+    want = gemm_reference(a, w, bias, epi, residual)
+    ops.gemm_simt(a, w, bias, epi, out, residual if epi == 2 else None)
+    got = (residual if epi == 2 else out).double().cpu()
+    # the rounding of K products and sums, each at most 2^-24 of the sum of magnitudes; a gated pair multiplies two of them
+    size = a.abs().double().cpu() @ w.abs().double().cpu().t() + bias.abs().double().cpu() + 4.0
+    bound = (K + 4) * 2.0 ** -24 * size
+    if epi == 3:
+        size, bound = size[:, 0::2] + size[:, 1::2], bound[:, 0::2] + bound[:, 1::2]
+        bound = bound * size * 1.2 + 1e-6 * (1.0 + want.abs())
+    assert bool(((got - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("Hq,Hkv,hd", [(14, 2, 64), (3, 3, 128), (9, 1, 64), (12, 2, 128)])
+@pytest.mark.parametrize("window", [None, 33])
+@pytest.mark.parametrize("bq", [16, 5])
+def test_float_attention(ops, Hq, Hkv, hd, window, bq):  # noqa: F811
+    lens, starts = [1, 16, 67, 33], [0, 63, 0, 130]
+    s = paged_setup(torch.float32, lens, starts, Hq, Hkv, hd, 16, 11)
+    ts, tq, nt = tiles_for(lens, bq)
+    out = torch.full((s["rows"], Hq * hd), float("nan"), device=dev())
+    ops.paged_attention_simt(s["q"], s["kc"], s["vc"], out, ts, tq, nt, s["span_row"], s["span_len"], s["span_pos"], s["bt"],
+                             s["max_pages"], 16, Hq, Hkv, hd, window or 0, hd ** -0.5, bq)
+    ref = attention_reference(s["full"], lens, starts, hd, window).reshape(s["rows"], Hq * hd)
+    got = out.cpu()
+    assert not torch.isnan(got).any()
+    assert torch.allclose(got, ref, atol=2e-5, rtol=2e-5), f"max diff {float((got - ref).abs().max())}"
