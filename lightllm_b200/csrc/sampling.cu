@@ -300,6 +300,135 @@ __device__ __forceinline__ float cluster_max(cg::cluster_group& cl, ClusterExcha
     return best;
 }
 
+// The exact threshold of a filter, found in five meetings of the cluster instead of one for each of 32 bits (a row with top-k and
+// top-p took 190 us that way at a vocabulary of 151,936): the values are counted (or their masses added) by bin, the bin in
+// which the wanted count or mass is reached is found bin by bin, its few values are gathered in one block, and each of them is
+// compared with all the others.  Masses are added as whole numbers of 2^-44 in three parts of 15 bits (32-bit atomics are the
+// hardware's own, and the 53,000 values that a block holds at most leave them room), so no sum depends on the order of the atomics.
+// A bin with more than BIN_LIST values (equal or nearly equal ones) is left to the search by bits, as are rows with values that are
+// not numbers or with an infinite maximum.  64 rows of 151,936 under mixed parameters: 228 -> 80 us; 8 rows of 32,017: 134 -> 34.
+constexpr int BINS = 1024;            // CL slices of 128
+constexpr int BIN_LIST = 1024;
+constexpr int BIN_SLICE = BINS / CL;
+struct Threshold {
+    unsigned hist[3][BINS];                       // counts or masses: bits 0-14, 15-29 and 30-44 of every value added up
+    unsigned long long slice_sum[BIN_SLICE];      // this block's slice of the bins over all blocks, running sums
+    unsigned long long total;                     // of the slice
+    unsigned long long before;                    // by the block that holds the bin: what lies in higher bins
+    int bin, members;                             // ... the bin and how many values it has; 0 members: not to be done here
+    int listed;
+    float value;                                  // the threshold
+    float list[BIN_LIST];
+};
+// bin_of(x): the bin of a value, higher values in lower bins, -1 for values that are not counted (below all bins); weight_of(x): its count
+// or mass.  `need_of(total)` is what the values at or above the threshold must reach.  Returns false (in all blocks) if the
+// threshold was not found; else *value is the largest value whose weight and that of all larger ones reach the need.
+template <typename BinOf, typename WeightOf, typename NeedOf>
+__device__ bool cluster_threshold(cg::cluster_group& cl, Threshold* th, const float* mine, int n, BinOf bin_of, WeightOf weight_of,
+                                  NeedOf need_of, float* value) {
+    const int tid = threadIdx.x, rank = (int)cl.block_rank();
+    for (int i = tid; i < 3 * BINS; i += CL_THREADS) (&th->hist[0][0])[i] = 0u;
+    if (tid == 0) { th->listed = 0; th->members = 0; th->bin = -1; }
+    __syncthreads();
+    auto add = [&](int b, unsigned long long w) {
+        const unsigned lo = (unsigned)w & 0x7fffu, mid = (unsigned)(w >> 15) & 0x7fffu, hi = (unsigned)(w >> 30);
+        if (lo) atomicAdd(&th->hist[0][b], lo);
+        if (mid) atomicAdd(&th->hist[1][b], mid);
+        if (hi) atomicAdd(&th->hist[2][b], hi);
+    };
+    unsigned long long least = 0ull;          // (the last bin is where most values of a long row may be: added up in the thread)
+    for (int i = tid; i < n; i += CL_THREADS) {
+        const float x = mine[i];
+        const int b = bin_of(x);
+        if (b == BINS - 1) least += weight_of(x);
+        else if (b >= 0) add(b, weight_of(x));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) least += __shfl_xor_sync(0xffffffffu, least, o);
+    if ((tid & 31) == 0) {
+        atomicAdd(&th->hist[0][BINS - 1], (unsigned)least & 0x7fffu);
+        atomicAdd(&th->hist[1][BINS - 1], (unsigned)(least >> 15) & 0x7fffu);
+        atomicAdd(&th->hist[2][BINS - 1], (unsigned)(least >> 30));
+    }
+    cl.sync();
+    // this block's slice of the bins, over all blocks, as running sums
+    if (tid < BIN_SLICE) {
+        unsigned long long sum = 0ull;
+#pragma unroll
+        for (int b = 0; b < CL; ++b) {
+            const Threshold* o = cl.map_shared_rank(th, b);
+            const int at = rank * BIN_SLICE + tid;
+            sum += o->hist[0][at] + ((unsigned long long)o->hist[1][at] << 15) + ((unsigned long long)o->hist[2][at] << 30);
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long up = __shfl_up_sync(0xffffffffu, sum, o);
+            if ((tid & 31) >= o) sum += up;
+        }
+        th->slice_sum[tid] = sum;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        unsigned long long sum = 0ull;
+        for (int w = 31; w < BIN_SLICE; w += 32) sum += th->slice_sum[w];
+        th->total = sum;
+    }
+    cl.sync();
+    unsigned long long below = 0ull, total = 0ull;          // weight of the slices before this one, and of all
+#pragma unroll
+    for (int b = 0; b < CL; ++b) {
+        const unsigned long long t = cl.map_shared_rank(th, b)->total;
+        if (b < rank) below += t;
+        total += t;
+    }
+    const unsigned long long need = need_of(total);
+    if (total < need || need == 0ull) return false;          // the same in every block
+    if (tid < BIN_SLICE) {
+        unsigned long long upto = below, own = th->slice_sum[tid];
+        for (int w = 31; w < tid - (tid & 31); w += 32) upto += th->slice_sum[w];
+        const unsigned long long prev = (tid & 31) ? th->slice_sum[tid - 1] : 0ull;
+        if (upto + prev < need && upto + own >= need) {          // exactly one thread of the cluster
+            th->bin = rank * BIN_SLICE + tid;
+            th->before = upto + prev;
+        }
+    }
+    cl.sync();
+    int owner = 0;
+#pragma unroll
+    for (int b = 0; b < CL; ++b)
+        if (cl.map_shared_rank(th, b)->bin >= 0) owner = b;
+    Threshold* at = cl.map_shared_rank(th, owner);
+    const int bin = at->bin;
+    for (int i = tid; i < n; i += CL_THREADS) {
+        const float x = mine[i];
+        if (bin_of(x) == bin) {
+            const int k = atomicAdd(&at->listed, 1);
+            if (k < BIN_LIST) at->list[k] = x;
+        }
+    }
+    cl.sync();
+    if (rank == owner) {
+        const int m = th->listed;
+        if (m <= BIN_LIST) {
+            for (int i = tid; i < m; i += CL_THREADS) {
+                const float x = th->list[i];
+                unsigned long long above = th->before, with = th->before;
+                for (int j = 0; j < m; ++j) {
+                    const float y = th->list[j];
+                    if (y > x) above += weight_of(y);
+                    if (y >= x) with += weight_of(y);
+                }
+                if (above < need && with >= need) { th->value = x; th->members = m; }      // equal values write the same
+            }
+        }
+    }
+    cl.sync();
+    const bool found = at->members > 0;
+    *value = at->value;
+    cl.sync();          // (the next search clears what is read here)
+    return found;
+}
+
 // First index of the largest value of the whole row (0 if nothing lies above -inf), the same in every block.
 __device__ int cluster_argmax(cg::cluster_group& cl, ClusterExchange* xc, const float* x, int begin, int n, float* shf,
                               int* shi) {
@@ -333,6 +462,7 @@ __global__ void __launch_bounds__(CL_THREADS) sample_cluster_kernel(const float*
                                                                     const float* __restrict__ uniform,
                                                                     int* __restrict__ out) {
     extern __shared__ float mine[];            // this block's `part` elements of the row
+    __shared__ Threshold th;
     __shared__ float shf[33];
     __shared__ int shi[33];
     __shared__ float chunk_sum[CL_THREADS];
@@ -358,12 +488,15 @@ __global__ void __launch_bounds__(CL_THREADS) sample_cluster_kernel(const float*
     const float tp = top_p ? top_p[r] : 1.0f;
     const float mp = min_p ? min_p[r] : 0.0f;
 
-    float mx = -INFINITY;
+    float mx = -INFINITY, odd = 0.0f;          // odd: how many values are not numbers
     for (int i = threadIdx.x; i < n; i += CL_THREADS) {
         const float v = x[begin + i] * inv_temp;
         mine[i] = v;
         mx = fmaxf(mx, v);
+        if (!(v == v)) odd += 1.0f;
     }
+    const bool filters = (k > 0 && k < V) || tp < 1.0f;
+    if (filters) odd = cluster_sum(cl, &xc, block_sum(odd, shf));
     mx = cluster_max(cl, &xc, block_max(mx, shf));
     if (mx == -INFINITY || !(mx == mx)) {        // every logit is -inf, or NaN: fall back to argmax
         const int idx = cluster_argmax(cl, &xc, x, begin, n, shf, shi);
@@ -372,9 +505,19 @@ __global__ void __launch_bounds__(CL_THREADS) sample_cluster_kernel(const float*
         return;
     }
 
-    // top-k: key of the k-th largest scaled logit (largest K with count(key >= K) >= k).
+    // top-k: key of the k-th largest scaled logit (largest K with count(key >= K) >= k).  By bins of 1/32 below the maximum where
+    // the row is one of numbers.
     unsigned key_k = 0u;
-    if (k > 0 && k < V) {
+    const bool numbers = odd == 0.0f && mx < INFINITY;
+    float value = 0.0f;
+    bool found = false;
+    if (k > 0 && k < V && numbers)
+        found = cluster_threshold(
+            cl, &th, mine, n, [mx](float v) { const float d = (mx - v) * 32.0f; return d < (float)BINS ? (int)d : -1; },
+            [](float) { return 1ull; }, [k](unsigned long long) { return (unsigned long long)k; }, &value);
+    if (found) {
+        key_k = ordered_key(value);
+    } else if (k > 0 && k < V) {
         for (int bit = 31; bit >= 0; --bit) {
             const unsigned cand = key_k | (1u << bit);
             float cnt = 0.0f;
@@ -395,7 +538,16 @@ __global__ void __launch_bounds__(CL_THREADS) sample_cluster_kernel(const float*
 
     // top-p: largest threshold on e whose kept mass still reaches p * z.
     unsigned key_p = 0u;
-    if (tp < 1.0f) {
+    found = false;
+    if (tp < 1.0f && tp > 0.0f && numbers)          // by bins of 1/32 of an octave below one (what is below 2^-32 shares the last)
+        found = cluster_threshold(
+            cl, &th, mine, n,
+            [](float e) { return e > 0.0f ? min(BINS - 1, (int)((0x3f800000u - __float_as_uint(e)) >> 18)) : -1; },
+            [](float e) { return (unsigned long long)(e * 17592186044416.0f); },
+            [tp](unsigned long long total) { return (unsigned long long)((double)tp * (double)total); }, &value);
+    if (found) {
+        key_p = ordered_key(value);
+    } else if (tp < 1.0f) {
         const float need = tp * z;
         for (int bit = 31; bit >= 0; --bit) {
             const unsigned cand = key_p | (1u << bit);
@@ -522,7 +674,7 @@ LLB_EXPORT int llb_sample(const float* logits, int R, int V, long long stride, c
     // long rows: a cluster of blocks per row, each with its part of the row in shared memory
     const int part = llb_ceil_div(V, CL);
     const size_t smem = (size_t)part * sizeof(float);
-    if (V >= 8192 && smem <= 216 * 1024 && R <= 65535) {
+    if (V >= 8192 && smem + sizeof(Threshold) + 4096 <= 227 * 1024 && R <= 65535) {
         static size_t configured = 0;
         if (smem > configured) {
             cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
