@@ -1460,6 +1460,7 @@ def decode_layers(descriptors: torch.Tensor, num_layers: int, residual: torch.Te
                   timeline_block: int = 0) -> None:
     """All layers of a decode step (one token per request, at most 64) in one persistent kernel, in place on the
     float32 ``residual`` [M, D].  ``block_tables`` / ``slot_mappings``: one int32 tensor per cache group (up to 4).
+    ``nsplit``: the most pieces that a request's keys are cut into (the kernel cuts them so that all pieces are of one length).
     ``timeline`` (int64, 2 * (2 + 64 * layers) words) receives the milestones of block ``timeline_block`` as (label, SM cycle) pairs."""
     M = residual.shape[0]
     if residual.dtype != torch.float32 or tuple(residual.shape) != (M, D):

@@ -74,28 +74,19 @@ class Segment:
         self.begin, self.end = begin, end
         (self.D, self.Hq, self.Hkv, self.hd, self.I, (self.rotary_dim, self.interleaved, _), self.scale) = sizes
         self.position = position
-        self.windows = [d["window"] for d in layers]
         self.descriptors = ops.decode_layers_descriptors(layers, self.D, self.Hq, self.Hkv, self.hd, self.I, device)
         self.keep = layers                   # the descriptors hold addresses of these tensors
         self.counters = ops.decode_layers_counters(device)
         self.scratch: Optional[torch.Tensor] = None
 
-    def splits(self, ctx) -> int:
-        """Pieces of a request's keys: enough items for all multiprocessors, none shorter than 128 keys."""
-        bound = ctx.max_pages * ctx.page_size              # the same for every step of this shape
-        span = max(bound if w == 0 else min(bound, w) for w in self.windows)
-        want = L.num_sms(ctx.device) // max(1, ctx.T * self.Hkv)
-        return max(1, min(ops.MAX_FUSED_SPLITS, want, -(-span // 128)))
-
     def run(self, residual: torch.Tensor, ctx) -> None:
-        nsplit = self.splits(ctx)
         need = ops.decode_layers_scratch_floats(MAX_ROWS, self.Hq, self.Hkv, self.hd, self.I, ops.MAX_FUSED_SPLITS)
         if self.scratch is None or self.scratch.numel() < need:
             self.scratch = torch.empty(need, dtype=torch.float32, device=residual.device)
         table = self.position.step_table(ctx) if self.rotary_dim else None
         ops.decode_layers(self.descriptors, self.end - self.begin, residual, self.D, self.Hq, self.Hkv, self.hd, self.I,
                           self.rotary_dim, self.interleaved, self.scale, table, ctx.span_pos, ctx.block_tables,
-                          ctx.slot_mapping, ctx.max_pages, ctx.page_size, nsplit, self.scratch, self.counters)
+                          ctx.slot_mapping, ctx.max_pages, ctx.page_size, ops.MAX_FUSED_SPLITS, self.scratch, self.counters)
 
 
 class FusedDecode:
