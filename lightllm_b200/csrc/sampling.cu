@@ -412,13 +412,15 @@ __device__ bool cluster_threshold(cg::cluster_group& cl, Threshold* th, const fl
         if (m <= BIN_LIST) {
             for (int i = tid; i < m; i += CL_THREADS) {
                 const float x = th->list[i];
+                const unsigned kx = ordered_key(x);          // (not the floats: a zero's sign decides what the caller keeps)
                 unsigned long long above = th->before, with = th->before;
                 for (int j = 0; j < m; ++j) {
                     const float y = th->list[j];
-                    if (y > x) above += weight_of(y);
-                    if (y >= x) with += weight_of(y);
+                    const unsigned ky = ordered_key(y);
+                    if (ky > kx) above += weight_of(y);
+                    if (ky >= kx) with += weight_of(y);
                 }
-                if (above < need && with >= need) { th->value = x; th->members = m; }      // equal values write the same
+                if (above < need && with >= need) { th->value = x; th->members = m; }      // equal keys: the same bits
             }
         }
     }

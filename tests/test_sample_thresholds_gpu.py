@@ -61,3 +61,26 @@ def test_rows_that_are_not_numbers(ops):  # noqa: F811
     f = lambda v, dt=torch.float32: torch.full((3,), v, dtype=dt, device=dev())  # noqa: E731
     ops.sample(x.to(dev()), f(1.0), f(50, torch.int32), f(0.9), f(0.0), f(0.4), out)
     assert all(0 <= t < V for t in out.tolist())
+
+
+@pytest.mark.parametrize("V", [2000, 8192, 151936])          # one block a row; a cluster of blocks
+def test_zeros_of_both_signs(ops, V):  # noqa: F811
+    """+0 lies above -0 in the order that top-k goes by: a k-th place among zeros keeps the same tokens at every launch."""
+    x = torch.full((V,), -30.0)
+    plus, minus = [200, 901, 1500], [17, 300, 1999]
+    x[100], x[plus], x[minus] = 1.0, 0.0, -0.0
+    us = [(i + 0.5) / 40 for i in range(40)]
+    many = [(k, u) for k in (2, 3, 4, 5, 6, 7) for u in us]
+    f = lambda v, dt=torch.float32: torch.tensor(v, dtype=dt, device=dev())  # noqa: E731
+    rows_ = x[None].repeat(len(many), 1).contiguous().to(dev())
+    out = torch.empty(len(many), dtype=torch.int32, device=dev())
+    args = f([1.0] * len(many)), f([m[0] for m in many], torch.int32), f([1.0] * len(many)), f([0.0] * len(many)), f([m[1] for m in many])
+    for _ in range(20):
+        ops.sample(rows_, *args, out)
+        got = out.tolist()
+        for k in (2, 3, 4, 5, 6, 7):
+            kept = sorted([100] + plus + (minus if k > 1 + len(plus) else []))
+            mass = np.cumsum([np.e if i == 100 else 1.0 for i in kept])
+            want = [kept[int(np.searchsorted(mass, u * mass[-1]))] for u in us]
+            assert got[: len(us)] == want, k
+            got = got[len(us):]
