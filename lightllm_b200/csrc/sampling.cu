@@ -8,8 +8,8 @@
 // renormalises (:198-243); min-p drops probabilities below min_p * max and renormalises
 // (:248-278); the draw is the first index whose cumulative mass reaches the uniform number,
 // skipping entries without mass (:284-334).  The reference sorts on the CPU; here each filter
-// is a threshold on the value found by a bitwise search over the float's ordered bit pattern
-// (32 counting passes), so a tie at the top-p boundary keeps all tied tokens where the
+// is a threshold on the value, found over the float's ordered bit pattern (in short rows bit by
+// bit, in long ones by bins of values), so a tie at the top-p boundary keeps all tied tokens where the
 // reference's sort keeps an unspecified subset.  The uniform number comes from the caller
 // (one per row), so the random stream belongs to the request, not to the kernel.
 #include "common.cuh"
@@ -28,6 +28,8 @@ __device__ __forceinline__ unsigned ordered_key(float f) {
     const unsigned u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
+
+__device__ __forceinline__ float key_value(unsigned key) { return __uint_as_float((key & 0x80000000u) ? key ^ 0x80000000u : ~key); }
 
 __device__ float block_sum(float v, float* sh) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -274,19 +276,6 @@ struct ClusterExchange {
     int turn;
 };
 
-__device__ __forceinline__ float cluster_sum(cg::cluster_group& cl, ClusterExchange* xc, float block_value) {
-    const int t = xc->turn;
-    if (threadIdx.x == 0) xc->f[t] = block_value;
-    cl.sync();
-    float total = 0.0f;
-#pragma unroll
-    for (int b = 0; b < CL; ++b) total += cl.map_shared_rank(xc, b)->f[t];
-    __syncthreads();                       // everyone has read `turn` before it moves
-    if (threadIdx.x == 0) xc->turn = t ^ 1;
-    __syncthreads();
-    return total;
-}
-
 __device__ __forceinline__ float cluster_max(cg::cluster_group& cl, ClusterExchange* xc, float block_value) {
     const int t = xc->turn;
     if (threadIdx.x == 0) xc->f[t] = block_value;
@@ -300,135 +289,275 @@ __device__ __forceinline__ float cluster_max(cg::cluster_group& cl, ClusterExcha
     return best;
 }
 
-// The exact threshold of a filter, found in five meetings of the cluster instead of one for each of 32 bits (a row with top-k and
-// top-p took 190 us that way at a vocabulary of 151,936): the values are counted (or their masses added) by bin, the bin in
-// which the wanted count or mass is reached is found bin by bin, its few values are gathered in one block, and each of them is
-// compared with all the others.  Masses are added as whole numbers of 2^-44 in three parts of 15 bits (32-bit atomics are the
-// hardware's own, and the 53,000 values that a block holds at most leave them room), so no sum depends on the order of the atomics.
-// A bin with more than BIN_LIST values (equal or nearly equal ones) is left to the search by bits, as are rows with values that are
-// not numbers or with an infinite maximum.  64 rows of 151,936 under mixed parameters: 228 -> 80 us; 8 rows of 32,017: 134 -> 34.
-constexpr int BINS = 1024;            // CL slices of 128
-constexpr int BIN_LIST = 1024;
-constexpr int BIN_SLICE = BINS / CL;
-struct Threshold {
-    unsigned hist[3][BINS];                       // counts or masses: bits 0-14, 15-29 and 30-44 of every value added up
-    unsigned long long slice_sum[BIN_SLICE];      // this block's slice of the bins over all blocks, running sums
-    unsigned long long total;                     // of the slice
-    unsigned long long before;                    // by the block that holds the bin: what lies in higher bins
-    int bin, members;                             // ... the bin and how many values it has; 0 members: not to be done here
-    int listed;
-    float value;                                  // the threshold
-    float list[BIN_LIST];
+// The maxima of a and b over the cluster in one meeting.
+__device__ __forceinline__ void cluster_max2(cg::cluster_group& cl, ClusterExchange* xc, float& a, float& b, float* sh) {
+    static_assert(CL_THREADS == 512, "sixteen warps, two numbers each");
+    const int t = xc->turn, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    a = llb_warp_max(a);
+    b = llb_warp_max(b);
+    if (lane == 0) {
+        sh[w] = a;
+        sh[16 + w] = b;
+    }
+    __syncthreads();
+    if (w == 0) {
+        float v = sh[lane];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if (lane == 0) xc->f[t] = v;
+        if (lane == 16) xc->i[t] = __float_as_int(v);
+    }
+    cl.sync();
+    a = b = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < CL; ++r) {
+        const ClusterExchange* o = cl.map_shared_rank(xc, r);
+        a = fmaxf(a, o->f[t]);
+        b = fmaxf(b, __int_as_float(o->i[t]));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) xc->turn = t ^ 1;
+    __syncthreads();
+}
+
+// The threshold of a filter over a row that lies in its cluster's shared memory: the largest key for which the weight of all values
+// with that key or a larger one reaches what is needed (a search bit by bit finds the same in 32 meetings of the cluster).  The weights
+// are counted by bin, every block adds up all blocks' bins and finds the one in which the need is reached, and the values of
+// that bin either go to a list of every block, where each is compared with all the others, or, where they are more than the list holds,
+// are binned anew over the keys that they span: two meetings a level, one or two levels for most rows (ties end at once, their keys
+// span one value).  A mass is added as a whole number of 2^-44 in three parts of 15 bits (32-bit atomics are the hardware's
+// own, and the 56,000 values that a block holds at most leave them room), so no sum depends on the order of the atomics.
+// What bounds it: the walks over shared memory (some 6 us a search at 151,936 values) and the meetings.  What falls into the last bin,
+// where most of a wide row lies, is added up in registers.  (Adding up in the warp what shares a bin before the atomic helped rows
+// of two values only, and cost all others a tenth.)  Three blocks fit a multiprocessor's registers at 40 a thread.
+// 64 rows of 151,936, us, by bits -> this: top-k 40 256 -> 75, top-k 20 and top-p 0.95 435 -> 89, top-p 0.9 of normal logits of
+// deviation 3 / 1 / 0.02: 221 / 228 / 229 -> 92 / 136 / 129, of equal ones 230 -> 126; one row 90 -> 28, 146 -> 33, 79 -> 40.
+constexpr int BINS = 256;
+constexpr int BIN_LIST = CL_THREADS / 4;      // four threads compare a member
+struct ThresholdList {
+    unsigned key[BIN_LIST];
+    unsigned long long weight[BIN_LIST];
 };
-// bin_of(x): the bin of a value, higher values in lower bins, -1 for values that are not counted (below all bins); weight_of(x): its count
-// or mass.  `need_of(total)` is what the values at or above the threshold must reach.  Returns false (in all blocks) if the
-// threshold was not found; else *value is the largest value whose weight and that of all larger ones reach the need.
-template <typename BinOf, typename WeightOf, typename NeedOf>
-__device__ bool cluster_threshold(cg::cluster_group& cl, Threshold* th, const float* mine, int n, BinOf bin_of, WeightOf weight_of,
-                                  NeedOf need_of, float* value) {
-    const int tid = threadIdx.x, rank = (int)cl.block_rank();
-    for (int i = tid; i < 3 * BINS; i += CL_THREADS) (&th->hist[0][0])[i] = 0u;
-    if (tid == 0) { th->listed = 0; th->members = 0; th->bin = -1; }
-    __syncthreads();
-    auto add = [&](int b, unsigned long long w) {
-        const unsigned lo = (unsigned)w & 0x7fffu, mid = (unsigned)(w >> 15) & 0x7fffu, hi = (unsigned)(w >> 30);
-        if (lo) atomicAdd(&th->hist[0][b], lo);
-        if (mid) atomicAdd(&th->hist[1][b], mid);
-        if (hi) atomicAdd(&th->hist[2][b], hi);
+struct Threshold {
+    unsigned hist[3][BINS];                   // counts or masses: bits 0-14, 15-29 and 30-44 of every value added up
+    unsigned long long warp_total[BINS / 32];
+    unsigned long long before, upto;          // what lies above the chosen bin, and with it
+    int bin;
+    unsigned value;                           // the threshold's key
+    unsigned long long reached;               // the weight of the threshold's and all larger values
+    float top, low;                           // of the whole row, kept here over the search by rank (registers are what limits blocks)
+    // This block's values in the bin span these keys, and block 0's count of the list.  Two slots in turn for each search: a slot is set
+    // anew two levels later, when everyone has met once more since its last reader; the second search's first one is set at the
+    // kernel's start.  For the same reason each search has a list of its own: blocks write into one another's, and some are at the
+    // second search while others still compare the first one's list.
+    unsigned key_lo[4], key_hi[4];
+    int listed[4];
+    __device__ void start(int slot) {
+        key_lo[slot] = 0xffffffffu;
+        key_hi[slot] = 0u;
+        listed[slot] = 0;
+    }
+    ThresholdList by_count;
+    union {
+        ThresholdList by_mass;
+        float chunk_sum[CL_THREADS];          // of the draw
     };
-    unsigned long long least = 0ull;          // (the last bin is where most values of a long row may be: added up in the thread)
-    for (int i = tid; i < n; i += CL_THREADS) {
-        const float x = mine[i];
-        const int b = bin_of(x);
-        if (b == BINS - 1) least += weight_of(x);
-        else if (b >= 0) add(b, weight_of(x));
-    }
+};
+__device__ __forceinline__ unsigned long long mass_of(float e) { return (unsigned long long)(e * 17592186044416.0f); }
+
+__device__ __forceinline__ void add_mass(unsigned (*hist)[BINS], int b, unsigned long long w) {
+    const unsigned lo = (unsigned)w & 0x7fffu, mid = (unsigned)(w >> 15) & 0x7fffu, hi = (unsigned)(w >> 30);
+    if (lo) atomicAdd(&hist[0][b], lo);
+    if (mid) atomicAdd(&hist[1][b], mid);
+    if (hi) atomicAdd(&hist[2][b], hi);
+}
+
+// Of counts (MASS false): `share` is how many values; with `scale` > 0 the first bins are 1 / scale wide below `top` (rows of
+// numbers), else they are steps of 2^24 keys.  Of masses: `share` of the whole mass; the values that are not zero take part,
+// `top` is the smallest of them (or zero); with `few` they are known to fit in the list, which saves the bins.
+template <bool MASS>
+__device__ __forceinline__ unsigned cluster_threshold(Threshold* th, const float* mine, int n, float top, float scale, float share, bool few) {
+    cg::cluster_group cl = cg::this_cluster();
+    constexpr int UNROLL = 4, PARTS = MASS ? 3 : 1;
+    const int tid = threadIdx.x, lane = tid & 31;
+    bool linear = !MASS && scale > 0.0f;
+    // the keys in play lie up to `reach` below `hi` (the largest mass is one), and the bins are made for a span of them: masses below
+    // 2^-20 share the last bin (most values of a wide row are there, and few sums need them)
+    unsigned hi = MASS ? ordered_key(1.0f) : 0xffffffffu, reach = MASS ? hi - (ordered_key(0.0f) + 1u) : hi;
+    unsigned span = MASS ? hi - max(ordered_key(top), ordered_key(9.5367432e-7f)) : hi;
+    unsigned long long before = 0ull, need = 0ull;
+    Threshold* zero = cl.map_shared_rank(th, 0);
+    for (int level = 0;; ++level) {
+        const int slot = (MASS ? 2 : 0) + (level & 1);
+        int first_rank = 0;          // (opaque, so that the eight blocks' addresses are made where they are used and not held in registers)
+        asm volatile("" : "+r"(first_rank));
+        // (span - 1) >> shift < BINS; all of a few in bin 0
+        const int shift = MASS && few ? 31 : span <= (unsigned)BINS ? 0 : 24 - __clz(span - 1u);
+        // the bins of UNROLL values from i0 on, higher values in lower bins; -1: not in play
+        float x[UNROLL];
+        int b[UNROLL];
+        auto bins_from = [&](int i0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) least += __shfl_xor_sync(0xffffffffu, least, o);
-    if ((tid & 31) == 0) {
-        atomicAdd(&th->hist[0][BINS - 1], (unsigned)least & 0x7fffu);
-        atomicAdd(&th->hist[1][BINS - 1], (unsigned)(least >> 15) & 0x7fffu);
-        atomicAdd(&th->hist[2][BINS - 1], (unsigned)(least >> 30));
-    }
-    cl.sync();
-    // this block's slice of the bins, over all blocks, as running sums
-    if (tid < BIN_SLICE) {
-        unsigned long long sum = 0ull;
+            for (int u = 0; u < UNROLL; ++u) {
+                const int i = i0 + u * CL_THREADS + tid;
+                x[u] = i < n ? mine[i] : 0.0f;
+                b[u] = i < n ? 0 : -1;
+            }
+            if (linear) {
 #pragma unroll
-        for (int b = 0; b < CL; ++b) {
-            const Threshold* o = cl.map_shared_rank(th, b);
-            const int at = rank * BIN_SLICE + tid;
-            sum += o->hist[0][at] + ((unsigned long long)o->hist[1][at] << 15) + ((unsigned long long)o->hist[2][at] << 30);
-        }
+                for (int u = 0; u < UNROLL; ++u) b[u] |= (int)fminf((top - x[u]) * scale, (float)(BINS - 1));
+            } else {
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long up = __shfl_up_sync(0xffffffffu, sum, o);
-            if ((tid & 31) >= o) sum += up;
-        }
-        th->slice_sum[tid] = sum;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        unsigned long long sum = 0ull;
-        for (int w = 31; w < BIN_SLICE; w += 32) sum += th->slice_sum[w];
-        th->total = sum;
-    }
-    cl.sync();
-    unsigned long long below = 0ull, total = 0ull;          // weight of the slices before this one, and of all
-#pragma unroll
-    for (int b = 0; b < CL; ++b) {
-        const unsigned long long t = cl.map_shared_rank(th, b)->total;
-        if (b < rank) below += t;
-        total += t;
-    }
-    const unsigned long long need = need_of(total);
-    if (total < need || need == 0ull) return false;          // the same in every block
-    if (tid < BIN_SLICE) {
-        unsigned long long upto = below, own = th->slice_sum[tid];
-        for (int w = 31; w < tid - (tid & 31); w += 32) upto += th->slice_sum[w];
-        const unsigned long long prev = (tid & 31) ? th->slice_sum[tid - 1] : 0ull;
-        if (upto + prev < need && upto + own >= need) {          // exactly one thread of the cluster
-            th->bin = rank * BIN_SLICE + tid;
-            th->before = upto + prev;
-        }
-    }
-    cl.sync();
-    int owner = 0;
-#pragma unroll
-    for (int b = 0; b < CL; ++b)
-        if (cl.map_shared_rank(th, b)->bin >= 0) owner = b;
-    Threshold* at = cl.map_shared_rank(th, owner);
-    const int bin = at->bin;
-    for (int i = tid; i < n; i += CL_THREADS) {
-        const float x = mine[i];
-        if (bin_of(x) == bin) {
-            const int k = atomicAdd(&at->listed, 1);
-            if (k < BIN_LIST) at->list[k] = x;
-        }
-    }
-    cl.sync();
-    if (rank == owner) {
-        const int m = th->listed;
-        if (m <= BIN_LIST) {
-            for (int i = tid; i < m; i += CL_THREADS) {
-                const float x = th->list[i];
-                const unsigned kx = ordered_key(x);          // (not the floats: a zero's sign decides what the caller keeps)
-                unsigned long long above = th->before, with = th->before;
-                for (int j = 0; j < m; ++j) {
-                    const float y = th->list[j];
-                    const unsigned ky = ordered_key(y);
-                    if (ky > kx) above += weight_of(y);
-                    if (ky >= kx) with += weight_of(y);
+                for (int u = 0; u < UNROLL; ++u) {
+                    const unsigned below = hi - (MASS ? __float_as_uint(x[u]) | 0x80000000u : ordered_key(x[u]));
+                    b[u] |= below <= reach ? (int)min(below >> shift, (unsigned)(BINS - 1)) : -1;
                 }
-                if (above < need && with >= need) { th->value = x; th->members = m; }      // equal keys: the same bits
+            }
+        };
+        int bin = 0;
+        if (!(MASS && few)) {
+            if (tid == 0 && (!MASS || level > 0)) th->start(slot);
+            for (int i = tid; i < PARTS * BINS; i += CL_THREADS) (&th->hist[0][0])[i] = 0u;
+            __syncthreads();
+            unsigned long long least = 0ull;
+#pragma unroll 1
+            for (int i0 = 0; i0 < n; i0 += UNROLL * CL_THREADS) {
+                bins_from(i0);
+#pragma unroll
+                for (int u = 0; u < UNROLL; ++u) {
+                    if (b[u] < 0) continue;
+                    const unsigned long long w = MASS ? mass_of(x[u]) : 1ull;
+                    if (b[u] == BINS - 1) least += w;
+                    else if (MASS) add_mass(th->hist, b[u], w);
+                    else atomicAdd(&th->hist[0][b[u]], 1u);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) least += __shfl_xor_sync(0xffffffffu, least, o);
+            if (lane == 0) {
+                if (MASS) add_mass(th->hist, BINS - 1, least);
+                else atomicAdd(&th->hist[0][BINS - 1], (unsigned)least);
+            }
+            cl.sync();
+            // the bins of all blocks, as running sums
+            unsigned long long own = 0ull, upto = 0ull;
+            if (tid < BINS) {
+#pragma unroll
+                for (int r = 0; r < CL; ++r) {
+                    const Threshold* o = cl.map_shared_rank(th, first_rank + r);
+                    own += o->hist[0][tid];
+                    if (MASS) own += ((unsigned long long)o->hist[1][tid] << 15) + ((unsigned long long)o->hist[2][tid] << 30);
+                }
+                upto = own;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned long long up = __shfl_up_sync(0xffffffffu, upto, o);
+                    if (lane >= o) upto += up;
+                }
+                if (lane == 31) th->warp_total[tid >> 5] = upto;
+            }
+            __syncthreads();
+            unsigned long long total = 0ull;
+#pragma unroll
+            for (int w = 0; w < BINS / 32; ++w) {
+                if (w < (tid >> 5)) upto += th->warp_total[w];
+                total += th->warp_total[w];
+            }
+            if (level == 0) need = max(MASS ? (unsigned long long)((double)share * (double)total) : (unsigned long long)share, 1ull);
+            if (tid < BINS && before + upto - own < need && before + upto >= need) {          // one thread of the block
+                th->bin = tid;
+                th->before = before + upto - own;
+                th->upto = before + upto;
+            }
+            __syncthreads();
+            bin = th->bin;
+            before = th->before;
+        }
+        // the bin's values: the keys that they span, and a list of them for every block as long as there is room
+        unsigned key_lo = 0xffffffffu, key_hi = 0u;
+        bool full = false;
+#pragma unroll 1
+        for (int i0 = 0; i0 < n; i0 += UNROLL * CL_THREADS) {
+            bins_from(i0);
+            bool any = false;
+#pragma unroll
+            for (int u = 0; u < UNROLL; ++u) any |= b[u] == bin;
+            if (!__any_sync(0xffffffffu, any)) continue;
+#pragma unroll
+            for (int u = 0; u < UNROLL; ++u) {
+                const bool member = b[u] == bin;
+                const unsigned members = __ballot_sync(0xffffffffu, member);
+                const unsigned key = ordered_key(x[u]);
+                if (member) {
+                    key_lo = min(key_lo, key);
+                    key_hi = max(key_hi, key);
+                }
+                if (members == 0u || full) continue;
+                const int first = __ffs(members) - 1;
+                int at = 0;
+                if (lane == first) at = atomicAdd(&zero->listed[slot], __popc(members));
+                at = __shfl_sync(0xffffffffu, at, first);
+                full = at >= BIN_LIST;
+                at += __popc(members & ((1u << lane) - 1u));
+                if (member && at < BIN_LIST) {
+                    const unsigned long long w = MASS ? mass_of(x[u]) : 1ull;
+#pragma unroll 1
+                    for (int r = 0; r < CL; ++r) {
+                        Threshold* o = cl.map_shared_rank(th, first_rank + r);
+                        ThresholdList& list = MASS ? o->by_mass : o->by_count;
+                        list.key[at] = key;
+                        list.weight[at] = w;
+                    }
+                }
             }
         }
+        key_lo = __reduce_min_sync(0xffffffffu, key_lo);
+        key_hi = __reduce_max_sync(0xffffffffu, key_hi);
+        if (lane == 0 && key_lo <= key_hi) {
+            atomicMin(&th->key_lo[slot], key_lo);
+            atomicMax(&th->key_hi[slot], key_hi);
+        }
+        cl.sync();
+        const int m = zero->listed[slot];
+        const Threshold* some = cl.map_shared_rank(th, lane % CL);
+        hi = __reduce_max_sync(0xffffffffu, some->key_hi[slot]);
+        reach = span = hi - __reduce_min_sync(0xffffffffu, some->key_lo[slot]);
+        if (span == 0u) {
+            if (tid == 0) th->reached = th->upto;
+            return hi;
+        }
+        if (m <= BIN_LIST) {
+            const ThresholdList& list = MASS ? th->by_mass : th->by_count;
+            const int i = tid >> 2;
+            const unsigned key = i < m ? list.key[i] : 0u;
+            unsigned long long above = before, with = before;
+            unsigned long long total = 0ull;
+            if (i < m) {
+                if (tid & 3) above = with = 0ull;
+                for (int j = tid & 3; j < m; j += 4) {
+                    const unsigned k = list.key[j];
+                    const unsigned long long w = list.weight[j];
+                    if (k > key) above += w;
+                    if (k >= key) with += w;
+                    if (MASS && few) total += w;
+                }
+            }
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                above += __shfl_xor_sync(0xffffffffu, above, o);
+                with += __shfl_xor_sync(0xffffffffu, with, o);
+                if (MASS && few) total += __shfl_xor_sync(0xffffffffu, total, o);
+            }
+            if (MASS && few) need = max((unsigned long long)((double)share * (double)total), 1ull);
+            if (i < m && above < need && with >= need) {          // equal keys write the same
+                th->value = key;
+                th->reached = with;
+            }
+            __syncthreads();
+            return th->value;
+        }
+        linear = false;
     }
-    cl.sync();
-    const bool found = at->members > 0;
-    *value = at->value;
-    cl.sync();          // (the next search clears what is read here)
-    return found;
 }
 
 // First index of the largest value of the whole row (0 if nothing lies above -inf), the same in every block.
@@ -456,7 +585,7 @@ __device__ int cluster_argmax(cg::cluster_group& cl, ClusterExchange* xc, const 
     return at < 0 ? 0 : at;
 }
 
-__global__ void __launch_bounds__(CL_THREADS) sample_cluster_kernel(const float* __restrict__ logits, int V, long long stride,
+__global__ void __launch_bounds__(CL_THREADS, 3) sample_cluster_kernel(const float* __restrict__ logits, int V, long long stride,
                                                                     int part, const float* __restrict__ temperature,
                                                                     const int* __restrict__ top_k,
                                                                     const float* __restrict__ top_p,
@@ -467,7 +596,6 @@ __global__ void __launch_bounds__(CL_THREADS) sample_cluster_kernel(const float*
     __shared__ Threshold th;
     __shared__ float shf[33];
     __shared__ int shi[33];
-    __shared__ float chunk_sum[CL_THREADS];
     __shared__ ClusterExchange xc;
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
@@ -475,7 +603,10 @@ __global__ void __launch_bounds__(CL_THREADS) sample_cluster_kernel(const float*
     const float* x = logits + (size_t)r * stride;
     const int begin = min(V, rank * part);
     const int n = min(part, V - begin);          // may be 0 for the last ranks of a short row
-    if (threadIdx.x == 0) xc.turn = 0;
+    if (threadIdx.x == 0) {
+        xc.turn = 0;
+        th.start(2);
+    }
     __syncthreads();
 
     const float temp = temperature[r];
@@ -490,16 +621,24 @@ __global__ void __launch_bounds__(CL_THREADS) sample_cluster_kernel(const float*
     const float tp = top_p ? top_p[r] : 1.0f;
     const float mp = min_p ? min_p[r] : 0.0f;
 
-    float mx = -INFINITY, odd = 0.0f;          // odd: how many values are not numbers
-    for (int i = threadIdx.x; i < n; i += CL_THREADS) {
-        const float v = x[begin + i] * inv_temp;
-        mine[i] = v;
-        mx = fmaxf(mx, v);
-        if (!(v == v)) odd += 1.0f;
+    const bool by_rank = k > 0 && k < V, by_mass = tp < 1.0f;
+    float mx = -INFINITY, low = -INFINITY;          // low: minus the smallest finite value; +inf where a value is not a number
+    if (by_rank || by_mass) {
+        for (int i = threadIdx.x; i < n; i += CL_THREADS) {
+            const float v = x[begin + i] * inv_temp;
+            mine[i] = v;
+            mx = fmaxf(mx, v);
+            low = fmaxf(low, v == v ? (v > -INFINITY ? -v : -INFINITY) : INFINITY);
+        }
+        cluster_max2(cl, &xc, mx, low, shf);
+    } else {
+        for (int i = threadIdx.x; i < n; i += CL_THREADS) {
+            const float v = x[begin + i] * inv_temp;
+            mine[i] = v;
+            mx = fmaxf(mx, v);
+        }
+        mx = cluster_max(cl, &xc, block_max(mx, shf));
     }
-    const bool filters = (k > 0 && k < V) || tp < 1.0f;
-    if (filters) odd = cluster_sum(cl, &xc, block_sum(odd, shf));
-    mx = cluster_max(cl, &xc, block_max(mx, shf));
     if (mx == -INFINITY || !(mx == mx)) {        // every logit is -inf, or NaN: fall back to argmax
         const int idx = cluster_argmax(cl, &xc, x, begin, n, shf, shi);
         if (rank == 0 && threadIdx.x == 0) out[r] = idx;
@@ -507,60 +646,37 @@ __global__ void __launch_bounds__(CL_THREADS) sample_cluster_kernel(const float*
         return;
     }
 
-    // top-k: key of the k-th largest scaled logit (largest K with count(key >= K) >= k).  By bins of 1/32 below the maximum where
-    // the row is one of numbers.
+    // top-k: key of the k-th largest scaled logit (largest K with count(key >= K) >= k).  The first bins are 1/8 wide below the maximum,
+    // and narrower where the whole row is narrower than they reach; a row with infinite values or NaN goes by keys alone.
     unsigned key_k = 0u;
-    const bool numbers = odd == 0.0f && mx < INFINITY;
-    float value = 0.0f;
-    bool found = false;
-    if (k > 0 && k < V && numbers)
-        found = cluster_threshold(
-            cl, &th, mine, n, [mx](float v) { const float d = (mx - v) * 32.0f; return d < (float)BINS ? (int)d : -1; },
-            [](float) { return 1ull; }, [k](unsigned long long) { return (unsigned long long)k; }, &value);
-    if (found) {
-        key_k = ordered_key(value);
-    } else if (k > 0 && k < V) {
-        for (int bit = 31; bit >= 0; --bit) {
-            const unsigned cand = key_k | (1u << bit);
-            float cnt = 0.0f;
-            for (int i = threadIdx.x; i < n; i += CL_THREADS) cnt += ordered_key(mine[i]) >= cand ? 1.0f : 0.0f;
-            cnt = cluster_sum(cl, &xc, block_sum(cnt, shf));
-            if (cnt >= (float)k) key_k = cand;
-        }
+    if (threadIdx.x == 0) {
+        th.top = mx;
+        th.low = low;
+        th.reached = (unsigned long long)V;
     }
+    __syncthreads();
+    if (by_rank) {
+        float scale = BINS / 32.0f;
+        if (mx + low > 0.0f) scale = fmaxf(scale, fminf((float)(BINS - 1) / (mx + low), 1e30f));
+        key_k = cluster_threshold<false>(&th, mine, n, mx, mx < INFINITY && low < INFINITY ? scale : 0.0f, (float)k, false);
+        __syncthreads();
+    }
+    mx = th.top;
     // e_i = exp(x_i/T - max) of the kept entries; everything below is in terms of e (max e = 1).
-    float z = 0.0f;
     for (int i = threadIdx.x; i < n; i += CL_THREADS) {
         const float v = mine[i];
-        const float e = ordered_key(v) < key_k ? 0.0f : expf(v - mx);
-        mine[i] = e;
-        z += e;
+        mine[i] = ordered_key(v) < key_k ? 0.0f : expf(v - mx);
     }
-    z = cluster_sum(cl, &xc, block_sum(z, shf));
-
-    // top-p: largest threshold on e whose kept mass still reaches p * z.
+    // top-p: largest threshold on e whose kept mass still reaches p of the whole.
     unsigned key_p = 0u;
-    found = false;
-    if (tp < 1.0f && tp > 0.0f && numbers)          // by bins of 1/32 of an octave below one (what is below 2^-32 shares the last)
-        found = cluster_threshold(
-            cl, &th, mine, n,
-            [](float e) { return e > 0.0f ? min(BINS - 1, (int)((0x3f800000u - __float_as_uint(e)) >> 18)) : -1; },
-            [](float e) { return (unsigned long long)(e * 17592186044416.0f); },
-            [tp](unsigned long long total) { return (unsigned long long)((double)tp * (double)total); }, &value);
-    if (found) {
-        key_p = ordered_key(value);
-    } else if (tp < 1.0f) {
-        const float need = tp * z;
-        for (int bit = 31; bit >= 0; --bit) {
-            const unsigned cand = key_p | (1u << bit);
-            float mass = 0.0f;
-            for (int i = threadIdx.x; i < n; i += CL_THREADS) {
-                const float e = mine[i];
-                if (e > 0.0f && ordered_key(e) >= cand) mass += e;
-            }
-            mass = cluster_sum(cl, &xc, block_sum(mass, shf));
-            if (mass >= need) key_p = cand;
+    if (by_mass) {
+        float least = expf(key_k ? key_value(key_k) - mx : -(mx + th.low));          // the smallest
+        if (!(mx < INFINITY && th.low < INFINITY)) {          // where one is not a number, everything stays, and the draw falls back to the argmax
+            least = -1.0f;
+            for (int i = threadIdx.x; i < n; i += CL_THREADS) least = mine[i] == mine[i] ? least : INFINITY;
+            least = cluster_max(cl, &xc, block_max(least, shf)) > 0.0f ? -1.0f : 0.0f;
         }
+        if (least >= 0.0f) key_p = tp > 0.0f ? cluster_threshold<true>(&th, mine, n, least, 0.0f, tp, th.reached <= (unsigned long long)BIN_LIST) : 0xffffffffu;
     }
     // min-p: probabilities below min_p * max probability are dropped; max e is 1.  What is kept stays in `mine`.
     const float e_min = mp > 0.0f ? mp : 0.0f;
@@ -577,9 +693,9 @@ __global__ void __launch_bounds__(CL_THREADS) sample_cluster_kernel(const float*
     const int cb = min(n, (int)threadIdx.x * per), ce = min(n, cb + per);
     float own = 0.0f;
     for (int i = cb; i < ce; ++i) own += mine[i];
-    chunk_sum[threadIdx.x] = own;
+    th.chunk_sum[threadIdx.x] = own;
     const float block_total = block_sum(own, shf);      // contains the barriers that publish chunk_sum
-    // every block learns every block's total (the same exchange as cluster_sum, but the parts are kept)
+    // every block learns every block's total (the same exchange as cluster_max, but the parts are kept and added up in rank order)
     const int t = xc.turn;
     if (threadIdx.x == 0) xc.f[t] = block_total;
     cl.sync();
@@ -620,8 +736,8 @@ __global__ void __launch_bounds__(CL_THREADS) sample_cluster_kernel(const float*
         if (!overshoot) {
             int c = 0;
             for (; c < CL_THREADS; ++c) {
-                if (chunk_sum[c] > 0.0f && run + chunk_sum[c] >= target) break;
-                run += chunk_sum[c];
+                if (th.chunk_sum[c] > 0.0f && run + th.chunk_sum[c] >= target) break;
+                run += th.chunk_sum[c];
             }
             if (c < CL_THREADS) {
                 const int b0 = min(n, c * per), e0 = min(n, b0 + per);
@@ -676,7 +792,7 @@ LLB_EXPORT int llb_sample(const float* logits, int R, int V, long long stride, c
     // long rows: a cluster of blocks per row, each with its part of the row in shared memory
     const int part = llb_ceil_div(V, CL);
     const size_t smem = (size_t)part * sizeof(float);
-    if (V >= 8192 && smem + sizeof(Threshold) + 4096 <= 227 * 1024 && R <= 65535) {
+    if (V >= 8192 && smem <= 216 * 1024 && R <= 65535) {          // (beside it 7 KB of the kernel's own)
         static size_t configured = 0;
         if (smem > configured) {
             cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
