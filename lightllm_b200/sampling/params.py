@@ -4,6 +4,8 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 
+GREEDY_BELOW = 1e-5          # temperatures under this one choose the largest logit
+
 
 @dataclass
 class SamplingParams:
@@ -32,4 +34,4 @@ class SamplingParams:
 
     @property
     def greedy(self) -> bool:
-        return self.temperature < 1e-5
+        return self.temperature < GREEDY_BELOW

@@ -15,7 +15,7 @@ import numpy as np
 import torch
 
 from ..csrc import ops
-from .params import SamplingParams
+from .params import GREEDY_BELOW, SamplingParams
 
 
 class RequestStream:
@@ -62,14 +62,14 @@ class Sampler:
             raise ValueError(f"{R} rows of logits but {len(request_ids)} requests and {len(params)} parameter sets")
         out = torch.empty(R, dtype=torch.int32, device=logits.device)
         temperature = [p.temperature for p in params]
-        if max(temperature, default=0.0) < 1e-5:          # (every row greedy, SamplingParams.greedy)
+        if all(t < GREEDY_BELOW for t in temperature):
             ops.argmax(logits, out)
             return out
         host = np.empty((5, R), dtype=np.float32)
         host[0] = temperature
         host[1] = [p.top_p for p in params]
         host[2] = [p.min_p for p in params]
-        host[3] = [0.0 if t < 1e-5 else self.stream(rid, p.seed).uniform() for rid, p, t in zip(request_ids, params, temperature)]
+        host[3] = [0.0 if t < GREEDY_BELOW else self.stream(rid, p.seed).uniform() for rid, p, t in zip(request_ids, params, temperature)]
         host[4].view(np.int32)[:] = [p.top_k for p in params]
         # (not waited for: from memory that is not pinned the driver has taken the numbers when the call returns)
         dev = torch.from_numpy(host).to(logits.device, non_blocking=True)
