@@ -673,10 +673,13 @@ __global__ void __launch_bounds__(128) paged_attention_tile_f32_kernel(AttnParam
     }
 }
 
-// Whether a call is one for the kernel above: floats, ordinary value rows, addresses in 16-byte steps.
+// Whether a call is one for the kernel above: floats, ordinary value rows, addresses in 16-byte steps, and tiles that the general
+// kernel takes too (its shared memory and the grid's second dimension), so that a call is refused whichever addresses it has.
 template <typename T>
 bool tile_f32_eligible(const AttnParams& p) {
     return sizeof(T) == 4 && p.nsplit == 1 && (p.hd == 64 || p.hd == 128) && p.hdv == p.hd && p.vrow % 4 == 0 && !p.v_shared &&
+           attention_smem_bytes(p.BQ, 1, p.hd, p.hdv) <= 220 * 1024 &&
+           (long long)p.Hkv * llb_ceil_div(p.BQ * (p.Hq / p.Hkv), TQ) <= 65535 &&
            (((uintptr_t)p.q | (uintptr_t)p.k_cache | (uintptr_t)p.v_cache | (uintptr_t)p.out) % 16) == 0;
 }
 
@@ -692,7 +695,6 @@ int launch_tile_f32(const AttnParams& p, int num_tiles, cudaStream_t stream) {
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
     const int vectors = p.BQ * (p.Hq / p.Hkv), chunks = llb_ceil_div(vectors, TQ);
-    LLB_REQUIRE((long long)p.Hkv * chunks <= 65535, "attention: too many heads for tiles of %d rows", p.BQ);
     paged_attention_tile_f32_kernel<HD><<<dim3(num_tiles, p.Hkv * chunks), 128, tile_f32_smem<HD>(), stream>>>(
         p, chunks, llb_ceil_div(vectors, chunks));
     return llb_check_launch("paged_attention_tile_f32");

@@ -45,3 +45,14 @@ def test_float_attention(ops, Hq, Hkv, hd, window, bq):  # noqa: F811
     got = out.cpu()
     assert not torch.isnan(got).any()
     assert torch.allclose(got, ref, atol=2e-5, rtol=2e-5), f"max diff {float((got - ref).abs().max())}"
+
+
+def test_a_tile_too_high_is_refused(ops):  # noqa: F811
+    """A tile whose rows the general kernel's shared memory cannot hold is refused in every dtype, at any address."""
+    from lightllm_b200.csrc.ops import KernelError
+    s = paged_setup(torch.float32, [500], [0], 2, 2, 64, 16, 3)
+    ts, tq, nt = tiles_for([500], 500)
+    out = torch.empty((500, 128), device=dev())
+    with pytest.raises(KernelError, match="use a smaller BQ"):
+        ops.paged_attention_simt(s["q"], s["kc"], s["vc"], out, ts, tq, nt, s["span_row"], s["span_len"], s["span_pos"], s["bt"],
+                                 s["max_pages"], 16, 2, 2, 64, 0, 0.125, 500)
