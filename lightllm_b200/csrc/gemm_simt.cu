@@ -369,7 +369,9 @@ int launch(const void* A, const void* W, const void* bias, void* out, float* res
         // The tile kernel: rows in 16-byte steps for cp.async, 64-column tiles in the grid's y.  From five rows on: at four the
         // streaming kernel, which reads the rows again for every pair of features, takes 21 us for 9,728 x 896 against 25 (and
         // 25 against 15 for 896 x 4,864), at six 26, at eight 30 and 45.
-        if (M > 4 && K % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0 && llb_ceil_div(N, F_BN) <= 65535)
+        // (More rows than the general kernel's grid counts are refused below, whatever their form.)
+        if (M > 4 && K % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0 && llb_ceil_div(N, F_BN) <= 65535 &&
+            llb_ceil_div(M, BM) <= 65535)
             return dispatch_f32<EPI>((const float*)A, (const float*)W, b, out, residual, M, N, K, glu, stream);
     }
     if (M <= MAXM) {

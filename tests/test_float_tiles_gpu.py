@@ -56,3 +56,12 @@ def test_a_tile_too_high_is_refused(ops):  # noqa: F811
     with pytest.raises(KernelError, match="use a smaller BQ"):
         ops.paged_attention_simt(s["q"], s["kc"], s["vc"], out, ts, tq, nt, s["span_row"], s["span_len"], s["span_pos"], s["bt"],
                                  s["max_pages"], 16, 2, 2, 64, 0, 0.125, 500)
+
+
+def test_too_many_rows_are_refused(ops):  # noqa: F811
+    """One row more than 65,535 tiles of 64 hold is refused whether or not the operands' rows are 16-byte steps."""
+    from lightllm_b200.csrc.ops import KernelError
+    for K in (4, 5):
+        a, w = torch.zeros((65535 * 64 + 1, K), device=dev()), torch.zeros((4, K), device=dev())
+        with pytest.raises(KernelError, match="too large for one launch"):
+            ops.gemm_simt(a, w, None, 0, torch.empty((a.shape[0], 4), device=dev()))
