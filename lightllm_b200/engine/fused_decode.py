@@ -17,7 +17,6 @@ from typing import List, Optional
 import torch
 
 from ..csrc import ops
-from ..parts import linear as L
 from ..parts.attention import AttentionMixer
 from ..parts.mlp import GatedMLP
 from ..parts.norm import RMSNorm
