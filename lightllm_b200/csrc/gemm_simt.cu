@@ -14,6 +14,8 @@
 // and a 64x64x16 tile kernel for everything else (odd inner sizes, 16-bit operands).
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "common.cuh"
 
 namespace {
@@ -178,8 +180,9 @@ __global__ void __launch_bounds__(256) gemm_rows_kernel(const TA* __restrict__ A
 
 // ---- many rows of floats ----------------------------------------------------------------------------------------------
 // A block makes a BM x 64 tile with four groups of 64 threads, each group over its own 8 columns of every 32-wide slice of
-// K; a thread holds BM/8 x 8 sums.  What bounds it is the FFMA pipe (256 of them against 16 16-byte shared loads per
-// thread and 4 columns), so the rest is arranged to keep two blocks of eight warps on every multiprocessor issuing them:
+// K; a thread holds BM/8 x 8 sums.  What bounds it is the dispatch of FFMA (256 of them against 16 16-byte shared loads per thread
+// and 4 columns; two thirds of the cycles issue, their pipe is busy for 47 %, and ready warps wait for the register file's ports),
+// so the rest is arranged to keep two blocks of eight warps on every multiprocessor issuing them:
 // operands by cp.async three slices deep, rows 36 floats apart (16-byte reads of 8 neighbouring rows meet no bank twice),
 // and K cut among the blocks of a cluster where the tiles alone would leave multiprocessors idle.  The groups' and then
 // the cluster's sums meet in shared memory in a fixed order.
@@ -317,14 +320,16 @@ template <int EPI, int BM>
 int launch_f32(const float* A, const float* W, const float* bias, void* out, float* residual, int M, int N, int K, LlbGluArgs glu,
                cudaStream_t stream) {
     constexpr int smem = f32_smem_bytes<BM>();
-    static bool configured[64] = {};
-    constexpr int sms = 148;
+    static std::atomic<int> sms_of[64] = {};          // 0: this device has not been set up
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<EPI, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    int sms = dev >= 0 && dev < 64 ? sms_of[dev].load() : 0;
+    if (sms == 0) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<EPI, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return llb_fail("gemm: cannot opt in to %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-        if (dev >= 0 && dev < 64) configured[dev] = true;
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return llb_fail("gemm: cannot ask for the multiprocessors: %s", cudaGetErrorString(e));
+        if (dev >= 0 && dev < 64) sms_of[dev].store(sms);
     }
     const int mt = llb_ceil_div(M, BM), nt = llb_ceil_div(N, F_BN), slices = llb_ceil_div(K, F_BK);
     // two blocks are resident on a multiprocessor: K is cut until the tiles fill them once, no piece below four slices
