@@ -339,8 +339,30 @@ struct ItemGeom {
 struct CutPlan {
     int before[MAX_ROWS + 1];        // pieces of the rows before
     int piece;
+    int window;                      // what it was made for
     ItemGeom first;                  // what the block's first item covers (for most blocks the only one), the same in every layer
 };
+constexpr int KEPT_CUTS = 4;         // cuts of other windows that a block keeps for the layers to come
+
+// What an item covers (its row's block table aside).
+__device__ __forceinline__ ItemGeom locate_item(const int* span_pos, int M, int Hkv, int window, const CutPlan& cut, int item) {
+    ItemGeom g;
+    g.bt = nullptr;
+    g.kvh = item % Hkv;
+    const int at = item / Hkv;
+    int r = 0;                                                    // the row whose pieces hold this one
+#pragma unroll 1
+    for (int step = MAX_ROWS / 2; step > 0; step >>= 1)
+        if (r + step < M && cut.before[r + step] <= at) r += step;
+    g.r = r;
+    g.sp = at - cut.before[r];
+    const int qpos = __ldg(span_pos + r);                         // cached keys: positions below the new token's
+    const int lo = window > 0 ? max(0, qpos - window + 1) : 0;
+    g.klo = lo + g.sp * cut.piece;
+    g.khi = min(qpos, g.klo + cut.piece);
+    g.owner = at + 1 == cut.before[r + 1];
+    return g;
+}
 // By one warp, for a layer's window.  Requests of a batch are at different places, so a fixed number of pieces a row leaves the
 // stage to its longest row (27 requests of 65 to 4,001 keys: two pieces a row, up to 2,000 keys an item where the average over
 // the blocks is 360); pieces of one length finish together.  They are as long as it takes for the items not to pass the blocks
@@ -348,7 +370,7 @@ struct CutPlan {
 // Measured, ms a step before -> after: those 27 requests at the 1.5B sizes 2.81 -> 2.05, 25 requests of 40 to 3,000 keys at the
 // 0.5B sizes 1.12 -> 0.95, 8 equal requests 0.776 -> 0.763 (no piece of zero keys any more).
 template <int BK>
-__device__ __noinline__ void make_cut(const int* span_pos, int M, int Hkv, int nsplit, int window, CutPlan* cut, int lane) {
+__device__ __forceinline__ void make_cut(const int* span_pos, int M, int Hkv, int nsplit, int window, CutPlan* cut, int lane) {
     int len[2], longest = 0, total = 0;
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
@@ -389,7 +411,32 @@ __device__ __noinline__ void make_cut(const int* span_pos, int M, int Hkv, int n
         cut->before[lane + 32 * u + 1] = base + sum;
         base += __shfl_sync(0xffffffffu, sum, 31);
     }
-    if (lane == 0) { cut->before[0] = 0; cut->piece = piece; }
+    if (lane == 0) { cut->before[0] = 0; cut->piece = piece; cut->window = window; }
+}
+
+// By one warp: the cut for a layer's window into `cut`.  A window that a layer before had is copied from where that cut is kept: made
+// anew at every change, layers that alternate between two windows paid 2 to 5 us each (8 layers at the 1.5B sizes, one request
+// of 2,048 keys: 374 us as one run of equal layers, 410 with windows none / 512 in turn).  The copy goes to the one place that
+// the stages read, so that they hold no pointer to it: with one, every model's steps were 4 % slower.
+template <int BK>
+__device__ __noinline__ void cut_for_window(const int* span_pos, int M, int Hkv, int nsplit, int window, bool fresh, CutPlan* cut,
+                                            CutPlan* kept, int lane) {
+    static_assert(sizeof(CutPlan) % 4 == 0, "copied by words");
+    if (fresh && lane < KEPT_CUTS) kept[lane].window = -1;
+    __syncwarp();
+    int slot = 0;
+    while (slot < KEPT_CUTS - 1 && kept[slot].window != window && kept[slot].window >= 0) ++slot;
+    const bool known = kept[slot].window == window;
+    __syncwarp();
+    if (!known) {
+        make_cut<BK>(span_pos, M, Hkv, nsplit, window, cut, lane);
+        __syncwarp();
+        if (lane == 0 && (int)blockIdx.x < cut->before[M] * Hkv) cut->first = locate_item(span_pos, M, Hkv, window, *cut, blockIdx.x);
+        __syncwarp();
+    }
+    const int* from = reinterpret_cast<const int*>(known ? kept + slot : cut);
+    int* to = reinterpret_cast<int*>(known ? cut : kept + slot);
+    for (int i = lane; i < (int)(sizeof(CutPlan) / 4); i += 32) to[i] = from[i];
 }
 
 // S3: the attention output of 64 columns (one head, or half of one), its pieces merged by their softmax weights:
@@ -497,28 +544,14 @@ struct LayerCache {
     float eps1;
     int window;
 };
-template <bool STORED = true>
 __device__ __forceinline__ ItemGeom item_geom(const FusedParams& p, const LayerCache& L, const CutPlan& cut, int item) {
     ItemGeom g;
-    if (STORED && item == (int)blockIdx.x) {
+    if (item == (int)blockIdx.x) {
         g = cut.first;
         g.bt = L.block_table + (size_t)g.r * p.max_pages;
         return g;
     }
-    g.kvh = item % p.Hkv;
-    const int at = item / p.Hkv;
-    int r = 0;                                                    // the row whose pieces hold this one
-#pragma unroll 1
-    for (int step = MAX_ROWS / 2; step > 0; step >>= 1)
-        if (r + step < p.M && cut.before[r + step] <= at) r += step;
-    g.r = r;
-    g.sp = at - cut.before[r];
-    const int qpos = __ldg(p.span_pos + g.r);
-    const int hi = qpos;                                          // cached keys: positions below the new token's
-    const int lo = L.window > 0 ? max(0, qpos - L.window + 1) : 0;
-    g.klo = lo + g.sp * cut.piece;
-    g.khi = min(hi, g.klo + cut.piece);
-    g.owner = at + 1 == cut.before[r + 1];
+    g = locate_item(p.span_pos, p.M, p.Hkv, L.window, cut, item);
     g.bt = L.block_table + (size_t)g.r * p.max_pages;
     return g;
 }
@@ -803,6 +836,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) decode_layers_kernel(const Fus
     __shared__ volatile int wait_ok[2];   // what the polling worker warp found, for the warps parked meanwhile (used in turn)
     __shared__ BlockPlan plan;
     __shared__ CutPlan cut;
+    __shared__ CutPlan kept_cuts[KEPT_CUTS];
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* a_tiles = smem;
@@ -1056,11 +1090,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) decode_layers_kernel(const Fus
             lc.block_table = p.block_tables[L->group]; lc.slot_mapping = p.slot_mapping[L->group];
             if (lc.window != cut_window) {        // (the layer before has merged its pieces: all blocks have met since)
                 worker_sync();
-                if (warp == 2) {
-                    make_cut<HD == 64 ? 32 : 16>(p.span_pos, p.M, p.Hkv, p.nsplit, lc.window, &cut, lane);
-                    __syncwarp();
-                    if (lane == 0 && (int)blockIdx.x < cut.before[p.M] * p.Hkv) cut.first = item_geom<false>(p, lc, cut, blockIdx.x);
-                }
+                if (warp == 2)
+                    cut_for_window<HD == 64 ? 32 : 16>(p.span_pos, p.M, p.Hkv, p.nsplit, lc.window, cut_window < 0, &cut, kept_cuts, lane);
                 cut_window = lc.window;
                 worker_sync();
             }

@@ -689,8 +689,8 @@ FUSED_CASES = [
 ]
 
 
-def fused_reference(h, layers, ctx_k, ctx_v, positions, Hq, Hkv, hd, rotary_dim, interleaved, theta, window):
-    """Plain float64 layers on the new tokens: h [M, D]; ctx_k/ctx_v[l][r]: the cached keys and values of request r."""
+def fused_reference(h, layers, ctx_k, ctx_v, positions, Hq, Hkv, hd, rotary_dim, interleaved, theta, windows):
+    """Plain float64 layers on the new tokens: h [M, D]; ctx_k/ctx_v[l][r]: the cached keys and values of request r; one window a layer."""
     from tests.plain import qwen2_plain as P
     M = h.shape[0]
     new_k = [[None] * M for _ in layers]
@@ -710,7 +710,7 @@ def fused_reference(h, layers, ctx_k, ctx_v, positions, Hq, Hkv, hd, rotary_dim,
             vv = torch.cat([ctx_v[li][r], v[r: r + 1]])
             qq = torch.zeros(kk.shape[0], Hq, hd, dtype=h.dtype)
             qq[-1] = q[r]
-            att[r] = P.plain_attention(qq, kk, vv, 1.0 / math.sqrt(hd), window)[-1].reshape(-1)
+            att[r] = P.plain_attention(qq, kk, vv, 1.0 / math.sqrt(hd), windows[li])[-1].reshape(-1)
             new_k[li][r], new_v[li][r] = k[r], v[r]
         h = h + P.plain_linear(att, w["w_o"])
         x = P.plain_rmsnorm(h, w["n2"], w["eps2"])
@@ -719,13 +719,15 @@ def fused_reference(h, layers, ctx_k, ctx_v, positions, Hq, Hkv, hd, rotary_dim,
 
 
 @pytest.mark.parametrize("case", FUSED_CASES)
-def test_decode_layers_against_plain_layers(ops, case):
+def test_decode_layers_against_plain_layers(ops, case, nsplit=None):
     """The persistent kernel on its own, at sizes the engine's tests do not have: first tokens, page edges, a window's
     edge, 64 rows, groups of 16, partial and interleaved rotation, float32 norm weights, no bias, no positions.  The
     residual after the layers and the keys and values it wrote are compared with plain float64 layers.  Run twice:
-    the second launch finds the scratch and the counters as the first left them."""
+    the second launch finds the scratch and the counters as the first left them.  (``window`` may be a list, one of each
+    layer; ``nsplit``: the most pieces a request.)"""
     D, Hq, Hkv, hd, I, page, rotary_dim, interleaved, bias, norm_dt, window, nl, contexts = case
     M = len(contexts)
+    windows = window if isinstance(window, list) else [window] * nl
     assert ops.decode_layers_supports(M, D, Hq, Hkv, hd, I, rotary_dim)
     g = torch.Generator().manual_seed(50 + D)
     bf = lambda t: t.to(torch.bfloat16)
@@ -768,15 +770,15 @@ def test_decode_layers_against_plain_layers(ops, case):
         layers.append(dict(w_qkv=dw["w_qkv"], w_o=dw["w_o"],
                            w_gate_up=torch.stack([dw["w_gate"], dw["w_up"]], dim=1).reshape(2 * I, D).contiguous(),
                            w_down=dw["w_down"], b_qkv=dw["b_qkv"], norm1_w=dw["n1"], norm2_w=dw["n2"], k_cache=kc, v_cache=vc,
-                           eps1=w["eps1"], eps2=w["eps2"], window=window or 0, group=0))
+                           eps1=w["eps1"], eps2=w["eps2"], window=windows[li] or 0, group=0))
         ref_layers.append({k: (v.double() if isinstance(v, torch.Tensor) else v) for k, v in w.items()})
     h0 = rn(M, D, s=2.0)
     positions = torch.tensor(contexts, dtype=torch.int32)
     want, new_k, new_v = fused_reference(h0.double(), ref_layers, ctx_k, ctx_v, positions.long(), Hq, Hkv, hd, rotary_dim,
-                                         interleaved, theta, window)
+                                         interleaved, theta, windows)
     desc = ops.decode_layers_descriptors(layers, D, Hq, Hkv, hd, I, dev())
     counters = ops.decode_layers_counters(dev())
-    nsplit = 5 if max(contexts) > 256 else 2
+    nsplit = nsplit or (5 if max(contexts) > 256 else 2)
     scratch = torch.full((ops.decode_layers_scratch_floats(M, Hq, Hkv, hd, I, nsplit),), float("nan"), device=dev())
     table = None
     if rotary_dim:
