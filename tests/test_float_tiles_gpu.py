@@ -47,6 +47,33 @@ def test_float_attention(ops, Hq, Hkv, hd, window, bq):  # noqa: F811
     assert torch.allclose(got, ref, atol=2e-5, rtol=2e-5), f"max diff {float((got - ref).abs().max())}"
 
 
+@pytest.mark.parametrize("Hq,Hkv,hd", [(6, 2, 64), (6, 2, 128), (4, 4, 128), (9, 1, 128)])
+@pytest.mark.parametrize("window,keep", [(0, 0), (33, 5), (70, 66), (-24, 0)])
+def test_float_attention_with_all_that_scores_take(ops, Hq, Hkv, hd, window, keep):  # noqa: F811
+    """Cap, slopes, sinks, a window (or a block of positions) and first keys that stay, against float64."""
+    lens, starts, cap, bq = [1, 16, 67, 33], [0, 63, 0, 130], 6.0, 16
+    s = paged_setup(torch.float32, lens, starts, Hq, Hkv, hd, 16, 12)
+    sinks, slopes = rnd((Hq,), torch.float32, 5), rnd((Hq,), torch.float32, 6, 0.05).abs()
+    ts, tq, nt = tiles_for(lens, bq)
+    out = torch.full((s["rows"], Hq * hd), float("nan"), device=dev())
+    ops.paged_attention_simt(s["q"], s["kc"], s["vc"], out, ts, tq, nt, s["span_row"], s["span_len"], s["span_pos"], s["bt"],
+                             s["max_pages"], 16, Hq, Hkv, hd, window, hd ** -0.5, bq, sinks=sinks, softcap=cap, keep=keep, slopes=slopes)
+    want = []
+    for (q, k, v), n, start in zip(s["full"], lens, starts):
+        q, k, v = q.double()[start:], k.double().repeat_interleave(Hq // Hkv, 1), v.double().repeat_interleave(Hq // Hkv, 1)
+        at, key = torch.arange(start, start + n)[:, None], torch.arange(start + n)[None]
+        first = at - window + 1 if window > 0 else at - at % -window if window < 0 else torch.zeros_like(at)
+        visible = (key <= at) & ((key >= first) | (key < keep))
+        x = cap * torch.tanh(torch.einsum("qhd,khd->hqk", q, k) * hd ** -0.5 / cap)
+        x = x - slopes.double().cpu()[:, None, None] * (at - key)
+        e = torch.where(visible, x.exp(), 0.0)          # (scores are at most the cap: no maximum to take off)
+        den = e.sum(-1) + sinks.double().cpu()[:, None].exp()
+        want.append(torch.einsum("hqk,khd->qhd", e / den[:, :, None], v).reshape(n, Hq * hd))
+    want, got = torch.cat(want), out.double().cpu()
+    assert not torch.isnan(got).any()
+    assert torch.allclose(got, want, atol=2e-5, rtol=2e-5), f"max diff {float((got - want).abs().max())}"
+
+
 def test_a_tile_too_high_is_refused(ops):  # noqa: F811
     """A tile whose rows the general kernel's shared memory cannot hold is refused in every dtype, at any address."""
     from lightllm_b200.csrc.ops import KernelError
