@@ -316,28 +316,55 @@ __global__ void __launch_bounds__(F_THREADS, 2) gemm_f32_kernel(const float* __r
     if (parts > 1) cg::this_cluster().sync();          // the others may still read this block's sums
 }
 
+// Multiprocessors of the current device.
+int device_sms() {
+    static std::atomic<int> known[64] = {};
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64) sms = known[dev].load();
+    if (sms == 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return 1;
+        if (dev >= 0 && dev < 64) known[dev].store(sms);
+    }
+    return sms;
+}
+
+// Into how many pieces K is cut: two blocks are resident on a multiprocessor, and the tiles shall fill them once; no piece
+// below four slices.  The order of a row's sum depends on it, and so its last bits depend on how many rows are beside it.
+int f32_split(int tiles, int slices) {
+    int split = 2 * device_sms() / tiles;
+    split = split > slices / 4 ? slices / 4 : split;
+    return split < 1 ? 1 : split > F_MAX_SPLIT ? F_MAX_SPLIT : split;
+}
+
+// Whether M rows, five to eight of them, are for the streaming kernel (fewer always are, more never).  It reads the rows again for every
+// pair of features; the tile kernel takes as long for five rows as for 16, and mostly less: 896 x 4,864 (features x K) 12 us, streaming
+// 29 to 41 at five to eight rows, 3,584 x 3,584 21 / 29 to 39, 2,048 x 64 3.3 / 3.3 to 3.9, 13,824 x 896 24 / 27 to 38.  Streaming is
+// ahead where a tile's chain of slices is the longer one: K of three to eight slices, which tiles hardly cut, under few features (896 x
+// 256 5.0 us, streaming 3.9 to 5.0; 2,048 x 128 4.1 / 3.3 to 4.1; 4,096 x 256 at five rows 5.2 / 4.7), and a longer K that is not cut
+// because every multiprocessor has a tile but few have two (9,728 x 896 23.6 / 17 to 21 at up to seven rows, 10,624 x 4,096 98 / 70 to 83).
+bool f32_streamed(int M, int N, int K) {
+    const int nt = llb_ceil_div(N, F_BN), slices = llb_ceil_div(K, F_BK), sms = device_sms();
+    if (M <= 4 || M > 8) return M <= 4;
+    if (slices <= 8) return slices >= 3 && (long long)nt * M <= 320;
+    return slices >= 16 && nt > sms && nt <= sms * 6 / 5 && nt * M <= 8 * sms;
+}
+
 template <int EPI, int BM>
 int launch_f32(const float* A, const float* W, const float* bias, void* out, float* residual, int M, int N, int K, LlbGluArgs glu,
                cudaStream_t stream) {
     constexpr int smem = f32_smem_bytes<BM>();
-    static std::atomic<int> sms_of[64] = {};          // 0: this device has not been set up
+    static std::atomic<bool> configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    int sms = dev >= 0 && dev < 64 ? sms_of[dev].load() : 0;
-    if (sms == 0) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<EPI, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (dev < 0 || dev >= 64 || !configured[dev].load()) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<EPI, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return llb_fail("gemm: cannot opt in to %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return llb_fail("gemm: cannot ask for the multiprocessors: %s", cudaGetErrorString(e));
-        if (dev >= 0 && dev < 64) sms_of[dev].store(sms);
+        if (dev >= 0 && dev < 64) configured[dev].store(true);
     }
     const int mt = llb_ceil_div(M, BM), nt = llb_ceil_div(N, F_BN), slices = llb_ceil_div(K, F_BK);
-    // two blocks are resident on a multiprocessor: K is cut until the tiles fill them once, no piece below four slices
-    int split = 2 * sms / (mt * nt);
-    split = split > slices / 4 ? slices / 4 : split;
-    split = split < 1 ? 1 : split > F_MAX_SPLIT ? F_MAX_SPLIT : split;
-    const int per = llb_ceil_div(slices, split);
-    split = llb_ceil_div(slices, per);
+    const int per = llb_ceil_div(slices, f32_split(mt * nt, slices));
+    const int split = llb_ceil_div(slices, per);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(mt, nt, split);
     cfg.blockDim = dim3(F_THREADS);
@@ -371,11 +398,9 @@ int launch(const void* A, const void* W, const void* bias, void* out, float* res
     const float* b = (const float*)bias;
     constexpr int MAXM = 8;
     if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4) {
-        // The tile kernel: rows in 16-byte steps for cp.async, 64-column tiles in the grid's y.  From five rows on: at four the
-        // streaming kernel, which reads the rows again for every pair of features, takes 21 us for 9,728 x 896 against 25 (and
-        // 25 against 15 for 896 x 4,864), at six 26, at eight 30 and 45.
-        // (More rows than the general kernel's grid counts are refused below, whatever their form.)
-        if (M > 4 && K % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0 && llb_ceil_div(N, F_BN) <= 65535 &&
+        // The tile kernel: rows in 16-byte steps for cp.async, 64-column tiles in the grid's y, not a call that the streaming kernel is
+        // better at.  (More rows than the general kernel's grid counts are refused below, whatever their form.)
+        if (!f32_streamed(M, N, K) && K % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0 && llb_ceil_div(N, F_BN) <= 65535 &&
             llb_ceil_div(M, BM) <= 65535)
             return dispatch_f32<EPI>((const float*)A, (const float*)W, b, out, residual, M, N, K, glu, stream);
     }

@@ -8,7 +8,9 @@ pytestmark = pytest.mark.gpu
 
 # rows around the heights of 16, 32 and 64; columns around 64 (odd ones too); K from one 16-byte step over ends of a slice
 # of 32 to sums that are cut among the blocks of a cluster (few tiles over a long K)
-SHAPES = [(4, 66, 36), (5, 66, 36), (9, 64, 4), (16, 63, 28), (17, 65, 32), (32, 2, 36), (33, 129, 100), (64, 128, 896), (65, 66, 4864), (389, 896, 1536)]
+SHAPES = [(4, 66, 36), (5, 66, 36), (9, 64, 4), (16, 63, 28), (17, 65, 32), (32, 2, 36), (33, 129, 100), (64, 128, 896), (65, 66, 4864), (389, 896, 1536),
+          # five to eight rows at the edges of what the row-streaming kernel takes of them: slices of K, tiles of features times rows
+          (5, 4096, 96), (5, 4097, 96), (8, 64, 64), (8, 64, 68), (8, 64, 256), (9, 64, 256), (8, 64, 260), (7, 9473, 512), (8, 9473, 512), (5, 11361, 512)]
 
 
 @pytest.mark.parametrize("M,N,K", SHAPES)
