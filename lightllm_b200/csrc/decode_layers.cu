@@ -415,9 +415,9 @@ __device__ __forceinline__ void make_cut(const int* span_pos, int M, int Hkv, in
 }
 
 // By one warp: the cut for a layer's window into `cut`.  A window that a layer before had is copied from where that cut is kept: made
-// anew at every change, layers that alternate between two windows paid 2 to 5 us each (8 layers at the 1.5B sizes, one request
-// of 2,048 keys: 374 us as one run of equal layers, 410 with windows none / 512 in turn).  The copy goes to the one place that
-// the stages read, so that they hold no pointer to it: with one, every model's steps were 4 % slower.
+// anew at every change, it lay on the path of every layer that alternates (eight layers with windows none / 512 in turn, 8 requests of
+// 2,048 keys: 419 us made anew, 405 kept at the 1.5B sizes, 252 and 243 at the 0.5B sizes).  The copy goes to the one place that the
+// stages read, so that they hold no pointer to it: with one, every model's steps were 4 % slower.
 template <int BK>
 __device__ __noinline__ void cut_for_window(const int* span_pos, int M, int Hkv, int nsplit, int window, bool fresh, CutPlan* cut,
                                             CutPlan* kept, int lane) {
