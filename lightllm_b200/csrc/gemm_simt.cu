@@ -1,5 +1,6 @@
-// Dense contraction on CUDA cores with float accumulation: the true 32-bit path of every
-// linear layer, and the path for shapes the tensor-core kernel refuses.
+// Dense contraction on CUDA cores with float accumulation: the 32-bit path of every linear layer with few rows or little
+// work (floats with more of both go to csrc/gemm_f32_tcgen05.cu, at no larger error), and the path for shapes the bf16
+// tensor-core kernel refuses.
 //
 // C[M,N] = A[M,K] * W[N,K]^T, W stored [out, in] as in the checkpoint
 // (src/engine/engine_server.cpp:1542-1544; the reference calls cublasSgemm for it,
@@ -10,13 +11,20 @@
 // (src/ops/elementwise.cu:27-33, engine_server.cpp:1875-1878).
 //
 // Three kernels: a row-streaming kernel for few rows (decode), where every weight row is read once by one warp with
-// 16-byte loads; a tile kernel for float operands whose rows are 16-byte multiples (the 32-bit path of every model);
+// 16-byte loads; a tile kernel for float operands whose rows are 16-byte multiples;
 // and a 64x64x16 tile kernel for everything else (odd inner sizes, 16-bit operands).
 #include <cooperative_groups.h>
 
 #include <atomic>
 
 #include "common.cuh"
+
+// csrc/gemm_f32_tcgen05.cu: the same of float operands on the tensor cores, split into bf16 numbers that add up to them.
+bool llb_gemm_f32_tcgen05_takes(const void* A, const void* W, int M, int N, int K);
+LLB_EXPORT long long llb_gemm_f32_scratch_bytes(int M, int K);
+LLB_EXPORT int llb_gemm_f32_tcgen05(const void* A, const void* W, const void* bias, void* out, float* residual, int epilogue, int M,
+                                    int N, int K, int glu_kind, float glu_alpha, float glu_limit, float glu_up_shift, void* scratch,
+                                    int* error_flag, cudaStream_t stream);
 
 namespace {
 
@@ -350,6 +358,19 @@ bool f32_streamed(int M, int N, int K) {
     return slices >= 16 && nt > sms && nt <= sms * 6 / 5 && nt * M <= 8 * sms;
 }
 
+// Whether floats go to the tensor cores (csrc/gemm_f32_tcgen05.cu).  That kernel and the one before it take 7 to 10 us whatever they are
+// given, so the products (of the rows that the tiles here would pad to) have to be worth it; us there / here at features x K:
+//   389 rows  64 x 896 13 / 10, 512 x 256 15 / 11, 256 x 896 14 / 15, 4,096 x 64 13 / 20, 9,728 x 896 58 / 227, 151,936 x 896 703 / 3,110
+//   100 rows  4,096 x 128 12 / 11, 4,096 x 256 14 / 16, 896 x 896 13 / 15, 4,096 x 896 15 / 35
+//   48 rows   2,048 x 512 11 / 10, 4,096 x 256 11 / 11, 4,096 x 512 11 / 15, 896 x 4,864 22 / 26
+// At 17 to 32 rows the tiles here are as low as the rows, and only many features make up for the long chain of slices there
+// (24 rows: 896 x 4,864 21 / 15, 4,096 x 896 13 / 13, 6,144 x 896 18 / 23, 9,728 x 896 26 / 31, 151,936 x 896 235 / 250).
+bool f32_split_pays(int M, int N, int K) {
+    if (M <= 16) return false;
+    if (M <= 32) return N >= 6144 && K >= 512;
+    return (long long)llb_ceil_div(M, 64) * 64 * N * K >= 80000000ll;
+}
+
 template <int EPI, int BM>
 int launch_f32(const float* A, const float* W, const float* bias, void* out, float* residual, int M, int N, int K, LlbGluArgs glu,
                cudaStream_t stream) {
@@ -436,20 +457,32 @@ int dispatch_epilogue(int epi, const void* A, const void* W, const void* bias, v
 
 }  // namespace
 
+// Bytes of scratch with which a contraction of these sizes goes to the tensor cores (0: it stays on CUDA cores).
+LLB_EXPORT long long llb_gemm_simt_scratch_bytes(int a_dtype, int w_dtype, int M, int N, int K) {
+    if (a_dtype != LLB_F32 || w_dtype != LLB_F32 || M <= 0 || N <= 0 || K <= 0 || K % 4 != 0 || llb_ceil_div(M, BM) > 65535) return 0;
+    return f32_split_pays(M, N, K) ? llb_gemm_f32_scratch_bytes(M, K) : 0;
+}
+
 // A [M,K] (a_dtype), W [N,K] (w_dtype), bias [N] float or null.  `out` is [M,N] of a_dtype
 // (STORE), [M,N] float (STORE_F32) or [M,N/2] of a_dtype (SWIGLU, N even); `residual` is
 // [M,N] float (RESIDUAL).  Supported: (float,float), (bf16,bf16), (bf16 activations, float weights).
 // glu_kind .. glu_up_shift: the gated activation of the GLU epilogue (LLB_GLU_*, see llb_glu); under STORE a kind of LlbAct
 // is a plain activation of every output.
+// scratch (16-byte aligned): null, or as llb_gemm_simt_scratch_bytes says; error_flag: raised when a wait ran out of time.
 LLB_EXPORT int llb_gemm_simt_glu(const void* A, int a_dtype, const void* W, const void* bias, int w_dtype, void* out,
                                  float* residual, int epilogue, int M, int N, int K, int glu_kind, float glu_alpha,
-                                 float glu_limit, float glu_up_shift, cudaStream_t stream) {
+                                 float glu_limit, float glu_up_shift, void* scratch, long long scratch_bytes,
+                                 int* error_flag, cudaStream_t stream) {
     const LlbGluArgs glu = LlbGluArgs{glu_kind, glu_alpha, glu_limit, glu_up_shift};
     if (M == 0) return 0;
     LLB_REQUIRE(M > 0 && N > 0 && K > 0, "gemm: bad sizes M=%d N=%d K=%d", M, N, K);
     LLB_REQUIRE(epilogue != LLB_EPI_SWIGLU || N % 2 == 0, "gemm: SwiGLU epilogue needs an even N, got %d", N);
     LLB_REQUIRE(epilogue != LLB_EPI_RESIDUAL || residual != nullptr, "gemm: residual epilogue without residual");
     LLB_REQUIRE(epilogue == LLB_EPI_RESIDUAL || out != nullptr, "gemm: output pointer is null");
+    const long long need = llb_gemm_simt_scratch_bytes(a_dtype, w_dtype, M, N, K);
+    if (need > 0 && scratch && scratch_bytes >= need && llb_gemm_f32_tcgen05_takes(A, W, M, N, K))
+        return llb_gemm_f32_tcgen05(A, W, bias, out, residual, epilogue, M, N, K, glu_kind, glu_alpha, glu_limit, glu_up_shift,
+                                    scratch, error_flag, stream);
     if (a_dtype == LLB_F32 && w_dtype == LLB_F32)
         return dispatch_epilogue<float, float>(epilogue, A, W, bias, out, residual, M, N, K, glu, stream);
     if (a_dtype == LLB_BF16 && w_dtype == LLB_BF16)
@@ -461,7 +494,8 @@ LLB_EXPORT int llb_gemm_simt_glu(const void* A, int a_dtype, const void* W, cons
 
 // The same with SiLU as the GLU epilogue's activation.
 LLB_EXPORT int llb_gemm_simt(const void* A, int a_dtype, const void* W, const void* bias, int w_dtype, void* out,
-                             float* residual, int epilogue, int M, int N, int K, cudaStream_t stream) {
+                             float* residual, int epilogue, int M, int N, int K, void* scratch, long long scratch_bytes,
+                             int* error_flag, cudaStream_t stream) {
     return llb_gemm_simt_glu(A, a_dtype, W, bias, w_dtype, out, residual, epilogue, M, N, K, LLB_GLU_SILU, 1.0f, 0.0f, 0.0f,
-                             stream);
+                             scratch, scratch_bytes, error_flag, stream);
 }

@@ -180,15 +180,18 @@ def _glu_args(glu):
 
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], epilogue: int,
               out: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None, glu=None) -> None:
-    """CUDA-core contraction a[M,K] @ w[N,K]^T with a fused epilogue (see EPI_*).  ``glu = (kind, alpha, limit,
+    """Contraction a[M,K] @ w[N,K]^T with a fused epilogue (see EPI_*) on CUDA cores, or with 32-bit accuracy on the tensor cores
+    (floats, more than a few rows).  ``glu = (kind, alpha, limit,
     up_shift)`` names the gated activation of the EPI_SWIGLU epilogue (see :func:`glu_act`; default SiLU)."""
     M, K = a.shape
     N, K2 = w.shape
     if K != K2:
         raise KernelError(f"gemm: a is {tuple(a.shape)} but w is {tuple(w.shape)}")
     _check_epilogue_args(a, N, M, bias, epilogue, out, residual)
-    _check(lib().llb_gemm_simt_glu(_ptr(a), _dt(a), _ptr(w), _ptr(bias), _dt(w), _ptr(out), _ptr(residual),
-                                   epilogue, M, N, K, *_glu_args(glu), _stream()))
+    need = lib().llb_gemm_simt_scratch_bytes(_dt(a), _dt(w), M, N, K)
+    scratch = torch.empty(need, dtype=torch.uint8, device=a.device) if need else None
+    _check(lib().llb_gemm_simt_glu(_ptr(a), _dt(a), _ptr(w), _ptr(bias), _dt(w), _ptr(out), _ptr(residual), epilogue, M, N, K,
+                                   *_glu_args(glu), _ptr(scratch), need, _ptr(async_error_flag(a.device)), _stream()))
 
 
 def _check_epilogue_args(a, N, M, bias, epilogue, out, residual) -> None:

@@ -37,7 +37,8 @@ int llb_gemm_decode(const void* W, const void* a_bf16, const float* x, const int
                     int Hkv, int hd, void* q_out, void* k_cache, void* v_cache, float* acc_scratch, long long scratch_floats,
                     int* counters, int* error_flag, cudaStream_t stream);
 int llb_gemm_simt(const void* A, int a_dtype, const void* W, const void* bias, int w_dtype, void* out, float* residual,
-                  int epilogue, int M, int N, int K, cudaStream_t stream);
+                  int epilogue, int M, int N, int K, void* scratch, long long scratch_bytes, int* error_flag, cudaStream_t stream);
+long long llb_gemm_simt_scratch_bytes(int a_dtype, int w_dtype, int M, int N, int K);
 int llb_gemm_tcgen05(const void* A, const void* W, const float* bias, void* out, float* residual, int epilogue, int M, int N,
                      int K, int split_k, float* partials, int* counters, int* error_flag, cudaStream_t stream);
 long long llb_gemm_tcgen05_partial_floats(int M, int N, int split_k);
@@ -145,8 +146,11 @@ struct Exec {
             used = mark;       // the kernels of the stream run in order: the next one may reuse the partials
             return rc;
         }
+        const long long mark = used, bytes = llb_gemm_simt_scratch_bytes(m.act_dtype, m.act_dtype, M, N, K);
+        void* scratch = bytes > 0 ? take(bytes) : nullptr;
+        used = mark;           // the kernels of the stream run in order: the next one may reuse it
         if (dry) return 0;
-        return llb_gemm_simt(x, m.act_dtype, w, bias, m.act_dtype, out, residual, epi, M, N, K, s.stream);
+        return llb_gemm_simt(x, m.act_dtype, w, bias, m.act_dtype, out, residual, epi, M, N, K, scratch, bytes, s.error_flag, s.stream);
     }
 
     // ---- the step's rotary tables (parts/rotary.py: once per step and set of frequencies) ----------------------------------

@@ -10,7 +10,11 @@ pytestmark = pytest.mark.gpu
 # of 32 to sums that are cut among the blocks of a cluster (few tiles over a long K)
 SHAPES = [(4, 66, 36), (5, 66, 36), (9, 64, 4), (16, 63, 28), (17, 65, 32), (32, 2, 36), (33, 129, 100), (64, 128, 896), (65, 66, 4864), (389, 896, 1536),
           # five to eight rows at the edges of what the row-streaming kernel takes of them: slices of K, tiles of features times rows
-          (5, 4096, 96), (5, 4097, 96), (8, 64, 64), (8, 64, 68), (8, 64, 256), (9, 64, 256), (8, 64, 260), (7, 9473, 512), (8, 9473, 512), (5, 11361, 512)]
+          (5, 4096, 96), (5, 4097, 96), (8, 64, 64), (8, 64, 68), (8, 64, 256), (9, 64, 256), (8, 64, 260), (7, 9473, 512), (8, 9473, 512), (5, 11361, 512),
+          # on the tensor cores: the smallest row counts and work that go there and those beside them, ends of slices of 32 and of
+          # tiles of 128 features and 160 tokens, odd features, K cut among 2, 4 and 8 blocks
+          (17, 6144, 512), (16, 6144, 512), (32, 6143, 512), (33, 1221, 1024), (33, 1220, 1024), (64, 641, 2052), (160, 896, 896), (161, 8200, 68), (320, 129, 2020),
+          (400, 517, 516), (1000, 300, 420), (389, 37889, 36), (389, 896, 4864), (389, 1500, 4)]
 
 
 @pytest.mark.parametrize("M,N,K", SHAPES)
@@ -31,6 +35,30 @@ def test_float_contraction(ops, M, N, K, epi):  # noqa: F811
         size, bound = size[:, 0::2] + size[:, 1::2], bound[:, 0::2] + bound[:, 1::2]
         bound = bound * size * 1.2 + 1e-6 * (1.0 + want.abs())
     assert bool(((got - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(161, 1030, 516), (40, 128, 10240)])          # a tile's K in one block, and cut among eight
+def test_float_contraction_of_what_bf16_does_not_hold(ops, M, N, K):  # noqa: F811
+    """Infinities, NaN, values that round to infinity in bf16 and sums beyond the floats, among ordinary rows, on the tensor cores."""
+    assert ops.lib().llb_gemm_simt_scratch_bytes(0, 0, M, N, K) > 0
+    a, w = rnd((M, K), torch.float32, 1), rnd((N, K), torch.float32, 2, 0.2)
+    w = torch.where(w.abs() < 1e-3, torch.full_like(w, 1e-3), w)          # (no zero: infinity times it is NaN)
+    a[0, K // 2], a[1, 3], a[2, K - 1], a[3, :2] = float("inf"), -float("inf"), float("nan"), float("inf")
+    a[4], a[4, 5], a[5, 7], a[6] = 0.0, 3.4e38, -3.39e38, 3.3e38
+    a[7] *= 1e-37
+    w[9, 0], w[9, 1] = 1.0, -1.0          # row 3 meets infinity minus infinity there
+    out = torch.full((M, N), 7.0, device=dev())
+    ops.gemm_simt(a, w, None, ops.EPI_STORE, out)
+    want, got = (a.double() @ w.double().t()).cpu(), out.double().cpu()
+    size = (a.abs().double() @ w.abs().double().t()).cpu()
+    bound = (K + 4) * 2.0 ** -24 * size + K * 2.0 ** -133          # (a third part below bf16's smallest number is lost)
+    safe = torch.isfinite(want) & (size < 3.0e38)                  # (no order of the sum passes the largest float)
+    assert bool(((got - want).abs()[safe] <= bound[safe]).all()) and int(safe.sum()) >= (M - 6) * N
+    assert bool((got[:2] == want[:2]).all()) and bool(torch.isnan(got[2]).all()) and bool(torch.isnan(got[3, 9]))
+    same_sign = (w[:, 0] * w[:, 1] > 0).cpu()
+    assert bool((got[3][same_sign] == want[3][same_sign]).all())
+    beyond = torch.isfinite(want[6]) & (want[6].abs() < 3.0e38) | torch.isnan(got[6]) | torch.isinf(got[6])
+    assert bool(beyond.all())          # sums that pass the largest float on the way are infinite or NaN, as with FFMA
 
 
 @pytest.mark.parametrize("Hq,Hkv,hd", [(14, 2, 64), (3, 3, 128), (9, 1, 64), (12, 2, 128)])
