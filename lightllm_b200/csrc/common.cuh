@@ -89,6 +89,29 @@ static inline LlbGluArgs llb_glu_silu() { return LlbGluArgs{LLB_GLU_SILU, 1.0f, 
 
 static inline int llb_ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// Launches of a chain of short kernels: the kernel may be set up while the one before it in the stream still runs, and begins with
+// llb_after_previous().  That waits until the kernel before has completed and its writes are visible, and only then lets the next
+// one be set up: whatever is done there before its own wait (a contraction asks for its weights) follows everything that was
+// launched before this kernel.  Measured: four prompts and 24 decoding steps of 81 short launches each, 12.75 -> 11.86 ms.
+template <typename... KArgs, typename... Args>
+static inline void llb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);          // (a failure is the runtime's last error, which llb_check_launch reads)
+}
+__device__ __forceinline__ void llb_after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // The first key position that a query at position qpos sees, under the one `window` argument of the attention kernels:
 //   window > 0   the latest `window` positions, the query's own included (a sliding window);
 //   window < 0   the positions of the query's own block of -window positions, blocks counted from position 0 of the

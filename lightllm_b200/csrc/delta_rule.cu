@@ -66,6 +66,7 @@ __device__ __forceinline__ float delta_head_log_decay(const DeltaParams& p, size
 
 template <int NR, int DG, bool HEAD>
 __global__ void __launch_bounds__(256) delta_rule_kernel(DeltaParams p) {
+    llb_after_previous();
     extern __shared__ __align__(16) float sm[];
     constexpr int PADF = delta_pad(NR, DG);
     constexpr int DPAD = DG * (NR + PADF);
@@ -182,6 +183,7 @@ __host__ __device__ inline long long delta_block_floats(int dpad) {
 
 template <bool HEAD>
 __global__ void __launch_bounds__(256) delta_blocks_prepare_kernel(DeltaParams p, int num_spans) {
+    llb_after_previous();
     extern __shared__ __align__(16) float sm[];
     constexpr int C = DELTA_STAGE;
     const int dim = p.dim, h = blockIdx.y;
@@ -275,6 +277,7 @@ __global__ void __launch_bounds__(256) delta_blocks_prepare_kernel(DeltaParams p
 
 template <int NR, int DG>
 __global__ void __launch_bounds__(64) delta_rule_blocked_kernel(DeltaParams p) {
+    llb_after_previous();
     extern __shared__ __align__(16) float sm[];
     constexpr int C = DELTA_STAGE;
     constexpr int PADF = delta_pad(NR, DG);
@@ -456,7 +459,7 @@ int launch_delta_as(const DeltaParams& p0, int num_spans, cudaStream_t stream) {
             if (e != cudaSuccess) return llb_fail("delta_rule: %s", cudaGetErrorString(e));
         }
         p.nr = NR; p.dg = DG;
-        delta_blocks_prepare_kernel<HEAD><<<dim3(p.max_blocks, p.H), 256, pre_bytes, stream>>>(p, num_spans);
+        llb_launch(delta_blocks_prepare_kernel<HEAD>, dim3(p.max_blocks, p.H), 256, pre_bytes, stream, p, num_spans);
         int rc = llb_check_launch("delta_blocks_prepare");
         if (rc) return rc;
         const size_t stage = ((size_t)delta_block_floats(DG * (NR + PADF)) + C * p.EV + C + 3) & ~(size_t)3;
@@ -466,14 +469,14 @@ int launch_delta_as(const DeltaParams& p0, int num_spans, cudaStream_t stream) {
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
             if (e != cudaSuccess) return llb_fail("delta_rule: %s", cudaGetErrorString(e));
         }
-        delta_rule_blocked_kernel<NR, DG><<<grid_b, threads_b, bytes, stream>>>(p);
+        llb_launch(delta_rule_blocked_kernel<NR, DG>, grid_b, threads_b, bytes, stream, p);
         return llb_check_launch("delta_rule_blocked");
     }
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(delta_rule_kernel<NR, DG, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return llb_fail("delta_rule: %s", cudaGetErrorString(e));
     }
-    delta_rule_kernel<NR, DG, HEAD><<<grid, threads, smem, stream>>>(p);
+    llb_launch(delta_rule_kernel<NR, DG, HEAD>, grid, threads, smem, stream, p);
     return llb_check_launch("delta_rule");
 }
 
@@ -506,6 +509,7 @@ constexpr int LR_ROWS = 16;
 
 template <typename TX, typename TW, typename TO>
 __global__ void __launch_bounds__(256) low_rank_up_kernel(LowRankParams p, int T) {
+    llb_after_previous();
     extern __shared__ __align__(16) float xs[];      // [LR_ROWS][R4]
     const int R4 = (p.R + 3) & ~3;
     const int t0 = blockIdx.y * LR_ROWS;
@@ -565,6 +569,7 @@ __device__ __forceinline__ float low_rank_finish(const LowRankParams& p, int n, 
 // and a step's few thousand outputs are spread over a hundred blocks instead of four.
 template <typename TX, typename TW, typename TO>
 __global__ void __launch_bounds__(256) low_rank_up_few_rows_kernel(LowRankParams p, int T) {
+    llb_after_previous();
     extern __shared__ __align__(16) float xs[];      // [T][R]
     for (int i = threadIdx.x; i < T * p.R; i += blockDim.x) {
         const int tl = i / p.R, r = i - tl * p.R;
@@ -593,14 +598,14 @@ int launch_low_rank(const LowRankParams& p, int T, int out_dtype, cudaStream_t s
     if (T <= LR_ROWS) {
         const dim3 grid_f((p.N + 7) / 8);
         const size_t smem_f = (size_t)T * p.R * sizeof(float);
-        if (out_dtype == LLB_F32) low_rank_up_few_rows_kernel<TX, TW, float><<<grid_f, 256, smem_f, stream>>>(p, T);
-        else low_rank_up_few_rows_kernel<TX, TW, __nv_bfloat16><<<grid_f, 256, smem_f, stream>>>(p, T);
+        if (out_dtype == LLB_F32) llb_launch(low_rank_up_few_rows_kernel<TX, TW, float>, grid_f, 256, smem_f, stream, p, T);
+        else llb_launch(low_rank_up_few_rows_kernel<TX, TW, __nv_bfloat16>, grid_f, 256, smem_f, stream, p, T);
         return llb_check_launch("low_rank_up_few_rows");
     }
     const dim3 grid((p.N + 255) / 256, (T + LR_ROWS - 1) / LR_ROWS);
     const size_t smem = (size_t)LR_ROWS * ((p.R + 3) & ~3) * sizeof(float);
-    if (out_dtype == LLB_F32) low_rank_up_kernel<TX, TW, float><<<grid, 256, smem, stream>>>(p, T);
-    else low_rank_up_kernel<TX, TW, __nv_bfloat16><<<grid, 256, smem, stream>>>(p, T);
+    if (out_dtype == LLB_F32) llb_launch(low_rank_up_kernel<TX, TW, float>, grid, 256, smem, stream, p, T);
+    else llb_launch(low_rank_up_kernel<TX, TW, __nv_bfloat16>, grid, 256, smem, stream, p, T);
     return llb_check_launch("low_rank_up");
 }
 

@@ -9,6 +9,7 @@ namespace {
 // dst[i] = (ACCUMULATE ? dst[i] : 0) + src[i], converted through float.
 template <typename TS, typename TD, bool ACCUMULATE>
 __global__ void cast_add_kernel(const TS* __restrict__ src, TD* __restrict__ dst, long long n) {
+    llb_after_previous();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         float v = llb_to_float(src[i]);
@@ -22,15 +23,16 @@ int launch_cast(const void* src, void* dst, long long n, int accumulate, cudaStr
     const int threads = 256;
     const int blocks = (int)((n + threads - 1) / threads < 1184 ? (n + threads - 1) / threads : 1184);
     if (accumulate)
-        cast_add_kernel<TS, TD, true><<<blocks, threads, 0, stream>>>((const TS*)src, (TD*)dst, n);
+        llb_launch(cast_add_kernel<TS, TD, true>, blocks, threads, 0, stream, (const TS*)src, (TD*)dst, n);
     else
-        cast_add_kernel<TS, TD, false><<<blocks, threads, 0, stream>>>((const TS*)src, (TD*)dst, n);
+        llb_launch(cast_add_kernel<TS, TD, false>, blocks, threads, 0, stream, (const TS*)src, (TD*)dst, n);
     return llb_check_launch("cast_add");
 }
 
 // out[t, 0:D] = a[t, :] (float, converted), out[t, D:2D] = b[t, :] (already in out's dtype)
 template <typename TO>
 __global__ void cast_concat_kernel(const float* __restrict__ a, const TO* __restrict__ b, TO* __restrict__ out, long long T, int D) {
+    llb_after_previous();
     const long long n = T * D, stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const long long t = i / D;
@@ -48,9 +50,9 @@ LLB_EXPORT int llb_cast_concat(const float* a, const void* b, void* out, int dty
     LLB_REQUIRE(T > 0 && D > 0 && a && b && out, "cast_concat: bad arguments");
     const long long n = T * D;
     const int blocks = (int)((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
-    if (dtype == LLB_F32) cast_concat_kernel<float><<<blocks, 256, 0, stream>>>(a, (const float*)b, (float*)out, T, D);
+    if (dtype == LLB_F32) llb_launch(cast_concat_kernel<float>, blocks, 256, 0, stream, a, (const float*)b, (float*)out, T, D);
     else if (dtype == LLB_BF16)
-        cast_concat_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(a, (const __nv_bfloat16*)b, (__nv_bfloat16*)out, T, D);
+        llb_launch(cast_concat_kernel<__nv_bfloat16>, blocks, 256, 0, stream, a, (const __nv_bfloat16*)b, (__nv_bfloat16*)out, T, D);
     else return llb_fail("cast_concat: unknown dtype %d", dtype);
     return llb_check_launch("cast_concat");
 }
@@ -76,6 +78,7 @@ namespace {
 template <typename TW>
 __global__ void __launch_bounds__(256) rmsnorm_add_kernel(const float* __restrict__ x, const TW* __restrict__ w,
                                                           float* __restrict__ dst, long long T, int D, float eps, float scale) {
+    llb_after_previous();
     const int lane = threadIdx.x & 31;
     const long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= T) return;
@@ -93,6 +96,7 @@ constexpr int NORM_SUM_MAX = 4;
 template <int V>
 __global__ void __launch_bounds__(256) rmsnorm_sum_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ dst,
                                                           int n, long long T, int D, float eps) {
+    llb_after_previous();
     __shared__ float part[NORM_SUM_MAX][8];
     const long long t = blockIdx.x;
     const int warps = blockDim.x >> 5;
@@ -138,6 +142,7 @@ __global__ void __launch_bounds__(256) rmsnorm_sum_kernel(const float* __restric
 template <int NV>
 __global__ void __launch_bounds__(256) rmsnorm_sum_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                float* __restrict__ dst, int n, long long T, int D, float eps) {
+    llb_after_previous();
     __shared__ float part[NORM_SUM_MAX][8];
     const long long t = blockIdx.x;
     const int warps = blockDim.x >> 5;
@@ -187,12 +192,14 @@ __global__ void __launch_bounds__(256) rmsnorm_sum_rows_kernel(const float* __re
 
 // x[t, d] = (x[t, d] + e[t, d]) + v[d]
 __global__ void add_sum_row_kernel(float* __restrict__ x, const float* __restrict__ e, const float* __restrict__ v, long long n, int D) {
+    llb_after_previous();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) x[i] = (x[i] + e[i]) + v[i % D];
 }
 
 // y[i] += a * x[i]; optionally the new y once more in bf16
 __global__ void axpy_kernel(const float* __restrict__ x, float* __restrict__ y, __nv_bfloat16* __restrict__ copy, long long n, float a) {
+    llb_after_previous();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const float v = fmaf(a, x[i], y[i]);
@@ -204,12 +211,14 @@ __global__ void axpy_kernel(const float* __restrict__ x, float* __restrict__ y, 
 // x[t, d] += v[d]
 template <typename TV>
 __global__ void add_row_kernel(float* __restrict__ x, const TV* __restrict__ v, long long n, int D) {
+    llb_after_previous();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) x[i] += llb_to_float(v[i % D]);
 }
 
 // x[i] = cap * tanh(x[i] / cap)
 __global__ void softcap_kernel(float* __restrict__ x, long long n, float cap) {
+    llb_after_previous();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) x[i] = cap * tanhf(x[i] / cap);
 }
@@ -226,9 +235,9 @@ LLB_EXPORT int llb_rmsnorm_add(const float* x, const void* w, int w_dtype, float
     // a warp a row; few rows get a block of one warp each, so that they spread over the SMs
     const int threads = T >= 2048 ? 256 : 32;
     const unsigned blocks = (unsigned)((T + threads / 32 - 1) / (threads / 32));
-    if (w_dtype == LLB_F32) rmsnorm_add_kernel<float><<<blocks, threads, 0, stream>>>(x, (const float*)w, dst, T, D, eps, scale);
+    if (w_dtype == LLB_F32) llb_launch(rmsnorm_add_kernel<float>, blocks, threads, 0, stream, x, (const float*)w, dst, T, D, eps, scale);
     else if (w_dtype == LLB_BF16)
-        rmsnorm_add_kernel<__nv_bfloat16><<<blocks, threads, 0, stream>>>(x, (const __nv_bfloat16*)w, dst, T, D, eps, scale);
+        llb_launch(rmsnorm_add_kernel<__nv_bfloat16>, blocks, threads, 0, stream, x, (const __nv_bfloat16*)w, dst, T, D, eps, scale);
     else return llb_fail("rmsnorm_add: unknown weight dtype %d", w_dtype);
     return llb_check_launch("rmsnorm_add");
 }
@@ -243,14 +252,14 @@ LLB_EXPORT int llb_rmsnorm_sum(const float* x, const float* w, float* dst, int n
     const bool vec = D % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0 && (uintptr_t)dst % 16 == 0;
     if (vec && D <= 2048) {
         const int quads = D / 4;
-        if (quads <= 256) rmsnorm_sum_rows_kernel<1><<<(unsigned)T, (quads + 31) / 32 * 32, 0, stream>>>(x, w, dst, n, T, D, eps);
-        else rmsnorm_sum_rows_kernel<2><<<(unsigned)T, 256, 0, stream>>>(x, w, dst, n, T, D, eps);
+        if (quads <= 256) llb_launch(rmsnorm_sum_rows_kernel<1>, (unsigned)T, (quads + 31) / 32 * 32, 0, stream, x, w, dst, n, T, D, eps);
+        else llb_launch(rmsnorm_sum_rows_kernel<2>, (unsigned)T, 256, 0, stream, x, w, dst, n, T, D, eps);
         return llb_check_launch("rmsnorm_sum");
     }
     const int per = vec ? D / 4 : D;
     const int threads = per <= 64 ? 64 : per <= 128 ? 128 : 256;
-    if (vec) rmsnorm_sum_kernel<4><<<(unsigned)T, threads, 0, stream>>>(x, w, dst, n, T, D, eps);
-    else rmsnorm_sum_kernel<1><<<(unsigned)T, threads, 0, stream>>>(x, w, dst, n, T, D, eps);
+    if (vec) llb_launch(rmsnorm_sum_kernel<4>, (unsigned)T, threads, 0, stream, x, w, dst, n, T, D, eps);
+    else llb_launch(rmsnorm_sum_kernel<1>, (unsigned)T, threads, 0, stream, x, w, dst, n, T, D, eps);
     return llb_check_launch("rmsnorm_sum");
 }
 
@@ -259,7 +268,7 @@ LLB_EXPORT int llb_add_sum_row(float* x, const float* e, const float* v, long lo
     if (T == 0) return 0;
     LLB_REQUIRE(T > 0 && D > 0 && x && e && v, "add_sum_row: bad arguments");
     const long long n = T * D;
-    add_sum_row_kernel<<<grid_for(n), 256, 0, stream>>>(x, e, v, n, D);
+    llb_launch(add_sum_row_kernel, grid_for(n), 256, 0, stream, x, e, v, n, D);
     return llb_check_launch("add_sum_row");
 }
 
@@ -267,7 +276,7 @@ LLB_EXPORT int llb_add_sum_row(float* x, const float* e, const float* v, long lo
 LLB_EXPORT int llb_axpy(const float* x, float* y, void* copy, long long n, float a, cudaStream_t stream) {
     if (n == 0) return 0;
     LLB_REQUIRE(n > 0 && x && y, "axpy: bad arguments");
-    axpy_kernel<<<grid_for(n), 256, 0, stream>>>(x, y, (__nv_bfloat16*)copy, n, a);
+    llb_launch(axpy_kernel, grid_for(n), 256, 0, stream, x, y, (__nv_bfloat16*)copy, n, a);
     return llb_check_launch("axpy");
 }
 
@@ -276,8 +285,8 @@ LLB_EXPORT int llb_add_row(float* x, const void* v, int v_dtype, long long T, in
     if (T == 0) return 0;
     LLB_REQUIRE(T > 0 && D > 0 && x && v, "add_row: bad arguments");
     const long long n = T * D;
-    if (v_dtype == LLB_F32) add_row_kernel<float><<<grid_for(n), 256, 0, stream>>>(x, (const float*)v, n, D);
-    else if (v_dtype == LLB_BF16) add_row_kernel<__nv_bfloat16><<<grid_for(n), 256, 0, stream>>>(x, (const __nv_bfloat16*)v, n, D);
+    if (v_dtype == LLB_F32) llb_launch(add_row_kernel<float>, grid_for(n), 256, 0, stream, x, (const float*)v, n, D);
+    else if (v_dtype == LLB_BF16) llb_launch(add_row_kernel<__nv_bfloat16>, grid_for(n), 256, 0, stream, x, (const __nv_bfloat16*)v, n, D);
     else return llb_fail("add_row: unknown dtype %d", v_dtype);
     return llb_check_launch("add_row");
 }
@@ -286,6 +295,6 @@ LLB_EXPORT int llb_add_row(float* x, const void* v, int v_dtype, long long T, in
 LLB_EXPORT int llb_softcap(float* x, long long n, float cap, cudaStream_t stream) {
     if (n == 0) return 0;
     LLB_REQUIRE(n > 0 && x && cap > 0.0f, "softcap: bad arguments");
-    softcap_kernel<<<grid_for(n), 256, 0, stream>>>(x, n, cap);
+    llb_launch(softcap_kernel, grid_for(n), 256, 0, stream, x, n, cap);
     return llb_check_launch("softcap");
 }

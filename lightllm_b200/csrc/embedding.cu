@@ -10,6 +10,7 @@ template <typename TW, typename TC>
 __global__ void embedding_kernel(const int* __restrict__ ids, const TW* __restrict__ table,
                                  float* __restrict__ out, int D, int V, int* __restrict__ err, float scale,
                                  TC* __restrict__ copy) {
+    llb_after_previous();
     const int t = blockIdx.x;
     const int id = ids[t];
     const bool ok = id >= 0 && id < V;
@@ -30,9 +31,9 @@ LLB_EXPORT int llb_embedding(const int* ids, const void* table, int table_dtype,
     LLB_REQUIRE(T > 0 && D > 0 && V > 0, "embedding: bad sizes T=%d D=%d V=%d", T, D, V);
     const int threads = D >= 256 ? 256 : 128;
     if (table_dtype == LLB_F32)
-        embedding_kernel<float, float><<<T, threads, 0, stream>>>(ids, (const float*)table, out, D, V, err, 1.0f, nullptr);
+        llb_launch(embedding_kernel<float, float>, T, threads, 0, stream, ids, (const float*)table, out, D, V, err, 1.0f, nullptr);
     else if (table_dtype == LLB_BF16)
-        embedding_kernel<__nv_bfloat16, float><<<T, threads, 0, stream>>>(ids, (const __nv_bfloat16*)table, out, D, V, err,
+        llb_launch(embedding_kernel<__nv_bfloat16, float>, T, threads, 0, stream, ids, (const __nv_bfloat16*)table, out, D, V, err,
                                                                          1.0f, nullptr);
     else
         return llb_fail("embedding: unknown table dtype %d", table_dtype);
@@ -47,12 +48,12 @@ LLB_EXPORT int llb_embedding_copied(const int* ids, const void* table, int table
     LLB_REQUIRE(!copy || copy_dtype == LLB_F32 || copy_dtype == table_dtype, "embedding: the copy is float or has the table's dtype");
     const int threads = D >= 256 ? 256 : 128;
     if (table_dtype == LLB_F32)
-        embedding_kernel<float, float><<<T, threads, 0, stream>>>(ids, (const float*)table, out, D, V, err, scale, (float*)copy);
+        llb_launch(embedding_kernel<float, float>, T, threads, 0, stream, ids, (const float*)table, out, D, V, err, scale, (float*)copy);
     else if (table_dtype == LLB_BF16 && copy_dtype == LLB_F32)
-        embedding_kernel<__nv_bfloat16, float><<<T, threads, 0, stream>>>(ids, (const __nv_bfloat16*)table, out, D, V, err, scale,
+        llb_launch(embedding_kernel<__nv_bfloat16, float>, T, threads, 0, stream, ids, (const __nv_bfloat16*)table, out, D, V, err, scale,
                                                                          (float*)copy);
     else if (table_dtype == LLB_BF16)
-        embedding_kernel<__nv_bfloat16, __nv_bfloat16><<<T, threads, 0, stream>>>(ids, (const __nv_bfloat16*)table, out, D, V,
+        llb_launch(embedding_kernel<__nv_bfloat16, __nv_bfloat16>, T, threads, 0, stream, ids, (const __nv_bfloat16*)table, out, D, V,
                                                                                  err, scale, (__nv_bfloat16*)copy);
     else
         return llb_fail("embedding: unknown table dtype %d", table_dtype);

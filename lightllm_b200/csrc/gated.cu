@@ -7,6 +7,7 @@ namespace {
 template <typename T>
 __global__ void glu_act_kernel(const T* __restrict__ in, T* __restrict__ out, long long n, int kind, float alpha,
                                float limit, float up_shift) {
+    llb_after_previous();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const float g = llb_to_float(in[2 * i]), u = llb_to_float(in[2 * i + 1]);
@@ -21,6 +22,7 @@ __global__ void __launch_bounds__(256) head_gate_kernel(const TX* __restrict__ x
                                                         int unit_rms, float eps, int per_head, int act,
                                                         const float* __restrict__ norm_w, int norm_w_heads,
                                                         const float* __restrict__ den) {
+    llb_after_previous();
     const int lane = threadIdx.x & 31;
     const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (item >= (long long)T * H) return;
@@ -54,8 +56,7 @@ int launch_head_gate(const void* x, const void* gate, long long gate_stride, voi
                      int unit_rms, float eps, int per_head, int act, const float* norm_w, int norm_w_heads,
                      const float* den, cudaStream_t s) {
     const long long items = (long long)T * H;
-    head_gate_kernel<TX, TG, TO><<<(unsigned)((items + 7) / 8), 256, 0, s>>>(
-        (const TX*)x, (const TG*)gate, gate_stride, (TO*)out, T, H, hd, unit_rms, eps, per_head, act, norm_w,
+    llb_launch(head_gate_kernel<TX, TG, TO>, (unsigned)((items + 7) / 8), 256, 0, s, (const TX*)x, (const TG*)gate, gate_stride, (TO*)out, T, H, hd, unit_rms, eps, per_head, act, norm_w,
         norm_w_heads, den);
     return llb_check_launch("head_gate");
 }
@@ -70,9 +71,9 @@ LLB_EXPORT int llb_glu_act(const void* in, void* out, int dtype, int M, int I, i
     const long long n = (long long)M * I;
     const int blocks = (int)((n + 255) / 256 < 2368 ? (n + 255) / 256 : 2368);
     if (dtype == LLB_F32)
-        glu_act_kernel<float><<<blocks, 256, 0, stream>>>((const float*)in, (float*)out, n, kind, alpha, limit, up_shift);
+        llb_launch(glu_act_kernel<float>, blocks, 256, 0, stream, (const float*)in, (float*)out, n, kind, alpha, limit, up_shift);
     else if (dtype == LLB_BF16)
-        glu_act_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, n, kind,
+        llb_launch(glu_act_kernel<__nv_bfloat16>, blocks, 256, 0, stream, (const __nv_bfloat16*)in, (__nv_bfloat16*)out, n, kind,
                                                                    alpha, limit, up_shift);
     else
         return llb_fail("glu_act: unknown dtype %d", dtype);
@@ -118,6 +119,7 @@ template <typename TO_, typename TG>
 __global__ void __launch_bounds__(256) talk_mix_kernel(const TO_* __restrict__ o, const float* __restrict__ talk,
                                                        const TG* __restrict__ gate, long long gate_stride,
                                                        TG* __restrict__ out, int T, int H, int G, int vd, int gated) {
+    llb_after_previous();
     const int lane = threadIdx.x & 31;
     const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (item >= (long long)T * H) return;
@@ -144,6 +146,7 @@ template <typename TO_, typename TG>
 __global__ void __launch_bounds__(256) talk_mix_staged_kernel(const TO_* __restrict__ o, const float* __restrict__ talk,
                                                               const TG* __restrict__ gate, long long gate_stride,
                                                               TG* __restrict__ out, int H, int G, int vd, int gated) {
+    llb_after_previous();
     extern __shared__ float tm_smem[];
     const int n = H * G * vd;
     float* so = tm_smem;          // [H, G, vd]
@@ -177,12 +180,12 @@ int launch_talk_mix(const void* o, const float* talk, const void* gate, long lon
                     int vd, int gated, cudaStream_t stream) {
     const size_t smem = ((size_t)H * G * vd + (size_t)H * H) * sizeof(float);
     if (smem <= 48 * 1024) {
-        talk_mix_staged_kernel<TO_, TG><<<(unsigned)T, 256, smem, stream>>>((const TO_*)o, talk, (const TG*)gate, gate_stride,
+        llb_launch(talk_mix_staged_kernel<TO_, TG>, (unsigned)T, 256, smem, stream, (const TO_*)o, talk, (const TG*)gate, gate_stride,
                                                                             (TG*)out, H, G, vd, gated);
         return llb_check_launch("talk_mix_staged");
     }
     const long long items = (long long)T * H;
-    talk_mix_kernel<TO_, TG><<<(unsigned)((items + 7) / 8), 256, 0, stream>>>((const TO_*)o, talk, (const TG*)gate, gate_stride,
+    llb_launch(talk_mix_kernel<TO_, TG>, (unsigned)((items + 7) / 8), 256, 0, stream, (const TO_*)o, talk, (const TG*)gate, gate_stride,
                                                                              (TG*)out, T, H, G, vd, gated);
     return llb_check_launch("talk_mix");
 }
@@ -215,6 +218,7 @@ namespace {
 template <typename TA, typename TO>
 __global__ void __launch_bounds__(256) diff_combine_kernel(const TA* __restrict__ a, TO* __restrict__ out, long long items, int vd,
                                                            float lambda, float eps, float mult) {
+    llb_after_previous();
     const int lane = threadIdx.x & 31;
     const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (item >= items) return;
@@ -241,12 +245,12 @@ LLB_EXPORT int llb_diff_combine(const void* a, int a_dtype, void* out, int dtype
     const long long items = (long long)T * H;
     const unsigned blocks = (unsigned)((items + 7) / 8);
     if (a_dtype == LLB_F32 && dtype == LLB_F32)
-        diff_combine_kernel<float, float><<<blocks, 256, 0, stream>>>((const float*)a, (float*)out, items, vd, lambda, eps, mult);
+        llb_launch(diff_combine_kernel<float, float>, blocks, 256, 0, stream, (const float*)a, (float*)out, items, vd, lambda, eps, mult);
     else if (a_dtype == LLB_F32 && dtype == LLB_BF16)
-        diff_combine_kernel<float, __nv_bfloat16><<<blocks, 256, 0, stream>>>((const float*)a, (__nv_bfloat16*)out, items, vd,
+        llb_launch(diff_combine_kernel<float, __nv_bfloat16>, blocks, 256, 0, stream, (const float*)a, (__nv_bfloat16*)out, items, vd,
                                                                              lambda, eps, mult);
     else if (a_dtype == LLB_BF16 && dtype == LLB_BF16)
-        diff_combine_kernel<__nv_bfloat16, __nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)a, (__nv_bfloat16*)out,
+        llb_launch(diff_combine_kernel<__nv_bfloat16, __nv_bfloat16>, blocks, 256, 0, stream, (const __nv_bfloat16*)a, (__nv_bfloat16*)out,
                                                                                      items, vd, lambda, eps, mult);
     else
         return llb_fail("diff_combine: unsupported dtypes %d, %d", a_dtype, dtype);

@@ -219,6 +219,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    llb_after_previous();          // (the block has its tensor memory: the next kernel's blocks may take what is left)
 
     if (nkb > 0) {
         if (warp == 0) {
@@ -891,7 +892,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, di
                                               cudaGetErrorString(e));
         configured = true;
     }
-    gemm_tcgen05_kernel<BN, EPI, SWAP><<<grid, NUM_THREADS, smem, stream>>>(ma, mb, p);
+    llb_launch(gemm_tcgen05_kernel<BN, EPI, SWAP>, grid, dim3(NUM_THREADS), smem, stream, ma, mb, p);
     return llb_check_launch("gemm_tcgen05");
 }
 

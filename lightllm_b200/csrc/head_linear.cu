@@ -47,6 +47,7 @@ constexpr int HL_ROWS = 16;     // tokens per block
 
 template <typename T>
 __global__ void __launch_bounds__(256) head_linear_kernel(HeadLinearParams p) {
+    llb_after_previous();
     extern __shared__ float xs[];          // [HL_ROWS][in]
     const int in = p.in, on = p.on;
     const int t0 = blockIdx.x * HL_ROWS, h = blockIdx.y;
@@ -83,6 +84,7 @@ constexpr int HL_OT = 64, HL_KB = 64, HL_PITCH = HL_KB * 2 + 16;
 
 template <int RG>
 __global__ void __launch_bounds__(128) head_linear_mma_kernel(HeadLinearParams p) {
+    llb_after_previous();
     constexpr int MR = 16 * RG, CW = 4 / RG, NT = HL_OT / CW / 8;          // n-tiles of 8 outputs a warp
     __shared__ __align__(16) uint8_t xs[2][MR * HL_PITCH];
     __shared__ __align__(16) uint8_t ws[2][HL_OT * HL_PITCH];
@@ -181,16 +183,16 @@ LLB_EXPORT int llb_head_linear_rotated(const void* x, long long x_stride, int x_
     if (dtype == LLB_BF16 && in % 8 == 0 && x_stride % 8 == 0 && x_off % 8 == 0 && x_head % 8 == 0 && (uintptr_t)x % 16 == 0 &&
         (uintptr_t)w % 16 == 0 && (uintptr_t)out % 16 == 0) {
         const int oz = (on + HL_OT - 1) / HL_OT;
-        if (T <= 16) head_linear_mma_kernel<1><<<dim3((T + 15) / 16, H, oz), 128, 0, stream>>>(p);
-        else head_linear_mma_kernel<4><<<dim3((T + 63) / 64, H, oz), 128, 0, stream>>>(p);
+        if (T <= 16) llb_launch(head_linear_mma_kernel<1>, dim3((T + 15) / 16, H, oz), 128, 0, stream, p);
+        else llb_launch(head_linear_mma_kernel<4>, dim3((T + 63) / 64, H, oz), 128, 0, stream, p);
         return llb_check_launch("head_linear_mma");
     }
     const size_t smem = (size_t)HL_ROWS * in * sizeof(float);
     LLB_REQUIRE(smem <= 48 * 1024, "head_linear: %d input features per head need %zu bytes of shared memory", in, smem);
     const dim3 grid((T + HL_ROWS - 1) / HL_ROWS, H);
     // zero rows beyond the tile's end are never read: acc of such rows is dropped
-    if (dtype == LLB_F32) head_linear_kernel<float><<<grid, 256, smem, stream>>>(p);
-    else if (dtype == LLB_BF16) head_linear_kernel<__nv_bfloat16><<<grid, 256, smem, stream>>>(p);
+    if (dtype == LLB_F32) llb_launch(head_linear_kernel<float>, grid, 256, smem, stream, p);
+    else if (dtype == LLB_BF16) llb_launch(head_linear_kernel<__nv_bfloat16>, grid, 256, smem, stream, p);
     else return llb_fail("head_linear: unknown dtype %d", dtype);
     return llb_check_launch("head_linear");
 }

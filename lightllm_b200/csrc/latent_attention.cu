@@ -42,6 +42,7 @@ struct LatentPrepareParams {
 // One block a token: RMS norms of both latents (float), the rotation, the cache row.
 template <typename T>
 __global__ void __launch_bounds__(128) latent_prepare_kernel(LatentPrepareParams p) {
+    llb_after_previous();
     const int t = blockIdx.x;
     const T* row = (const T*)p.src + (size_t)t * p.stride;
     float sq = 0.0f, sc = 0.0f;
@@ -118,6 +119,7 @@ __device__ __forceinline__ void l_cluster_sync() {          // a hardware barrie
 // RG: row groups of 16 pairs; NTW: the most value n-tiles (8 columns each) a warp owns (even); CLUSTER: the key range is cut.
 template <int RG, int NTW, bool CLUSTER>
 __global__ void __launch_bounds__(LTHREADS) latent_attention_kernel(LatentParams p) {
+    llb_after_previous();
     constexpr int CW = 8 / RG, MR = 16 * RG, NK = 8 / CW;          // NK: key n-tiles (8 keys each) a warp scores
     extern __shared__ __align__(16) uint8_t smem[];
     const int pitch = p.pitch, H = p.H, W = p.W;
@@ -402,13 +404,15 @@ int launch_latent_as(const LatentParams& p, int blocks, cudaStream_t stream) {
     cfg.blockDim = dim3(LTHREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = CLUSTER ? p.nsplit : 1;
-    attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = CLUSTER ? p.nsplit : 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = CLUSTER ? 1 : 0;
+    cfg.numAttrs = CLUSTER ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, latent_attention_kernel<RG, NTW, CLUSTER>, p);
     if (e != cudaSuccess) return llb_fail("latent_attention: launch failed: %s", cudaGetErrorString(e));
     return llb_check_launch("latent_attention");
@@ -446,8 +450,8 @@ LLB_EXPORT int llb_latent_prepare(const void* src, int dtype, long long stride, 
     p.src = src; p.stride = stride; p.q_off = q_off; p.c_off = c_off; p.rot_off = rot_off; p.q_rank = q_rank; p.r = r; p.rd = rd;
     p.interleaved = interleaved ? 1 : 0; p.q_w = q_w; p.c_w = c_w; p.inv_freq = inv_freq; p.positions = positions; p.slots = slots;
     p.q_out = q_out; p.cache = cache; p.eps = eps;
-    if (dtype == LLB_F32) latent_prepare_kernel<float><<<T, 128, 0, stream>>>(p);
-    else if (dtype == LLB_BF16) latent_prepare_kernel<__nv_bfloat16><<<T, 128, 0, stream>>>(p);
+    if (dtype == LLB_F32) llb_launch(latent_prepare_kernel<float>, T, 128, 0, stream, p);
+    else if (dtype == LLB_BF16) llb_launch(latent_prepare_kernel<__nv_bfloat16>, T, 128, 0, stream, p);
     else return llb_fail("latent_prepare: unknown dtype %d", dtype);
     return llb_check_launch("latent_prepare");
 }

@@ -63,6 +63,8 @@ __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.
 
 __global__ void __launch_bounds__(THREADS, 1)
 latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const LatentTcParams p) {
+    // (no word to the kernel after this one: set up early it could take the tensor memory that a block of this grid still wants)
+    griddep_wait();
     __shared__ __align__(8) uint64_t bars[5 + 2 * MAX_STAGES];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_s;
@@ -364,6 +366,6 @@ LLB_EXPORT int llb_latent_attention_tcgen05(const void* q, const void* cache, vo
         if (e != cudaSuccess) return llb_fail("latent_attention_tcgen05: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
         configured = smem;
     }
-    latent_attention_tcgen05_kernel<<<(unsigned)tiles, THREADS, smem, stream>>>(mq, mk, p);
+    llb_launch(latent_attention_tcgen05_kernel, (unsigned)tiles, THREADS, smem, stream, mq, mk, p);
     return llb_check_launch("latent_attention_tcgen05");
 }

@@ -29,6 +29,7 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const float* __restrict_
                                                         const TW* __restrict__ b, TO* __restrict__ out,
                                                         const int* __restrict__ rows, int D, float eps,
                                                         __nv_bfloat16* __restrict__ copy) {
+    llb_after_previous();
     __shared__ float part[32];
     __shared__ float total;
     const int r = blockIdx.x;
@@ -103,6 +104,7 @@ __global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* __rest
                                                              const TW* __restrict__ b, TO* __restrict__ out,
                                                              const int* __restrict__ rows, int R, int D, float eps,
                                                              __nv_bfloat16* __restrict__ copy) {
+    llb_after_previous();
     const int lane = threadIdx.x & 31;
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= R) return;
@@ -151,17 +153,17 @@ int launch_ln(const float* x, const void* w, const void* b, void* out, const int
     const bool aligned = D % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0 && (uintptr_t)b % 16 == 0 &&
                          (uintptr_t)out % 16 == 0 && (uintptr_t)copy % 8 == 0;
     if (aligned && D <= 128 * 8)
-        layernorm_warp_kernel<TW, TO, 8, ACC><<<(R + 7) / 8, threads, 0, s>>>(x, (const TW*)w, (const TW*)b, (TO*)out, rows,
+        llb_launch(layernorm_warp_kernel<TW, TO, 8, ACC>, (R + 7) / 8, threads, 0, s, x, (const TW*)w, (const TW*)b, (TO*)out, rows,
                                                                               R, D, eps, copy);
     else if (aligned && D <= 128 * 16)
-        layernorm_warp_kernel<TW, TO, 16, ACC><<<(R + 7) / 8, threads, 0, s>>>(x, (const TW*)w, (const TW*)b, (TO*)out, rows,
+        llb_launch(layernorm_warp_kernel<TW, TO, 16, ACC>, (R + 7) / 8, threads, 0, s, x, (const TW*)w, (const TW*)b, (TO*)out, rows,
                                                                                R, D, eps, copy);
     else if (D <= threads * 4)
-        layernorm_kernel<TW, TO, 4, ACC><<<R, threads, 0, s>>>(x, (const TW*)w, (const TW*)b, (TO*)out, rows, D, eps, copy);
+        llb_launch(layernorm_kernel<TW, TO, 4, ACC>, R, threads, 0, s, x, (const TW*)w, (const TW*)b, (TO*)out, rows, D, eps, copy);
     else if (D <= threads * 16)
-        layernorm_kernel<TW, TO, 16, ACC><<<R, threads, 0, s>>>(x, (const TW*)w, (const TW*)b, (TO*)out, rows, D, eps, copy);
+        llb_launch(layernorm_kernel<TW, TO, 16, ACC>, R, threads, 0, s, x, (const TW*)w, (const TW*)b, (TO*)out, rows, D, eps, copy);
     else
-        layernorm_kernel<TW, TO, 0, ACC><<<R, threads, 0, s>>>(x, (const TW*)w, (const TW*)b, (TO*)out, rows, D, eps, copy);
+        llb_launch(layernorm_kernel<TW, TO, 0, ACC>, R, threads, 0, s, x, (const TW*)w, (const TW*)b, (TO*)out, rows, D, eps, copy);
     return llb_check_launch("layernorm");
 }
 

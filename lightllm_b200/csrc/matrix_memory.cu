@@ -51,6 +51,7 @@ __device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.0f) - 
 // totals meet in shared memory, and every thread folds the totals of the warps before its own onto the running maximum.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) memory_gates_kernel(GateParams p, int num_spans) {
+    llb_after_previous();
     __shared__ float wa[WARPS], wb[WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long item = blockIdx.x;
@@ -136,6 +137,7 @@ enum { MM_LOCAL = 1, MM_OUT = 3 };
 
 template <typename T, int NR, int DG, int MODE>
 __global__ void __launch_bounds__(256) matrix_memory_kernel(MemParams p) {
+    llb_after_previous();
     extern __shared__ __align__(16) float sm[];
     constexpr int PADF = DG > 1 ? 4 : 0;                 // keeps the DG threads of a column on different banks
     constexpr int DPAD = DG * (NR + PADF);
@@ -249,6 +251,7 @@ __global__ void __launch_bounds__(256) matrix_memory_kernel(MemParams p) {
 // start_0 = the request's state (zero at position 0); start_c = keeps_(c-1) * start_(c-1) + contribution_(c-1).
 // One thread per element of a head's state; the pieces of a span one after the other.
 __global__ void __launch_bounds__(256) matrix_memory_scan_kernel(MemParams p) {
+    llb_after_previous();
     const int span = blockIdx.x, h = blockIdx.y;
     const int slen = p.span_len[span];
     const int pieces = (slen + p.chunk - 1) / p.chunk;
@@ -289,8 +292,8 @@ int launch_memory_as(const MemParams& p, int num_items, cudaStream_t stream) {
     dim3 grid(num_items, p.H, llb_ceil_div(p.vdim + 1, p.EV));
     const int threads = ((p.EV * DG + 31) / 32) * 32;
     const size_t smem = ((size_t)2 * MM_STAGE * DG * (NR + PADF) + (size_t)MM_STAGE * p.EV + 2 * MM_STAGE) * sizeof(float);
-    if (p.mode == MM_LOCAL) matrix_memory_kernel<T, NR, DG, MM_LOCAL><<<grid, threads, smem, stream>>>(p);
-    else matrix_memory_kernel<T, NR, DG, MM_OUT><<<grid, threads, smem, stream>>>(p);
+    if (p.mode == MM_LOCAL) llb_launch(matrix_memory_kernel<T, NR, DG, MM_LOCAL>, grid, threads, smem, stream, p);
+    else llb_launch(matrix_memory_kernel<T, NR, DG, MM_OUT>, grid, threads, smem, stream, p);
     return llb_check_launch("matrix_memory");
 }
 
@@ -327,9 +330,9 @@ LLB_EXPORT int llb_memory_gates(const float* pre, long long T, long long pre_str
     const long long items = (long long)num_spans * H;
     LLB_REQUIRE(items < (1ll << 31), "memory_gates: too many spans and heads");
     // rows per span on average: long spans take a block of eight warps each, single tokens a warp
-    if (T >= 128ll * num_spans) memory_gates_kernel<8><<<(unsigned)items, 256, 0, stream>>>(p, num_spans);
-    else if (T >= 48ll * num_spans) memory_gates_kernel<2><<<(unsigned)items, 64, 0, stream>>>(p, num_spans);
-    else memory_gates_kernel<1><<<(unsigned)items, 32, 0, stream>>>(p, num_spans);
+    if (T >= 128ll * num_spans) llb_launch(memory_gates_kernel<8>, (unsigned)items, 256, 0, stream, p, num_spans);
+    else if (T >= 48ll * num_spans) llb_launch(memory_gates_kernel<2>, (unsigned)items, 64, 0, stream, p, num_spans);
+    else llb_launch(memory_gates_kernel<1>, (unsigned)items, 32, 0, stream, p, num_spans);
     return llb_check_launch("memory_gates");
 }
 
@@ -369,7 +372,7 @@ LLB_EXPORT int llb_matrix_memory(const void* src, int dtype, long long row_strid
             const size_t plane = (size_t)dim * (vdim + 1);
             int z = (int)((plane + 255) / 256);
             if (z > 64) z = 64;
-            matrix_memory_scan_kernel<<<dim3(num_spans, H, z), 256, 0, stream>>>(p);
+            llb_launch(matrix_memory_scan_kernel, dim3(num_spans, H, z), 256, 0, stream, p);
             rc = llb_check_launch("matrix_memory_scan");
             continue;
         }

@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const TX* __restrict__ x
                                                         int groups, int keep, float renorm_eps, int n_gate,
                                                         float* __restrict__ idw, float* __restrict__ gate_out,
                                                         const float* __restrict__ bias) {
+    llb_after_previous();
     extern __shared__ __align__(16) float sm[];  // the token's row [D4], then score [E], choice [E]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int t = blockIdx.x;
@@ -152,6 +153,7 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const TX* __restrict__ x
 // One block per (token, expert): the weight is read once, the F activations in 16-byte pieces where they are aligned.
 template <typename TA>
 __global__ void __launch_bounds__(128) moe_scale_kernel(TA* __restrict__ act, const float* __restrict__ dense, int F) {
+    llb_after_previous();
     const float wgt = dense[blockIdx.x];
     TA* a = act + (size_t)blockIdx.x * F;
     constexpr int V = 16 / sizeof(TA);
@@ -176,6 +178,7 @@ __global__ void __launch_bounds__(128) moe_scale_kernel(TA* __restrict__ act, co
 // expert's rows a pair gets depends on the order of the atomic adds; no result depends on it.
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ ids, int pairs, int E, int align, int max_tiles,
                                                         int* __restrict__ slot, int* __restrict__ tile_group) {
+    llb_after_previous();
     extern __shared__ int sh[];                  // count [E], cursor [E]
     int* count = sh;
     int* cursor = sh + E;
@@ -201,6 +204,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
 template <typename TX>
 __global__ void __launch_bounds__(128) moe_gather_kernel(const TX* __restrict__ x, const int* __restrict__ slot, int top, int D,
                                                          TX* __restrict__ xs) {
+    llb_after_previous();
     const int i = blockIdx.x;
     if (slot[i] < 0) return;
     const TX* src = x + (size_t)(i / top) * D;
@@ -221,6 +225,7 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
                                                           const float* __restrict__ weights, int top, int D,
                                                           float* __restrict__ residual, const TX* __restrict__ x,
                                                           const float* __restrict__ idw) {
+    llb_after_previous();
     const int t = blockIdx.x;
     const float wi = idw ? idw[t] : 0.0f;
     for (int d = threadIdx.x; d < D; d += blockDim.x) {
@@ -272,6 +277,7 @@ constexpr int PAIR_WARP_OUTS = PAIR_OUTS / 8;          // outputs a warp
 __global__ void __launch_bounds__(256) moe_pairs_gate_up_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                                 const int* __restrict__ ids, int top, int D, int F,
                                                                 __nv_bfloat16* __restrict__ act, LlbGluArgs glu) {
+    llb_after_previous();
     extern __shared__ __align__(16) float xs[];          // [D]
     const int pair = blockIdx.y, e = ids[pair];
     if (e < 0) return;                                   // a pair without an expert
@@ -301,6 +307,7 @@ __global__ void __launch_bounds__(256) moe_pairs_gate_up_kernel(const __nv_bfloa
 // y[pair, d] = W_down[e][d, :] . act[pair, :] with expert e's down matrix in rows e * D .. of w
 __global__ void __launch_bounds__(256) moe_pairs_down_kernel(const __nv_bfloat16* __restrict__ act, const __nv_bfloat16* __restrict__ w,
                                                              const int* __restrict__ ids, int D, int F, float* __restrict__ y) {
+    llb_after_previous();
     extern __shared__ __align__(16) float as[];          // [F]
     const int pair = blockIdx.y, e = ids[pair];
     if (e < 0) {                                         // a pair without an expert: zeros, which the combine step skips anyway
@@ -338,13 +345,11 @@ LLB_EXPORT int llb_moe_pairs_glu(const void* x, const int* ids, int pairs, int t
     if (pairs == 0) return 0;
     LLB_REQUIRE(pairs > 0 && top > 0 && x && ids && w_gate_up && w_down && act && y, "moe_pairs: bad arguments");
     LLB_REQUIRE(D > 0 && F > 0 && D % 8 == 0 && F % 8 == 0 && D <= 12288 && F <= 12288, "moe_pairs: D=%d, F=%d must be multiples of 8", D, F);
-    moe_pairs_gate_up_kernel<<<dim3((F + PAIR_OUTS - 1) / PAIR_OUTS, pairs), 256, D * sizeof(float), stream>>>(
-        (const __nv_bfloat16*)x, (const __nv_bfloat16*)w_gate_up, ids, top, D, F, (__nv_bfloat16*)act,
+    llb_launch(moe_pairs_gate_up_kernel, dim3((F + PAIR_OUTS - 1) / PAIR_OUTS, pairs), 256, D * sizeof(float), stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w_gate_up, ids, top, D, F, (__nv_bfloat16*)act,
         LlbGluArgs{glu_kind, glu_alpha, glu_limit, glu_up_shift});
     int rc = llb_check_launch("moe_pairs_gate_up");
     if (rc) return rc;
-    moe_pairs_down_kernel<<<dim3((D + PAIR_OUTS - 1) / PAIR_OUTS, pairs), 256, F * sizeof(float), stream>>>(
-        (const __nv_bfloat16*)act, (const __nv_bfloat16*)w_down, ids, D, F, y);
+    llb_launch(moe_pairs_down_kernel, dim3((D + PAIR_OUTS - 1) / PAIR_OUTS, pairs), 256, F * sizeof(float), stream, (const __nv_bfloat16*)act, (const __nv_bfloat16*)w_down, ids, D, F, y);
     return llb_check_launch("moe_pairs_down");
 }
 
@@ -359,7 +364,7 @@ LLB_EXPORT int llb_moe_sort(const int* ids, int pairs, int E, int align, int max
     if (pairs == 0) return 0;
     LLB_REQUIRE(pairs > 0 && E > 0 && E <= 4096 && align > 0 && ids && slot && tile_group, "moe_sort: bad arguments");
     LLB_REQUIRE(max_tiles >= pairs / align + E, "moe_sort: %d tiles cannot hold %d pairs of %d experts", max_tiles, pairs, E);
-    moe_sort_kernel<<<1, 1024, 2 * E * sizeof(int), stream>>>(ids, pairs, E, align, max_tiles, slot, tile_group);
+    llb_launch(moe_sort_kernel, 1, 1024, 2 * E * sizeof(int), stream, ids, pairs, E, align, max_tiles, slot, tile_group);
     return llb_check_launch("moe_sort");
 }
 
@@ -368,9 +373,9 @@ LLB_EXPORT int llb_moe_gather(const void* x, int dtype, const int* slot, int pai
                               cudaStream_t stream) {
     if (pairs == 0) return 0;
     LLB_REQUIRE(pairs > 0 && top > 0 && D > 0 && x && slot && xs, "moe_gather: bad arguments");
-    if (dtype == LLB_F32) moe_gather_kernel<float><<<pairs, 128, 0, stream>>>((const float*)x, slot, top, D, (float*)xs);
+    if (dtype == LLB_F32) llb_launch(moe_gather_kernel<float>, pairs, 128, 0, stream, (const float*)x, slot, top, D, (float*)xs);
     else if (dtype == LLB_BF16)
-        moe_gather_kernel<__nv_bfloat16><<<pairs, 128, 0, stream>>>((const __nv_bfloat16*)x, slot, top, D, (__nv_bfloat16*)xs);
+        llb_launch(moe_gather_kernel<__nv_bfloat16>, pairs, 128, 0, stream, (const __nv_bfloat16*)x, slot, top, D, (__nv_bfloat16*)xs);
     else return llb_fail("moe_gather: unknown dtype %d", dtype);
     return llb_check_launch("moe_gather");
 }
@@ -384,9 +389,9 @@ LLB_EXPORT int llb_moe_combine_identity(const float* y, const int* slot, const f
     LLB_REQUIRE(T > 0 && top >= 0 && D > 0 && residual && (top == 0 || (y && slot && weights)), "moe_combine: bad arguments");
     LLB_REQUIRE((x == nullptr) == (idw == nullptr), "moe_combine: the identity term needs both x and its weights");
     if (x_dtype == LLB_BF16 && x)
-        moe_combine_kernel<__nv_bfloat16><<<T, 256, 0, stream>>>(y, slot, weights, top, D, residual, (const __nv_bfloat16*)x, idw);
+        llb_launch(moe_combine_kernel<__nv_bfloat16>, T, 256, 0, stream, y, slot, weights, top, D, residual, (const __nv_bfloat16*)x, idw);
     else if (x_dtype == LLB_F32 || !x)
-        moe_combine_kernel<float><<<T, 256, 0, stream>>>(y, slot, weights, top, D, residual, (const float*)x, idw);
+        llb_launch(moe_combine_kernel<float>, T, 256, 0, stream, y, slot, weights, top, D, residual, (const float*)x, idw);
     else
         return llb_fail("moe_combine: unknown dtype %d", x_dtype);
     return llb_check_launch("moe_combine");
@@ -427,12 +432,11 @@ LLB_EXPORT int llb_moe_route_biased(const void* x, int x_dtype, const float* w, 
     LLB_REQUIRE(smem <= 48 * 1024, "moe_route: rows of %d numbers do not fit in shared memory", D);
     const unsigned blocks = (unsigned)T;
     if (x_dtype == LLB_F32)
-        moe_route_kernel<float><<<blocks, warps * 32, smem, stream>>>((const float*)x, w, correction, T, D, E, top, softmax,
+        llb_launch(moe_route_kernel<float>, blocks, warps * 32, smem, stream, (const float*)x, w, correction, T, D, E, top, softmax,
                                                                       renorm, scale, ids, weights, dense, real, groups, keep,
                                                                       renorm_eps, n_gate, idw, gate_out, bias);
     else if (x_dtype == LLB_BF16)
-        moe_route_kernel<__nv_bfloat16><<<blocks, warps * 32, smem, stream>>>(
-            (const __nv_bfloat16*)x, w, correction, T, D, E, top, softmax, renorm, scale, ids, weights, dense, real, groups,
+        llb_launch(moe_route_kernel<__nv_bfloat16>, blocks, warps * 32, smem, stream, (const __nv_bfloat16*)x, w, correction, T, D, E, top, softmax, renorm, scale, ids, weights, dense, real, groups,
             keep, renorm_eps, n_gate, idw, gate_out, bias);
     else
         return llb_fail("moe_route: unknown dtype %d", x_dtype);
@@ -460,8 +464,8 @@ LLB_EXPORT int llb_moe_scale(void* act, int dtype, const float* dense, int T, in
     LLB_REQUIRE(T > 0 && E > 0 && F > 0 && act && dense, "moe_scale: bad arguments");
     LLB_REQUIRE((long long)T * E < (1ll << 31), "moe_scale: too many rows");
     const unsigned blocks = (unsigned)((long long)T * E);
-    if (dtype == LLB_F32) moe_scale_kernel<float><<<blocks, 128, 0, stream>>>((float*)act, dense, F);
-    else if (dtype == LLB_BF16) moe_scale_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>((__nv_bfloat16*)act, dense, F);
+    if (dtype == LLB_F32) llb_launch(moe_scale_kernel<float>, blocks, 128, 0, stream, (float*)act, dense, F);
+    else if (dtype == LLB_BF16) llb_launch(moe_scale_kernel<__nv_bfloat16>, blocks, 128, 0, stream, (__nv_bfloat16*)act, dense, F);
     else return llb_fail("moe_scale: unknown dtype %d", dtype);
     return llb_check_launch("moe_scale");
 }

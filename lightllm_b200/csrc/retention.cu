@@ -59,6 +59,7 @@ enum { RET_LOCAL = 1, RET_OUT = 3 };
 
 template <typename T, int NR, int DG, int MODE, bool GATED>
 __global__ void __launch_bounds__(256) retention_kernel(RetParams p) {
+    llb_after_previous();
     extern __shared__ __align__(16) float sm[];
     constexpr int PADF = DG > 1 ? 4 : 0;                 // keeps the DG threads of a column on different banks
     constexpr int DPAD = DG * (NR + PADF);
@@ -195,6 +196,7 @@ __global__ void __launch_bounds__(256) retention_kernel(RetParams p) {
 // start_0 = the request's state (zero at position 0); start_c = decay^(tokens of piece c-1) * start_(c-1) + A_(c-1).
 // One thread per element of a head's state; the pieces of a span one after the other.
 __global__ void __launch_bounds__(256) retention_scan_kernel(RetParams p) {
+    llb_after_previous();
     const int span = blockIdx.x, h = blockIdx.y;
     const int slen = p.span_len[span];
     const int pieces = (slen + p.chunk - 1) / p.chunk;
@@ -243,7 +245,7 @@ int launch_retention_mode(const RetParams& p, int num_items, cudaStream_t stream
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return llb_fail("retention: cannot opt in to %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     }
-    retention_kernel<T, NR, DG, MODE, GATED><<<grid, threads, smem, stream>>>(p);
+    llb_launch(retention_kernel<T, NR, DG, MODE, GATED>, grid, threads, smem, stream, p);
     return llb_check_launch("retention");
 }
 
@@ -280,7 +282,7 @@ int run_retention(RetParams& p, int dtype, int num_spans, int num_items, int mul
             const size_t plane = (size_t)p.dim * p.vdim;
             int z = (int)((plane + 255) / 256);
             if (z > 64) z = 64;
-            retention_scan_kernel<<<dim3(num_spans, p.H, z), 256, 0, stream>>>(p);
+            llb_launch(retention_scan_kernel, dim3(num_spans, p.H, z), 256, 0, stream, p);
             rc = llb_check_launch("retention_scan");
             continue;
         }

@@ -20,6 +20,7 @@ __global__ void rope_kv_write_kernel(const T* __restrict__ qkv, const int* __res
                                      int rotary_dim, int interleaved, T* __restrict__ q_out,
                                      T* __restrict__ k_cache, T* __restrict__ v_cache, int Hq, int Hkv, int hd,
                                      int write_kv) {
+    llb_after_previous();
     const int t = blockIdx.x;
     const int pos = positions[t];
     const int qkv_stride = (Hq + 2 * Hkv) * hd;
@@ -74,12 +75,10 @@ LLB_EXPORT int llb_rope_kv_write(const void* qkv, int dtype, const int* position
     LLB_REQUIRE(rotary_dim == 0 || inv_freq != nullptr, "rope_kv_write: inv_freq is null");
     const int threads = 256;
     if (dtype == LLB_F32)
-        rope_kv_write_kernel<float><<<T, threads, 0, stream>>>(
-            (const float*)qkv, positions, slot_mapping, inv_freq, rotary_dim, interleaved, (float*)q_out,
+        llb_launch(rope_kv_write_kernel<float>, T, threads, 0, stream, (const float*)qkv, positions, slot_mapping, inv_freq, rotary_dim, interleaved, (float*)q_out,
             (float*)k_cache, (float*)v_cache, Hq, Hkv, hd, write_kv);
     else if (dtype == LLB_BF16)
-        rope_kv_write_kernel<__nv_bfloat16><<<T, threads, 0, stream>>>(
-            (const __nv_bfloat16*)qkv, positions, slot_mapping, inv_freq, rotary_dim, interleaved,
+        llb_launch(rope_kv_write_kernel<__nv_bfloat16>, T, threads, 0, stream, (const __nv_bfloat16*)qkv, positions, slot_mapping, inv_freq, rotary_dim, interleaved,
             (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, Hq, Hkv, hd, write_kv);
     else
         return llb_fail("rope_kv_write: unknown dtype %d", dtype);
@@ -90,6 +89,7 @@ LLB_EXPORT int llb_rope_kv_write(const void* qkv, int dtype, const int* position
 // step (the reference recomputes them on the host for every layer, src/engine/engine_server.cpp:1553-1589).
 __global__ void rope_table_kernel(const int* __restrict__ positions, const float* __restrict__ inv_freq,
                                   float2* __restrict__ table, int T, int half, int transposed) {
+    llb_after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= T * half) return;
     // token-major [T, half], or pair-major [half, T] (consecutive threads then walk along the tokens)
@@ -105,7 +105,7 @@ LLB_EXPORT int llb_rope_table(const int* positions, const float* inv_freq, float
     if (T == 0 || half == 0) return 0;
     LLB_REQUIRE(T > 0 && half > 0 && positions && inv_freq && table, "rope_table: bad arguments");
     const int n = T * half;
-    rope_table_kernel<<<llb_ceil_div(n, 256), 256, 0, stream>>>(positions, inv_freq, (float2*)table, T, half,
+    llb_launch(rope_table_kernel, llb_ceil_div(n, 256), 256, 0, stream, positions, inv_freq, (float2*)table, T, half,
                                                                 transposed ? 1 : 0);
     return llb_check_launch("rope_table");
 }
@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(256) qkv_prepare_kernel(
     const float* __restrict__ q_norm_w, const float* __restrict__ k_norm_w, float eps, const int* __restrict__ positions,
     const float* __restrict__ inv_freq, int rotary_dim, int interleaved, const int* __restrict__ slot_mapping,
     T* __restrict__ q_out, T* __restrict__ k_cache, T* __restrict__ v_cache) {
+    llb_after_previous();
     __shared__ float part[8];
     const int t = blockIdx.x;
     const int pos = positions[t];
@@ -225,13 +226,12 @@ LLB_EXPORT int llb_qkv_prepare(const void* src, int dtype, long long row_stride,
     const int share = T >= 256 ? 1 : (per_token + 255) / 256 < 8 ? (per_token + 255) / 256 : 8;
     const dim3 grid(T, share < 1 ? 1 : share);
     if (dtype == LLB_F32)
-        qkv_prepare_kernel<float><<<grid, 256, 0, stream>>>((const float*)src, row_stride, q_off, k_off, v_off, Hq, Hkv, hd,
+        llb_launch(qkv_prepare_kernel<float>, grid, 256, 0, stream, (const float*)src, row_stride, q_off, k_off, v_off, Hq, Hkv, hd,
                                                          hdv, q_norm_w, k_norm_w, eps, positions, inv_freq, rotary_dim,
                                                          interleaved, slot_mapping, (float*)q_out, (float*)k_cache,
                                                          (float*)v_cache);
     else if (dtype == LLB_BF16)
-        qkv_prepare_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(
-            (const __nv_bfloat16*)src, row_stride, q_off, k_off, v_off, Hq, Hkv, hd, hdv, q_norm_w, k_norm_w, eps, positions,
+        llb_launch(qkv_prepare_kernel<__nv_bfloat16>, grid, 256, 0, stream, (const __nv_bfloat16*)src, row_stride, q_off, k_off, v_off, Hq, Hkv, hd, hdv, q_norm_w, k_norm_w, eps, positions,
             inv_freq, rotary_dim, interleaved, slot_mapping, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_cache,
             (__nv_bfloat16*)v_cache);
     else
@@ -262,6 +262,7 @@ __global__ void __launch_bounds__(256) head_prepare_kernel(
     int v_mode, int v_width, const float* __restrict__ q_norm_w, const float* __restrict__ k_norm_w, float eps,
     const int* __restrict__ positions, const float* __restrict__ inv_freq, int rotary_dim, int interleaved,
     const int* __restrict__ slot_mapping, T* __restrict__ q_out, T* __restrict__ k_cache, T* __restrict__ v_cache) {
+    llb_after_previous();
     extern __shared__ float2 cs[];          // (cos, sin) of the token's angles, one a pair: every head turns by the same
     const int t = blockIdx.x;
     const int lane = threadIdx.x & 31;
@@ -362,12 +363,10 @@ LLB_EXPORT int llb_head_prepare(const void* src, int dtype, long long row_stride
     const dim3 grid(T, share < 1 ? 1 : share);
     const size_t smem = (size_t)(rotary_dim / 2) * sizeof(float2);
     if (dtype == LLB_F32)
-        head_prepare_kernel<float><<<grid, 256, smem, stream>>>(
-            (const float*)src, row_stride, q_off, k_off, v_off, Hq, Hk, hd, q_maps, v_mode, v_width, q_norm_w, k_norm_w, eps,
+        llb_launch(head_prepare_kernel<float>, grid, 256, smem, stream, (const float*)src, row_stride, q_off, k_off, v_off, Hq, Hk, hd, q_maps, v_mode, v_width, q_norm_w, k_norm_w, eps,
             positions, inv_freq, rotary_dim, interleaved, slot_mapping, (float*)q_out, (float*)k_cache, (float*)v_cache);
     else if (dtype == LLB_BF16)
-        head_prepare_kernel<__nv_bfloat16><<<grid, 256, smem, stream>>>(
-            (const __nv_bfloat16*)src, row_stride, q_off, k_off, v_off, Hq, Hk, hd, q_maps, v_mode, v_width, q_norm_w,
+        llb_launch(head_prepare_kernel<__nv_bfloat16>, grid, 256, smem, stream, (const __nv_bfloat16*)src, row_stride, q_off, k_off, v_off, Hq, Hk, hd, q_maps, v_mode, v_width, q_norm_w,
             k_norm_w, eps, positions, inv_freq, rotary_dim, interleaved, slot_mapping, (__nv_bfloat16*)q_out,
             (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache);
     else

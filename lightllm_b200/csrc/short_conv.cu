@@ -72,6 +72,7 @@ __device__ __forceinline__ int span_of_row(const int* span_row, int num_spans, i
 
 template <typename T>
 __global__ void __launch_bounds__(128) conv_prepare_kernel(ConvParams p) {
+    llb_after_previous();
     const int lane = threadIdx.x & 31;
     const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (item >= (long long)p.T * p.total_heads) return;
@@ -185,6 +186,7 @@ __global__ void __launch_bounds__(128) conv_prepare_kernel(ConvParams p) {
 // is shorter than the tail) before it writes.
 template <typename T>
 __global__ void __launch_bounds__(256) conv_tail_kernel(ConvParams p) {
+    llb_after_previous();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int span = blockIdx.y;
     if (c >= p.C) return;
@@ -260,8 +262,8 @@ LLB_EXPORT int llb_conv_prepare_temp(const void* src, int src_dtype, long long r
     }
     const long long items = (long long)T * p.total_heads;
     const unsigned blocks = (unsigned)((items + 3) / 4);
-    if (src_dtype == LLB_F32) conv_prepare_kernel<float><<<blocks, 128, 0, stream>>>(p);
-    else if (src_dtype == LLB_BF16) conv_prepare_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>(p);
+    if (src_dtype == LLB_F32) llb_launch(conv_prepare_kernel<float>, blocks, 128, 0, stream, p);
+    else if (src_dtype == LLB_BF16) llb_launch(conv_prepare_kernel<__nv_bfloat16>, blocks, 128, 0, stream, p);
     else return llb_fail("conv_prepare: unknown dtype %d", src_dtype);
     return llb_check_launch("conv_prepare");
 }
@@ -293,8 +295,8 @@ LLB_EXPORT int llb_conv_tail_update(const void* src, int src_dtype, long long ro
     p.span_row = span_row; p.span_len = span_len; p.span_pos = span_pos; p.span_slot = span_slot;
     p.state = state; p.state_stride = state_stride; p.tail_off = tail_off;
     const dim3 grid((C + 255) / 256, num_spans);
-    if (src_dtype == LLB_F32) conv_tail_kernel<float><<<grid, 256, 0, stream>>>(p);
-    else if (src_dtype == LLB_BF16) conv_tail_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(p);
+    if (src_dtype == LLB_F32) llb_launch(conv_tail_kernel<float>, grid, 256, 0, stream, p);
+    else if (src_dtype == LLB_BF16) llb_launch(conv_tail_kernel<__nv_bfloat16>, grid, 256, 0, stream, p);
     else return llb_fail("conv_tail_update: unknown dtype %d", src_dtype);
     return llb_check_launch("conv_tail_update");
 }
@@ -351,6 +353,7 @@ template <> struct ConvVec<__nv_bfloat16, 4> {
 // TAPS: the most taps this instantiation carries (a smaller `taps` leaves its first slots unused).
 template <typename T, int V, int TAPS, int ROWS>
 __global__ void __launch_bounds__(128) conv_act_kernel(ConvActParams p) {
+    llb_after_previous();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     if (c >= p.C) return;
     const int t0 = blockIdx.y * ROWS, t1 = min(p.T, t0 + ROWS);
@@ -425,11 +428,11 @@ int launch_conv_act_rows(const ConvActParams& p, cudaStream_t stream) {
     const int groups = (p.C + V - 1) / V;
     const unsigned gx = (unsigned)((groups + 127) / 128);
     if ((long long)gx * p.T <= 148 * 8 || p.fuse_tail)
-        conv_act_kernel<T, V, TAPS, 1><<<dim3(gx, p.T), 128, 0, stream>>>(p);
+        llb_launch(conv_act_kernel<T, V, TAPS, 1>, dim3(gx, p.T), 128, 0, stream, p);
     else if ((long long)gx * p.T <= 148 * 32)
-        conv_act_kernel<T, V, TAPS, 4><<<dim3(gx, (p.T + 3) / 4), 128, 0, stream>>>(p);
+        llb_launch(conv_act_kernel<T, V, TAPS, 4>, dim3(gx, (p.T + 3) / 4), 128, 0, stream, p);
     else
-        conv_act_kernel<T, V, TAPS, 16><<<dim3(gx, (p.T + 15) / 16), 128, 0, stream>>>(p);
+        llb_launch(conv_act_kernel<T, V, TAPS, 16>, dim3(gx, (p.T + 15) / 16), 128, 0, stream, p);
     return llb_check_launch("conv_act");
 }
 

@@ -69,6 +69,7 @@ constexpr int WALK_STAGE = 16;
 
 template <typename T, int NR, int DG>
 __global__ void __launch_bounds__(256) ssm_walk_kernel(SsmParams p) {
+    llb_after_previous();
     extern __shared__ __align__(16) float sm[];
     constexpr int PADF = DG > 1 ? 4 : 0;
     constexpr int DPAD = DG * (NR + PADF);
@@ -160,7 +161,7 @@ int launch_walk_as(SsmParams p, int num_spans, cudaStream_t stream) {
         const cudaError_t e = cudaFuncSetAttribute(ssm_walk_kernel<T, NR, DG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return llb_fail("state_space: %s", cudaGetErrorString(e));
     }
-    ssm_walk_kernel<T, NR, DG><<<grid, threads, smem, stream>>>(p);
+    llb_launch(ssm_walk_kernel<T, NR, DG>, grid, threads, smem, stream, p);
     return llb_check_launch("state_space_walk");
 }
 
@@ -181,6 +182,7 @@ constexpr int STEP_THREADS = 128;
 
 template <typename T, int ROWS>
 __global__ void __launch_bounds__(STEP_THREADS) ssm_step_kernel(SsmParams p) {
+    llb_after_previous();
     extern __shared__ __align__(16) float sm[];       // B [N], C [N], then (16-byte aligned) the partial sums [RT][vdim]
     const int span = blockIdx.x, h = blockIdx.y;
     const int N = p.N, vdim = p.vdim, CP = vdim >> 2, RT = STEP_THREADS / CP;
@@ -253,9 +255,9 @@ int launch_step(const SsmParams& p, int num_spans, cudaStream_t stream) {
     const int RT = STEP_THREADS / (p.vdim / 4), rows = (p.N + RT - 1) / RT;
     const size_t smem = ((size_t)((2 * p.N + 3) & ~3) + (size_t)RT * p.vdim) * sizeof(float);
     const dim3 grid(num_spans, p.H);
-    if (rows <= 4) ssm_step_kernel<T, 4><<<grid, STEP_THREADS, smem, stream>>>(p);
-    else if (rows <= 8) ssm_step_kernel<T, 8><<<grid, STEP_THREADS, smem, stream>>>(p);
-    else ssm_step_kernel<T, 16><<<grid, STEP_THREADS, smem, stream>>>(p);
+    if (rows <= 4) llb_launch(ssm_step_kernel<T, 4>, grid, STEP_THREADS, smem, stream, p);
+    else if (rows <= 8) llb_launch(ssm_step_kernel<T, 8>, grid, STEP_THREADS, smem, stream, p);
+    else llb_launch(ssm_step_kernel<T, 16>, grid, STEP_THREADS, smem, stream, p);
     return llb_check_launch("state_space_step");
 }
 
@@ -289,6 +291,7 @@ struct ChunkShape {
 
 template <int MT, int EV, int MODE>
 __global__ void __launch_bounds__(128) ssm_chunk_kernel(SsmParams p) {
+    llb_after_previous();
     using Sh = ChunkShape<MT, EV>;
     constexpr int NP = Sh::NP, NB = Sh::NB, XB = Sh::XB, NE = EV / 8, KS = NP / 16, NST = Sh::NST;
     extern __shared__ __align__(16) uint8_t smem[];
@@ -557,6 +560,7 @@ __global__ void __launch_bounds__(128) ssm_chunk_kernel(SsmParams p) {
 
 // start_0 = the request's state (zero at position 0); start_c = keep_(c-1) * start_(c-1) + contribution_(c-1).
 __global__ void __launch_bounds__(256) ssm_scan_kernel(SsmParams p) {
+    llb_after_previous();
     const int span = blockIdx.x, h = blockIdx.y;
     const int slen = p.span_len[span];
     const int pieces = (slen + p.chunk - 1) / p.chunk;
@@ -604,7 +608,7 @@ int launch_chunk(const SsmParams& p, int num_items, cudaStream_t stream) {
         if (e != cudaSuccess) return llb_fail("state_space: %s", cudaGetErrorString(e));
         configured = true;
     }
-    ssm_chunk_kernel<MT, EV, MODE><<<dim3(num_items, p.H, llb_ceil_div(p.vdim, EV)), 128, bytes, stream>>>(p);
+    llb_launch(ssm_chunk_kernel<MT, EV, MODE>, dim3(num_items, p.H, llb_ceil_div(p.vdim, EV)), 128, bytes, stream, p);
     return llb_check_launch("state_space_chunks");
 }
 
@@ -627,6 +631,7 @@ template <typename TZ, int V>
 __global__ void __launch_bounds__(256) gated_group_norm_kernel(const float* __restrict__ y, const TZ* __restrict__ z,
                                                                long long z_stride, const float* __restrict__ w,
                                                                TZ* __restrict__ out, int size, int parts, float eps) {
+    llb_after_previous();
     const int t = blockIdx.x, part = blockIdx.y;
     const int n = size * parts;
     const float* yr = y + (size_t)t * n + (size_t)part * size;
@@ -693,8 +698,8 @@ int launch_group_norm(const float* y, const void* z, long long z_stride, const f
     const int per = vec ? 4 : 1;
     int threads = 32 * ((size / per + 31) / 32);
     threads = threads > 256 ? 256 : threads < 32 ? 32 : threads;
-    if (vec) gated_group_norm_kernel<TZ, 4><<<grid, threads, 0, stream>>>(y, (const TZ*)z, z_stride, w, (TZ*)out, size, parts, eps);
-    else gated_group_norm_kernel<TZ, 1><<<grid, threads, 0, stream>>>(y, (const TZ*)z, z_stride, w, (TZ*)out, size, parts, eps);
+    if (vec) llb_launch(gated_group_norm_kernel<TZ, 4>, grid, threads, 0, stream, y, (const TZ*)z, z_stride, w, (TZ*)out, size, parts, eps);
+    else llb_launch(gated_group_norm_kernel<TZ, 1>, grid, threads, 0, stream, y, (const TZ*)z, z_stride, w, (TZ*)out, size, parts, eps);
     return llb_check_launch("gated_group_norm");
 }
 
@@ -743,7 +748,7 @@ LLB_EXPORT int llb_state_space(const void* xbc, int dtype, long long stride, int
             if (pass == 1) {
                 int z = (N * vdim + 255) / 256;
                 if (z > 64) z = 64;
-                ssm_scan_kernel<<<dim3(num_spans, H, z), 256, 0, stream>>>(p);
+                llb_launch(ssm_scan_kernel, dim3(num_spans, H, z), 256, 0, stream, p);
                 rc = llb_check_launch("state_space_scan");
                 continue;
             }

@@ -51,6 +51,7 @@ template <typename TO, int V> __device__ __forceinline__ void store_row(TO* p, c
 // One block a row: the row and the one before it are read once for the sums of squares and again (from cache) for the result.
 template <typename TO, int V>
 __global__ void __launch_bounds__(256) norm_shift_kernel(ShiftParams p) {
+    llb_after_previous();
     const int t = blockIdx.x, D = p.D;
     int lo = 0, hi = p.num_spans - 1;          // the last span whose first row is <= t
     while (lo < hi) {
@@ -141,8 +142,8 @@ int launch_norm_shift(const ShiftParams& p, int T, cudaStream_t stream) {
     const int per = vec ? 4 : 1;
     int threads = 32 * ((p.D / per + 31) / 32);
     threads = threads > 256 ? 256 : threads < 32 ? 32 : threads;
-    if (vec) norm_shift_kernel<TO, 4><<<T, threads, 0, stream>>>(p);
-    else norm_shift_kernel<TO, 1><<<T, threads, 0, stream>>>(p);
+    if (vec) llb_launch(norm_shift_kernel<TO, 4>, T, threads, 0, stream, p);
+    else llb_launch(norm_shift_kernel<TO, 1>, T, threads, 0, stream, p);
     return llb_check_launch("norm_shift");
 }
 
