@@ -121,13 +121,53 @@ __global__ void __launch_bounds__(256) rmsnorm_warp_kernel(const float* __restri
     }
 }
 
+// One block per row of a float input whose width is a multiple of 4 and at most 4 * NV * blockDim: a thread asks for its NV pieces of 16
+// bytes of the row and of the weights at once, so that a row costs one trip to memory however few rows there are.
+template <typename TW, typename TO, int NV>
+__global__ void __launch_bounds__(512) rmsnorm_block_kernel(const float* __restrict__ x, const TW* __restrict__ w, TO* __restrict__ out,
+                                                            const int* __restrict__ rows, int D, float eps) {
+    __shared__ float part[16];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int r = blockIdx.x;
+    const float* xr = x + (size_t)(rows ? rows[r] : r) * D;
+    float4 v[NV], g[NV];
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int d = (i * blockDim.x + threadIdx.x) * 4;
+        v[i] = d < D ? *reinterpret_cast<const float4*>(xr + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        g[i] = d < D ? load4(w + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+    ss = llb_warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float total = 0.0f;
+    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) total += part[k];
+    const float inv = 1.0f / sqrtf(total / (float)D + eps);
+    TO* o = out + (size_t)r * D;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int d = (i * blockDim.x + threadIdx.x) * 4;
+        if (d < D) store4(o + d, make_float4(v[i].x * inv * g[i].x, v[i].y * inv * g[i].y, v[i].z * inv * g[i].z, v[i].w * inv * g[i].w));
+    }
+}
+
+// A warp per row leaves most multiprocessors without a row until there are about as many rows as multiprocessors; beyond, both are alike.
+// us a launch in a chain of them, warps / block: 896 wide 27 rows 1.66 / 1.31, 100 1.74 / 1.42, 148 1.75 / 1.75; 1,536 wide 27 rows 2.14 /
+// 1.35, 148 2.24 / 2.23.  Wider rows always take a block (3,584 wide, single floats a thread before: 8 rows 2.24 -> 1.55, 2,048 9.6 -> 7.5).
+static bool norm_by_warps(int R, int D) { return D <= 128 * 16 && R >= 148; }
+
 template <typename TI, typename TW, typename TO>
 static int launch_rmsnorm(const void* x, const void* w, void* out, const int* rows, int R, int D, float eps,
                           cudaStream_t stream) {
     const int threads = 256;
     cudaError_t e;
-    if (std::is_same<TI, float>::value && D % 4 == 0 && D <= 128 * 16 && (uintptr_t)x % 16 == 0 &&
-        (uintptr_t)w % 16 == 0 && (uintptr_t)out % 16 == 0 && R >= 8) {
+    const bool vec = std::is_same<TI, float>::value && D % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0 &&
+                     (uintptr_t)out % 16 == 0;
+    if (vec && norm_by_warps(R, D)) {
         const dim3 grid((R + 7) / 8);
         if (D <= 128 * 8)
             e = launch_pdl(rmsnorm_warp_kernel<TW, TO, 8>, grid, dim3(threads), stream, (const float*)x, (const TW*)w,
@@ -135,6 +175,12 @@ static int launch_rmsnorm(const void* x, const void* w, void* out, const int* ro
         else
             e = launch_pdl(rmsnorm_warp_kernel<TW, TO, 16>, grid, dim3(threads), stream, (const float*)x, (const TW*)w,
                            (TO*)out, rows, R, D, eps);
+    } else if (vec && D <= 8192) {
+        const int quads = D / 4, per = quads <= 512 ? 1 : quads <= 1024 ? 2 : 4;
+        const dim3 block(((quads + per - 1) / per + 31) / 32 * 32);
+        if (per == 1) e = launch_pdl(rmsnorm_block_kernel<TW, TO, 1>, dim3(R), block, stream, (const float*)x, (const TW*)w, (TO*)out, rows, D, eps);
+        else if (per == 2) e = launch_pdl(rmsnorm_block_kernel<TW, TO, 2>, dim3(R), block, stream, (const float*)x, (const TW*)w, (TO*)out, rows, D, eps);
+        else e = launch_pdl(rmsnorm_block_kernel<TW, TO, 4>, dim3(R), block, stream, (const float*)x, (const TW*)w, (TO*)out, rows, D, eps);
     } else if (D <= threads * 4)
         e = launch_pdl(rmsnorm_kernel<TI, TW, TO, 4>, dim3(R), dim3(threads), stream, (const TI*)x, (const TW*)w, (TO*)out, rows, D, eps);
     else if (D <= threads * 16)
