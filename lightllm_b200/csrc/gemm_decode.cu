@@ -6,15 +6,27 @@
 //   epilogue ROPE_KV   bias, rotary positions on q and k (src/ops/rope.cu:54-59, every pair), q to its
 //                      buffer, k and v into their cache pages (src/kv_cache/paged_attention.cu:1150-1163);
 //   epilogue SWIGLU    SiLU(gate) * up on interleaved weight rows (src/engine/engine_server.cpp:1875-1878);
-//   epilogue RESIDUAL  adds into the float residual stream, split-K by atomic adds (engine_server.cpp:1870-1871);
+//   epilogue RESIDUAL  adds into the float residual stream (engine_server.cpp:1870-1871);
+//   epilogue STORE     bf16 output, optionally through a plain activation;
 //   epilogue STORE_F32 float output (the head's logits).
 //
 // The weights take the MMA's 128-row A role and stream through a TMA ring; the few activation rows are
-// the B operand (BN = 16, 32 or 64 columns of tensor memory).  Every launch is a programmatic dependent
+// the B operand (BN = 16, 32 or 64 columns of tensor memory).  Few tiles of features over a long K are cut along K among the
+// blocks of a thread-block cluster: every block sends the sums it has of a token straight into the shared memory of the block
+// that finishes that token (token t: block t mod C), the cluster meets once, and each block adds up and finishes its tokens in a
+// fixed order.  A block alone does the same within its own shared memory.  So the epilogue reads its features side by side,
+// whatever the tensor memory's layout, and is spread over eight warps of every block.  Measured (us that the launch adds to the chain
+// of a step at the 0.5B sizes; four epilogue warps on the accumulators' layout and adds into memory -> now): 64 rows gate/up 16.3 ->
+// 10.2, q/k/v 10.0 -> 8.0, o_proj 6.9 -> 6.4; 32 rows gate/up 11.5 -> 7.4, q/k/v 9.5 -> 5.6.  What bounds it: the launch before must have
+// completed (1 us), then activations, products, the meeting and the outputs, each a trip to L2 or to another multiprocessor of
+// half a microsecond to one; the weights' 17 MB of gate/up are 2.7 us of the copy rate.
+//
+// Every launch is a programmatic dependent
 // launch: a block initialises its barriers, allocates tensor memory and already requests its first weight
 // tiles while the kernel before it is still running, and only then waits for that kernel
 // (griddepcontrol.wait) before it reads activations or writes anything.  Waits on mbarriers are bounded
 // in time as in the other tensor-core kernels.
+#include <atomic>
 #include <utility>
 
 #include "tcgen05_common.cuh"
@@ -26,13 +38,15 @@ using namespace t5;
 constexpr int TILE_M = 128;
 constexpr int TILE_K = 64;
 // Depth of the TMA ring: a block streams its weights at (bytes in flight) / latency.  Grids of a few blocks
-// get a deep ring (8 stages, one block per SM); grids of many blocks (the head) a short one (4 stages), so
-// that two blocks share an SM.
-constexpr int DEEP = 8, SHALLOW = 4;
-constexpr int NUM_THREADS = 192;
+// get a deep ring (8 stages, one block per SM; 6 where the received sums of 64 rows lie beside it); grids of many blocks (the
+// head) a short one (4 stages), so that two blocks share an SM.
+constexpr int DEEP = 8, MIDDLE = 6, SHALLOW = 4;
+constexpr int WORKERS = 256;                // warps 2-9
+constexpr int NUM_THREADS = 64 + WORKERS;
+constexpr int MAX_CLUSTER = 8;
 constexpr uint32_t A_BYTES = TILE_M * TILE_K * 2;
 
-enum { DEPI_STORE_F32 = 1, DEPI_RESIDUAL = 2, DEPI_SWIGLU = 3, DEPI_ROPE_KV = 4 };
+enum { DEPI_STORE_F32 = 1, DEPI_RESIDUAL = 2, DEPI_SWIGLU = 3, DEPI_ROPE_KV = 4, DEPI_STORE = 5 };
 
 struct DecodeGemmParams {
     // NORM prologue
@@ -53,12 +67,10 @@ struct DecodeGemmParams {
     __nv_bfloat16* q_out;      // [M, Hq * hd]
     __nv_bfloat16* k_cache;    // [slots, Hkv, hd]
     __nv_bfloat16* v_cache;
-    // split-K with a fused epilogue: partial sums meet in acc_scratch [BN, N] (zero between launches),
-    // counters[n-tile] counts the splits that have arrived; the last one runs the epilogue and cleans up
-    float* acc_scratch;
-    int* counters;
+    int cluster;               // blocks of a cluster: neighbouring pieces of K whose sums meet (1: a block alone)
+    uint32_t recv_offset;      // where they meet, behind the operand tiles (over the weight ring when alone)
     int* error_flag;
-    LlbGluArgs glu;            // the gated activation of the GLU epilogue
+    LlbGluArgs glu;            // the gated activation of the GLU epilogue, the plain one of STORE, the scale of the float ones
 };
 
 // How the rotary epilogue treats one output feature n (row `row` of the block's tile): whether it is rotated, with
@@ -82,21 +94,94 @@ __device__ __forceinline__ RopeRow rope_row(const DecodeGemmParams& p, int n, in
     }
     return r;
 }
-// (cos, sin) and cache rows of tokens m0 .. m0+15 for that feature; the loads do not depend on each other.
-__device__ __forceinline__ void rope_fetch(const DecodeGemmParams& p, const RopeRow& r, int n, int m0, float2 (&cs)[16],
-                                           int (&slot)[16]) {
-    const int half = p.rotary_dim / 2;
+// (cos, sin) and cache rows of four of the block's tokens (i0, i0 + 2, ..) for that feature; the loads do not depend on each other.
+constexpr int ROPE_BATCH = 4;
+__device__ __forceinline__ void rope_fetch(const DecodeGemmParams& p, const RopeRow& r, int n, int rank, int i0, int mine,
+                                           float2 (&cs)[ROPE_BATCH], int (&slot)[ROPE_BATCH]) {
     const bool cached = n < p.N && n >= p.Hq * p.hd && p.slot_mapping != nullptr;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const int m = m0 + j;
-        cs[j] = (r.rotate && m < p.M) ? __ldg(p.rope_table + (size_t)m * half + r.fi) : make_float2(1.0f, 0.0f);
-        slot[j] = (cached && m < p.M) ? __ldg(p.slot_mapping + m) : -1;
+    for (int u = 0; u < ROPE_BATCH; ++u) {
+        const int i = i0 + u * (WORKERS / TILE_M), m = rank + i * p.cluster;
+        cs[u] = (r.rotate && i < mine) ? __ldg(p.rope_table + (size_t)m * (p.rotary_dim / 2) + r.fi) : make_float2(1.0f, 0.0f);
+        slot[u] = (cached && i < mine) ? __ldg(p.slot_mapping + m) : -1;
+    }
+}
+// The sum of what the blocks of the cluster sent of one token's features, in the order of K: slot i of every source, `slots` apart.
+__device__ __forceinline__ float2 recv_pair(const float* recv, int cluster, int slots, int i, int f) {
+    float2 v = *reinterpret_cast<const float2*>(recv + i * TILE_M + f);
+    for (int src = 1; src < cluster; ++src) {
+        const float2 u = *reinterpret_cast<const float2*>(recv + (src * slots + i) * TILE_M + f);
+        v.x += u.x;
+        v.y += u.y;
+    }
+    return v;
+}
+__device__ __forceinline__ float recv_one(const float* recv, int cluster, int slots, int i, int f) {
+    float v = recv[i * TILE_M + f];
+    for (int src = 1; src < cluster; ++src) v += recv[(src * slots + i) * TILE_M + f];
+    return v;
+}
+// One token m and two neighbouring features n, n + 1 (n even).
+template <int EPI>
+__device__ __forceinline__ void finish_pair(const DecodeGemmParams& p, float2 v, float2 bias, int m, int n, bool alone) {
+    const bool has1 = n + 1 < p.N;
+    v.x += bias.x;
+    v.y += bias.y;
+    if (EPI == DEPI_SWIGLU) {
+        if (has1)
+            ((__nv_bfloat16*)p.out)[(size_t)m * (p.N / 2) + (n >> 1)] =
+                __float2bfloat16_rn(llb_glu(v.x, v.y, p.glu.kind, p.glu.alpha, p.glu.limit, p.glu.up_shift));
+        return;
+    }
+    const size_t at = (size_t)m * p.N + n;
+    if (EPI == DEPI_STORE) {
+        __nv_bfloat16* o = (__nv_bfloat16*)p.out + at;
+        const __nv_bfloat162 h = __floats2bfloat162_rn(llb_act(v.x, p.glu.kind), llb_act(v.y, p.glu.kind));
+        if (has1 && ((uintptr_t)o & 3) == 0) {
+            *reinterpret_cast<__nv_bfloat162*>(o) = h;
+        } else {
+            o[0] = h.x;
+            if (has1) o[1] = h.y;
+        }
+        return;
+    }
+    const float f = llb_out_scale(p.glu);
+    v.x *= f;
+    v.y *= f;
+    float* o = (EPI == DEPI_STORE_F32 ? (float*)p.out : p.residual) + at;
+    if (EPI == DEPI_RESIDUAL && !alone) {
+        if (has1 && ((uintptr_t)o & 7) == 0) {
+            asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(o), "f"(v.x), "f"(v.y) : "memory");
+        } else {
+            atomicAdd(o, v.x);
+            if (has1) atomicAdd(o + 1, v.y);
+        }
+    } else if (has1 && ((uintptr_t)o & 7) == 0) {
+        if (EPI == DEPI_RESIDUAL) {
+            const float2 r = *reinterpret_cast<const float2*>(o);
+            v.x += r.x;
+            v.y += r.y;
+        }
+        *reinterpret_cast<float2*>(o) = v;
+    } else {
+        o[0] = EPI == DEPI_RESIDUAL ? o[0] + v.x : v.x;
+        if (has1) o[1] = EPI == DEPI_RESIDUAL ? o[1] + v.y : v.y;
     }
 }
 
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&r)[8]) {
+    uint32_t* u = reinterpret_cast<uint32_t*>(r);
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
+                 : "r"(taddr)
+                 : "memory");
+    tmem_wait_ld();
+}
+
+// (Rings of up to five stages are for two blocks on a multiprocessor: ten warps lie three to a scheduler, so that both fit only from 80
+// registers down; the bound for three blocks gives 64.)
 template <int BN, int EPI, bool NORM, int STAGES>
-__global__ void __launch_bounds__(NUM_THREADS)
+__global__ void __launch_bounds__(NUM_THREADS, STAGES <= 5 ? 3 : 1)
 gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                    const DecodeGemmParams p) {
     constexpr uint32_t B_BYTES = BN * TILE_K * 2;
@@ -105,14 +190,14 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __shared__ __align__(8) uint64_t empty_bar[8];
     __shared__ __align__(8) uint64_t acc_bar, b_ready_bar;
     __shared__ uint32_t tmem_slot;
-    __shared__ int abort_s, last_s;
+    __shared__ int abort_s;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* a_tiles = smem;                             // STAGES weight tiles
     uint8_t* b_tiles = smem + STAGES * A_BYTES;          // NORM: num_kb resident tiles; else STAGES tiles
     const int b_count = NORM ? p.num_kb : STAGES;
     (void)b_count;
-    float* stage_f = (float*)a_tiles;     // ROPE_KV: [128][BN + 1] floats over the weight ring, which is idle by then
+    float* recv = (float*)(smem + p.recv_offset);        // [cluster][slots][128]: this block's tokens' sums, from every block
     volatile int* abort_flag = &abort_s;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -137,8 +222,16 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
     if (threadIdx.x == 0) griddep_launch_dependents();
+    // the others of the cluster have begun: waited for before anything is sent to them
+    __syncwarp();
+    if (p.cluster > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    const int rank = (int)blockIdx.z % p.cluster, slots = (BN + p.cluster - 1) / p.cluster;
+    bool ok = true;
+    RopeRow rr;                     // the rotary epilogue's feature and first tokens
+    float2 cs[ROPE_BATCH];
+    int slot_of[ROPE_BATCH];
 
-    if (nkb > 0) {
+    {
         if (warp == 0) {
             if (lane == 0) {
                 // Weights do not depend on the kernel before this one: request the first tiles at once.
@@ -162,7 +255,6 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         } else if (warp == 1) {
             if (lane == 0) {
                 constexpr uint32_t idesc = idesc_bf16(TILE_M, BN);
-                bool ok = true;
                 if (NORM) ok = mbar_wait(&b_ready_bar, 0, abort_flag);
                 for (int i = 0; i < nkb && ok; ++i) {
                     const int s = i % STAGES;
@@ -180,9 +272,8 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 if (ok) umma_commit(&acc_bar);
             }
         } else {
-            const int quarter = warp & 3;
             griddep_wait();
-            if (NORM) {
+            if (NORM && warp < 6) {
                 // B operand = RMSNorm(x) * w for all K, as bf16 in the swizzled K-major tiles.  One warp per row.
                 if (p.K <= 1024 && p.M <= 8) {
                     // Few short rows: a warp asks for both of its rows at once and keeps them in registers (8 float4
@@ -291,130 +382,91 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 fence_async_smem();
                 mbar_arrive(&b_ready_bar);
             }
-            const int row = quarter * 32 + lane;     // row of the tile = TMEM lane = output feature
-            const int n = n0 + row;
-            // Rotary epilogue: what this output feature needs of the first 16 tokens (their angles' cos and sin,
-            // their cache rows) is asked for now, while the tensor cores still work; loaded one by one inside the
-            // loop over the tokens, each of these reads would be a round trip of its own.
-            RopeRow rr;
-            float2 cs_first[16];
-            int slot_first[16];
-            if (EPI == DEPI_ROPE_KV) {
-                rr = rope_row(p, n, row);
-                rope_fetch(p, rr, n, 0, cs_first, slot_first);
+            if (EPI == DEPI_ROPE_KV) {          // asked for while the tensor cores still work
+                const int e = threadIdx.x - 64;
+                rr = rope_row(p, n0 + (e & (TILE_M - 1)), e & (TILE_M - 1));
+                rope_fetch(p, rr, n0 + (e & (TILE_M - 1)), rank, e >> 7, (p.M - rank + p.cluster - 1) / p.cluster, cs, slot_of);
             }
-            bool ok = mbar_wait(&acc_bar, 0, abort_flag);
+            ok = mbar_wait(&acc_bar, 0, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
             tc_fence_after();
-            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-            const bool meet = (EPI == DEPI_ROPE_KV || EPI == DEPI_SWIGLU) && gridDim.z > 1;
-            if (meet) {
-                // Partial sums of the splits meet in scratch; the split that arrives last runs the epilogue.
-                if (ok) {      // uniform over the warp: tcgen05.ld is a warp-wide instruction
-#pragma unroll 1
-                    for (int c0 = 0; c0 < BN; c0 += 16) {
-                        float v[16];
-                        tmem_ld16(taddr + c0, v);
+        }
+        __syncwarp();
+        if (p.cluster > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (warp >= 2 && ok) {
+            // eight warps: a quarter of the features and half of the tokens each; every token's sums go to the block that finishes it
+            constexpr int COLS = BN / 2;
+            const int row = (warp & 3) * 32 + lane, c0 = ((warp - 2) >> 2) * COLS;
+            const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + c0;
+            const uint32_t own = smem_u32(recv) + (uint32_t)((rank * slots) * TILE_M + row) * 4;
+            int slot = c0 / p.cluster, dst = c0 - slot * p.cluster;          // of token c0 + c + j, counted on
 #pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (c0 + j < p.M && n < p.N) atomicAdd(p.acc_scratch + (size_t)(c0 + j) * p.N + n, v[j]);
+            for (int c = 0; c < COLS; c += 8) {
+                if (c0 + c >= p.M) break;          // (uniform)
+                float v[8];
+                tmem_ld8(taddr + c, v);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (c0 + c + j < p.M) {
+                        const uint32_t at = own + (uint32_t)slot * (TILE_M * 4);
+                        if (p.cluster > 1)
+                            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(mapa_u32(at, (uint32_t)dst)), "f"(v[j]) : "memory");
+                        else
+                            recv[slot * TILE_M + row] = v[j];
                     }
+                    if (++dst == p.cluster) { dst = 0; ++slot; }
                 }
-                __threadfence();
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (warp == 2 && lane == 0) last_s = (atomicAdd(p.counters + blockIdx.x, 1) == (int)gridDim.z - 1) ? 1 : 0;
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                ok = ok && last_s != 0;
-                if (ok) __threadfence();
             }
-            // This thread's row of the tile, 16 columns (tokens) at a time: from tensor memory, or from the
-            // meeting place (which is left zeroed for the next launch).
-            auto load16 = [&](int c0, float (&v)[16]) {
-                if (!meet) {
-                    tmem_ld16(taddr + c0, v);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        v[j] = 0.0f;
-                        if (c0 + j < p.M && n < p.N) {
-                            float* a = p.acc_scratch + (size_t)(c0 + j) * p.N + n;
-                            v[j] = __ldcg(a);
-                            __stcg(a, 0.0f);
-                        }
-                    }
-                }
-            };
-            const float bias = (p.bias && n < p.N && (meet || blockIdx.z == 0)) ? p.bias[n] : 0.0f;
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (p.cluster > 1) {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        } else if (warp >= 2) {
+            asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory");
+        }
+        if (warp >= 2 && ok) {
+            const int e = threadIdx.x - 64;
+            const int mine = (p.M - rank + p.cluster - 1) / p.cluster;          // tokens rank, rank + cluster, ...
+            const int piece = (int)blockIdx.z / p.cluster;                      // of K, when several clusters add into the residual
             if (EPI == DEPI_ROPE_KV) {
-                // Stage the tile (+ bias) as float; the barrier is reached by all four warps whatever happened.
-                if (ok) {
-#pragma unroll 1
-                    for (int c0 = 0; c0 < BN; c0 += 16) {
-                        float v[16];
-                        load16(c0, v);
+                // a feature a thread: rotate pairs of rows of one head and scatter to q and the cache pages
+                const int row = e & (TILE_M - 1), n = n0 + row;
+                const int q_end = p.Hq * p.hd, k_end = q_end + p.Hkv * p.hd;
+                const float bias = (p.bias && n < p.N) ? p.bias[n] : 0.0f;
+                const float other_bias = (p.bias && rr.rotate) ? p.bias[n0 + rr.partner] : 0.0f;
+                for (int i0 = e >> 7; n < p.N && i0 < mine; i0 += ROPE_BATCH * (WORKERS / TILE_M)) {
+                    if (i0 != e >> 7) rope_fetch(p, rr, n, rank, i0, mine, cs, slot_of);
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) stage_f[row * (BN + 1) + c0 + j] = v[j] + bias;
-                    }
-                }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-            }
-            if (ok) {
-                if (EPI == DEPI_ROPE_KV) {
-                    // Rotate pairs of rows of one head and scatter to q and the cache pages, 16 tokens at a time.
-                    if (n < p.N) {
-                        const int q_end = p.Hq * p.hd, k_end = q_end + p.Hkv * p.hd;
-                        for (int m0 = 0; m0 < p.M; m0 += 16) {
-                            float2 cs[16];
-                            int slot[16];
-                            if (m0 == 0) {
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) { cs[j] = cs_first[j]; slot[j] = slot_first[j]; }
-                            } else {
-                                rope_fetch(p, rr, n, m0, cs, slot);
-                            }
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                const int m = m0 + j;
-                                if (m >= p.M) break;
-                                float val = stage_f[row * (BN + 1) + m];
-                                if (rr.rotate) {
-                                    const float other = stage_f[rr.partner * (BN + 1) + m];
-                                    val = rr.first ? val * cs[j].x - other * cs[j].y : val * cs[j].x + other * cs[j].y;
-                                }
-                                const __nv_bfloat16 h = __float2bfloat16_rn(val);
-                                if (n < q_end) {
-                                    p.q_out[(size_t)m * q_end + n] = h;
-                                } else if (slot[j] >= 0) {
-                                    if (n < k_end) p.k_cache[(size_t)slot[j] * (p.Hkv * p.hd) + (n - q_end)] = h;
-                                    else p.v_cache[(size_t)slot[j] * (p.Hkv * p.hd) + (n - k_end)] = h;
-                                }
-                            }
+                    for (int u = 0; u < ROPE_BATCH; ++u) {
+                        const int i = i0 + u * (WORKERS / TILE_M), m = rank + i * p.cluster;
+                        if (i >= mine) break;
+                        float val = recv_one(recv, p.cluster, slots, i, row) + bias;
+                        if (rr.rotate) {
+                            const float other = recv_one(recv, p.cluster, slots, i, rr.partner) + other_bias;
+                            val = rr.first ? val * cs[u].x - other * cs[u].y : val * cs[u].x + other * cs[u].y;
                         }
-                    }
-                } else {
-#pragma unroll 1
-                    for (int c0 = 0; c0 < BN; c0 += 16) {
-                        float v[16];
-                        load16(c0, v);
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const int m = c0 + j;
-                            float val = v[j] + bias;
-                            if (EPI == DEPI_STORE_F32 || EPI == DEPI_RESIDUAL) val *= llb_out_scale(p.glu);
-                            if (EPI == DEPI_SWIGLU) {
-                                const float other = __shfl_xor_sync(0xffffffffu, val, 1);   // gate: even rows, up: odd rows
-                                if ((lane & 1) == 0 && m < p.M && n + 1 < p.N)
-                                    ((__nv_bfloat16*)p.out)[(size_t)m * (p.N / 2) + (n >> 1)] =
-                                        __float2bfloat16_rn(llb_glu(val, other, p.glu.kind, p.glu.alpha, p.glu.limit, p.glu.up_shift));
-                            } else if (m < p.M && n < p.N) {
-                                const size_t idx = (size_t)m * p.N + n;
-                                if (EPI == DEPI_STORE_F32) ((float*)p.out)[idx] = val;
-                                else if (gridDim.z == 1) p.residual[idx] += val;
-                                else atomicAdd(p.residual + idx, val);
-                            }
+                        const __nv_bfloat16 h = __float2bfloat16_rn(val);
+                        if (n < q_end) {
+                            p.q_out[(size_t)m * q_end + n] = h;
+                        } else if (slot_of[u] >= 0) {
+                            if (n < k_end) p.k_cache[(size_t)slot_of[u] * (p.Hkv * p.hd) + (n - q_end)] = h;
+                            else p.v_cache[(size_t)slot_of[u] * (p.Hkv * p.hd) + (n - k_end)] = h;
                         }
                     }
                 }
-                if (meet && warp == 2 && lane == 0) atomicExch(p.counters + blockIdx.x, 0);
+            } else {
+                const int f = (e & 63) * 2, n = n0 + f;
+                float2 bias = make_float2(0.0f, 0.0f);
+                if (p.bias && piece == 0) {
+                    if (n < p.N) bias.x = p.bias[n];
+                    if (n + 1 < p.N) bias.y = p.bias[n + 1];
+                }
+                const bool alone = (int)gridDim.z == p.cluster;
+                if (n < p.N)
+                    for (int i = e >> 6; i < mine; i += WORKERS / 64)
+                        finish_pair<EPI>(p, recv_pair(recv, p.cluster, slots, i, f), bias, rank + i * p.cluster, n, alone);
             }
         }
     }
@@ -455,35 +507,140 @@ int cached_map(const void* ptr, long long rows, long long cols, int box, CUtenso
     return 0;
 }
 
-size_t smem_bytes(int BN, int stages, int b_tiles) {
-    // the rotary epilogue stages its tile over the weight ring (128 x 65 floats < 8 x 16 KB)
-    return (size_t)stages * A_BYTES + (size_t)b_tiles * BN * TILE_K * 2 + 1024;
+// Operand tiles, and behind them room for what a cluster's blocks send (a block alone uses the ring, which is idle by then).
+size_t tile_bytes(int BN, int stages, int b_tiles) { return (size_t)stages * A_BYTES + (size_t)b_tiles * BN * TILE_K * 2; }
+size_t recv_bytes(int BN, int cluster) { return cluster > 1 ? (size_t)cluster * llb_ceil_div(BN, cluster) * TILE_M * 4 : 0; }
+constexpr size_t SMEM_LIMIT = 224 * 1024;
+
+// How many clusters of `size` blocks of this kernel the device holds at once (asked once a kernel, size and device).
+template <int BN, int EPI, bool NORM, int STAGES>
+int clusters_at_once(int size, size_t smem) {
+    static std::atomic<int> known[64][MAX_CLUSTER + 1] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const bool cached = dev >= 0 && dev < 64;
+    if (cached && known[dev][size].load()) return known[dev][size].load() - 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, size);
+    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = size;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_decode_kernel<BN, EPI, NORM, STAGES>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    if (cached) known[dev][size].store(n + 1);
+    return n;
 }
 
 template <int BN, int EPI, bool NORM, int STAGES>
-int launch_stages(const CUtensorMap& mw, const CUtensorMap& mx, const DecodeGemmParams& p, int split_k, cudaStream_t stream) {
-    const size_t smem = smem_bytes(BN, STAGES, NORM ? p.num_kb : STAGES);
-    LLB_REQUIRE(smem <= 224 * 1024, "gemm_decode: K=%d with %d rows needs %zu bytes of shared memory", p.K, BN, smem);
-    static size_t configured = 0;
-    if (smem > configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_decode_kernel<BN, EPI, NORM, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return llb_fail("gemm_decode: cannot opt in to %zu bytes of shared memory: %s", smem,
-                                              cudaGetErrorString(e));
-        configured = smem;
-    }
-    dim3 grid(llb_ceil_div(p.N, TILE_M), 1, split_k);
-    cudaError_t e = launch_pdl(gemm_decode_kernel<BN, EPI, NORM, STAGES>, grid, dim3(NUM_THREADS), smem, stream, mw, mx, p);
+int configure(size_t smem) {
+    static std::atomic<size_t> configured[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const bool cached = dev >= 0 && dev < 64;
+    if (cached && configured[dev].load() >= smem) return 0;
+    const cudaError_t e = cudaFuncSetAttribute(gemm_decode_kernel<BN, EPI, NORM, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return llb_fail("gemm_decode: cannot opt in to %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    if (cached) configured[dev].store(smem);
+    return 0;
+}
+
+template <int BN, int EPI, bool NORM, int STAGES>
+int launch_stages(const CUtensorMap& mw, const CUtensorMap& mx, DecodeGemmParams p, int cluster, int pieces, cudaStream_t stream) {
+    const int b_tiles = NORM ? p.num_kb : STAGES;
+    const size_t tiles = tile_bytes(BN, STAGES, b_tiles), smem = tiles + recv_bytes(BN, cluster) + 1024;
+    LLB_REQUIRE(smem <= SMEM_LIMIT, "gemm_decode: K=%d with %d rows needs %zu bytes of shared memory", p.K, BN, smem);
+    int rc = configure<BN, EPI, NORM, STAGES>(smem);
+    if (rc) return rc;
+    p.kb_per_split = llb_ceil_div(p.num_kb, cluster * pieces);
+    p.cluster = cluster;
+    p.recv_offset = cluster > 1 ? (uint32_t)tiles : 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(llb_ceil_div(p.N, TILE_M), 1, cluster * pieces);
+    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = 1;
+    at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = cluster;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_decode_kernel<BN, EPI, NORM, STAGES>, mw, mx, p);
     if (e != cudaSuccess) return llb_fail("gemm_decode: launch failed: %s", cudaGetErrorString(e));
     return llb_check_launch("gemm_decode");
 }
 
+int device_sms() {
+    static std::atomic<int> known[64] = {};
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64) sms = known[dev].load();
+    if (sms == 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return 1;
+        if (dev >= 0 && dev < 64) known[dev].store(sms);
+    }
+    return sms;
+}
+
+// K in `pieces` x `cluster` parts.  Asked for a number of parts: clusters of up to 8 of them.  Asked to choose (split_k = 0): the tiles
+// of features alone leave most multiprocessors idle where there are few of them, and a block's part of K then is its time, so the
+// largest clusters that all find a place at once; tiles that fill more than half of the multiprocessors get two blocks each with short
+// rings, two blocks a multiprocessor (9,728 x 896, us with the norm before it: 8 rows 8.7 -> 7.4, 64 rows 12.6 -> 11.3; 17,920 x 1,536 at 27
+// rows 15.0 -> 13.8).  Up to 32 rows the residual is cheap enough to add to from every block, with as many parts as multiprocessors
+// and no meeting (896 x 896, 8 rows 4.2 us; in clusters 19 rows 5.5); 64 rows' additions are not (6.9 -> 6.4).
 template <int BN, int EPI, bool NORM>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const DecodeGemmParams& p, int split_k, cudaStream_t stream) {
+    constexpr int RING = BN == 64 ? MIDDLE : DEEP;          // beside the received sums
+    const int tiles = llb_ceil_div(p.N, TILE_M), sms = device_sms();
+    const bool may_cut = EPI != DEPI_STORE_F32 && !(EPI == DEPI_SWIGLU && p.N % 2);
+    int cluster = 1, pieces = 1;
+    auto even = [&](int parts) { return llb_ceil_div(p.num_kb, llb_ceil_div(p.num_kb, parts)); };          // without empty parts
+    if (may_cut && EPI == DEPI_RESIDUAL && BN <= 32) {
+        pieces = even(split_k > 0 ? (split_k < p.num_kb ? split_k : p.num_kb) : tiles < sms ? (sms / tiles < p.num_kb ? sms / tiles : p.num_kb) : 1);
+    } else if (may_cut) {
+        const int most = split_k > 0 ? split_k : tiles < sms ? sms / tiles : 1;
+        cluster = even(most < p.num_kb ? most : p.num_kb);
+        if (cluster > MAX_CLUSTER) cluster = even(MAX_CLUSTER);
+        const size_t room = tile_bytes(BN, RING, NORM ? p.num_kb : RING) + recv_bytes(BN, MAX_CLUSTER) + 1024;
+        if (cluster > 1 && room > SMEM_LIMIT) cluster = 1;          // (a normed operand that is resident over a long K)
+        if (cluster > 1) {
+            const int rc = configure<BN, EPI, NORM, RING>(room);
+            if (rc) return rc;
+            while (split_k == 0 && cluster > 1 && clusters_at_once<BN, EPI, NORM, RING>(cluster, room) < tiles) cluster = even(cluster - 1);
+            // several clusters along K add into the residual
+            if (EPI == DEPI_RESIDUAL && split_k == 0 && cluster == even(MAX_CLUSTER))
+                while (llb_ceil_div(p.num_kb, cluster * pieces) > 6 && even(cluster * (pieces + 1)) == cluster * (pieces + 1) &&
+                       clusters_at_once<BN, EPI, NORM, RING>(cluster, room) >= tiles * (pieces + 1))
+                    ++pieces;
+        }
+    }
+    if (cluster > 1) return launch_stages<BN, EPI, NORM, RING>(mw, mx, p, cluster, pieces, stream);
+    if constexpr (!NORM && EPI != DEPI_STORE_F32) {
+        // more tiles than half the multiprocessors: two blocks a tile, and two of them on a multiprocessor
+        constexpr int PAIR = BN == 16 ? 5 : BN == 32 ? 4 : 3;
+        constexpr size_t room = (size_t)PAIR * (A_BYTES + BN * TILE_K * 2) + BN * TILE_M * 4 + 1024;
+        if (split_k == 0 && may_cut && pieces == 1 && tiles <= sms && p.num_kb >= 4) {
+            const int rc = configure<BN, EPI, NORM, PAIR>(room);
+            if (rc) return rc;
+            return launch_stages<BN, EPI, NORM, PAIR>(mw, mx, p, 2, 1, stream);
+        }
+    }
     // the float-store epilogue is the head's: a vocabulary's worth of blocks
-    if (EPI == DEPI_STORE_F32 && !NORM && llb_ceil_div(p.N, TILE_M) >= 256)
-        return launch_stages<BN, EPI, NORM, SHALLOW>(mw, mx, p, split_k, stream);
-    return launch_stages<BN, EPI, NORM, DEEP>(mw, mx, p, split_k, stream);
+    if constexpr (EPI == DEPI_STORE_F32 && !NORM)
+        if (tiles >= 256) return launch_stages<BN, EPI, NORM, SHALLOW>(mw, mx, p, 1, pieces, stream);
+    return launch_stages<BN, EPI, NORM, DEEP>(mw, mx, p, 1, pieces, stream);
 }
 
 template <int BN, bool NORM>
@@ -494,6 +651,8 @@ int dispatch_epi(int epi, const CUtensorMap& mw, const CUtensorMap& mx, const De
         case DEPI_RESIDUAL: return launch<BN, DEPI_RESIDUAL, NORM>(mw, mx, p, split_k, s);
         case DEPI_SWIGLU: return launch<BN, DEPI_SWIGLU, NORM>(mw, mx, p, split_k, s);
         case DEPI_ROPE_KV: return launch<BN, DEPI_ROPE_KV, NORM>(mw, mx, p, split_k, s);
+        case DEPI_STORE:
+            if constexpr (!NORM) return launch<BN, DEPI_STORE, false>(mw, mx, p, split_k, s);
     }
     return llb_fail("gemm_decode: unknown epilogue %d", epi);
 }
@@ -513,35 +672,32 @@ LLB_EXPORT int llb_gemm_decode_supports(int M, int N, int K, int norm, int epilo
     if (M < 1 || M > 64 || K % 8 != 0 || N < 1) return 0;
     const int BN = M <= 16 ? 16 : M <= 32 ? 32 : 64;
     const int num_kb = llb_ceil_div(K, TILE_K);
-    if (smem_bytes(BN, DEEP, norm ? num_kb : DEEP) > 224 * 1024) return 0;
+    if (tile_bytes(BN, DEEP, norm ? num_kb : DEEP) + 1024 > SMEM_LIMIT) return 0;
     if (epilogue == DEPI_SWIGLU && N % 2) return 0;
     if (epilogue == DEPI_ROPE_KV && (hd < 2 || TILE_M % hd != 0)) return 0;
+    if (epilogue == DEPI_STORE && norm) return 0;
     return 1;
 }
 
 // W [N, K] bf16 (K a multiple of 8).  Activations: with norm != 0 the float rows x[x_rows[r]] (or x[r])
 // of width K, normalised with norm_w (float, or bf16 when norm_w_bf16) and eps inside the kernel; else
-// a_bf16 [M, K].  Epilogues: 1 store float out[M, N]; 2 add into residual[M, N] (split_k >= 1);
+// a_bf16 [M, K].  Epilogues: 1 store float out[M, N]; 2 add into residual[M, N];
 // 3 SwiGLU out[M, N/2] bf16; 4 rotary + q_out + cache write (N = (Hq + 2 Hkv) * hd; without
 // slot_mapping only q is written and N = Hq * hd); rope_table [M, rotary_dim/2] holds (cos, sin) of each
-// token's angle (llb_rope_table).  split_k > 1 with epilogue 3 or 4 needs acc_scratch (scratch_floats >= BN * N
-// floats, all zero on entry and left zero) and counters (one int per 128 output features, zero on entry and left zero).
+// token's angle (llb_rope_table); 5 store bf16 out[M, N].  split_k: into how many parts K is cut (8 at most where the parts meet in a
+// cluster), 0: as the sizes and the device suggest.
 static int gemm_decode_impl(const void* W, const void* a_bf16, const float* x, const int* x_rows, const void* norm_w,
                             int norm_w_bf16, float eps, int norm, const float* bias, void* out, float* residual,
                             int epilogue, int M, int N, int K, int split_k,
                             const int* slot_mapping, const float* rope_table, int rotary_dim, int interleaved, int Hq,
-                            int Hkv, int hd, void* q_out, void* k_cache, void* v_cache, float* acc_scratch,
-                            long long scratch_floats, int* counters, int* error_flag, LlbGluArgs glu, cudaStream_t stream) {
+                            int Hkv, int hd, void* q_out, void* k_cache, void* v_cache, int* error_flag, LlbGluArgs glu,
+                            cudaStream_t stream) {
     if (M == 0) return 0;
     LLB_REQUIRE(llb_gemm_decode_supports(M, N, K, norm, epilogue, hd), "gemm_decode: unsupported shape M=%d N=%d K=%d", M, N, K);
     LLB_REQUIRE(((uintptr_t)W % 16 == 0), "gemm_decode: weights must be 16-byte aligned");
     LLB_REQUIRE(norm ? (x != nullptr && norm_w != nullptr && (uintptr_t)x % 16 == 0 && (uintptr_t)norm_w % 16 == 0)
                      : (a_bf16 != nullptr && (uintptr_t)a_bf16 % 16 == 0), "gemm_decode: bad activation operand");
-    LLB_REQUIRE(split_k >= 1 && epilogue != DEPI_STORE_F32 || split_k == 1, "gemm_decode: the float-store epilogue takes no split_k");
-    if (split_k > 1 && (epilogue == DEPI_ROPE_KV || epilogue == DEPI_SWIGLU))
-        LLB_REQUIRE(acc_scratch != nullptr && counters != nullptr && scratch_floats >= (long long)(M <= 16 ? 16 : M <= 32 ? 32 : 64) * N,
-                    "gemm_decode: split_k=%d with a fused epilogue needs %lld floats of zeroed scratch and counters",
-                    split_k, (long long)(M <= 16 ? 16 : M <= 32 ? 32 : 64) * N);
+    LLB_REQUIRE(split_k >= 0 && (epilogue != DEPI_STORE_F32 || split_k <= 1), "gemm_decode: the float-store epilogue takes no split_k");
     if (epilogue == DEPI_ROPE_KV) {
         const int hkv = slot_mapping ? Hkv : 0;
         LLB_REQUIRE(N == (Hq + 2 * hkv) * hd && rotary_dim % 2 == 0 && rotary_dim <= hd && q_out &&
@@ -551,13 +707,9 @@ static int gemm_decode_impl(const void* W, const void* a_bf16, const float* x, c
     p.x = x; p.x_rows = x_rows; p.norm_w = norm_w; p.norm_w_bf16 = norm_w_bf16; p.eps = eps;
     p.bias = bias; p.out = out; p.residual = residual; p.M = M; p.N = N; p.K = K;
     p.num_kb = llb_ceil_div(K, TILE_K);
-    if (split_k > p.num_kb) split_k = p.num_kb;
-    p.kb_per_split = llb_ceil_div(p.num_kb, split_k);
-    split_k = llb_ceil_div(p.num_kb, p.kb_per_split);
     p.slot_mapping = slot_mapping; p.rope_table = (const float2*)rope_table; p.rotary_dim = rotary_dim;
     p.interleaved = interleaved; p.Hq = Hq; p.Hkv = slot_mapping ? Hkv : 0; p.hd = hd;
     p.q_out = (__nv_bfloat16*)q_out; p.k_cache = (__nv_bfloat16*)k_cache; p.v_cache = (__nv_bfloat16*)v_cache;
-    p.acc_scratch = acc_scratch; p.counters = counters;
     p.error_flag = error_flag;
     p.glu = glu;
     CUtensorMap mw, mx;
@@ -576,22 +728,21 @@ LLB_EXPORT int llb_gemm_decode(const void* W, const void* a_bf16, const float* x
                                int norm_w_bf16, float eps, int norm, const float* bias, void* out, float* residual,
                                int epilogue, int M, int N, int K, int split_k,
                                const int* slot_mapping, const float* rope_table, int rotary_dim, int interleaved, int Hq,
-                               int Hkv, int hd, void* q_out, void* k_cache, void* v_cache, float* acc_scratch,
-                               long long scratch_floats, int* counters, int* error_flag, cudaStream_t stream) {
+                               int Hkv, int hd, void* q_out, void* k_cache, void* v_cache, int* error_flag, cudaStream_t stream) {
     return gemm_decode_impl(W, a_bf16, x, x_rows, norm_w, norm_w_bf16, eps, norm, bias, out, residual, epilogue, M, N, K,
                             split_k, slot_mapping, rope_table, rotary_dim, interleaved, Hq, Hkv, hd, q_out, k_cache, v_cache,
-                            acc_scratch, scratch_floats, counters, error_flag, llb_glu_silu(), stream);
+                            error_flag, llb_glu_silu(), stream);
 }
 
-// The GLU epilogue (bf16 operand, no norm prologue) with another gated activation (LLB_GLU_*, see llb_glu).
-LLB_EXPORT int llb_gemm_decode_glu(const void* W, const void* a_bf16, const float* bias, void* out, int M, int N, int K,
-                                   int split_k, float* acc_scratch, long long scratch_floats, int* counters,
-                                   int* error_flag, int glu_kind, float glu_alpha, float glu_limit, float glu_up_shift,
+// The GLU epilogue with another gated activation (LLB_GLU_*, see llb_glu), or the store epilogue with a plain one (a kind of LlbAct,
+// else none); bf16 operand, no norm prologue.
+LLB_EXPORT int llb_gemm_decode_glu(const void* W, const void* a_bf16, const float* bias, void* out, int epilogue, int M, int N, int K,
+                                   int split_k, int* error_flag, int glu_kind, float glu_alpha, float glu_limit, float glu_up_shift,
                                    cudaStream_t stream) {
-    return gemm_decode_impl(W, a_bf16, nullptr, nullptr, nullptr, 0, 0.0f, 0, bias, out, nullptr, DEPI_SWIGLU, M, N, K,
-                            split_k, nullptr, nullptr, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr, acc_scratch,
-                            scratch_floats, counters, error_flag, LlbGluArgs{glu_kind, glu_alpha, glu_limit, glu_up_shift},
-                            stream);
+    LLB_REQUIRE(epilogue == DEPI_SWIGLU || epilogue == DEPI_STORE, "gemm_decode_glu: epilogue %d takes no activation", epilogue);
+    return gemm_decode_impl(W, a_bf16, nullptr, nullptr, nullptr, 0, 0.0f, 0, bias, out, nullptr, epilogue, M, N, K,
+                            split_k, nullptr, nullptr, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr, error_flag,
+                            LlbGluArgs{glu_kind, glu_alpha, glu_limit, glu_up_shift}, stream);
 }
 
 // The float-store and residual epilogues (bf16 operand, no norm prologue) with every output (bias included) times `scale`.
@@ -600,6 +751,6 @@ LLB_EXPORT int llb_gemm_decode_scaled(const void* W, const void* a_bf16, const f
                                       cudaStream_t stream) {
     LLB_REQUIRE(epilogue == DEPI_STORE_F32 || epilogue == DEPI_RESIDUAL, "gemm_decode_scaled: epilogue %d takes no scale", epilogue);
     return gemm_decode_impl(W, a_bf16, nullptr, nullptr, nullptr, 0, 0.0f, 0, bias, out, residual, epilogue, M, N, K,
-                            split_k, nullptr, nullptr, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, 0, nullptr,
-                            error_flag, LlbGluArgs{LLB_OUT_SCALE, scale, 0.0f, 0.0f}, stream);
+                            split_k, nullptr, nullptr, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr, error_flag,
+                            LlbGluArgs{LLB_OUT_SCALE, scale, 0.0f, 0.0f}, stream);
 }

@@ -56,7 +56,6 @@ namespace {
 constexpr int F32 = 0, BF16 = 1;                 // the library's dtype codes
 constexpr int PAGE = 16;                         // tokens of a cache page
 constexpr int EXPECTED_ABI = 25;
-constexpr int DECODE_ROWS = 64;                  // rows that the fused decode contractions take (their meeting place is sized for it)
 constexpr int CLUSTER_MERGE_MAX_KEYS = 8192;     // up to here the decode attention merges its pieces inside a cluster
 
 [[noreturn]] void die(const std::string& what) {
@@ -643,11 +642,6 @@ int main(int argc, char** argv) {
     const int max_T = opt.max_batch_tokens + nreq;
     float* residual = (float*)dev.alloc((size_t)max_T * D * 4);
     float* logits = (float*)dev.alloc((size_t)nreq * V * 4);
-    const int Nqkv = (cfg.heads + 2 * cfg.kv_heads) * hd, widest = std::max(Nqkv, 2 * cfg.intermediate);
-    const long long splitk_floats = (long long)DECODE_ROWS * widest;
-    float* splitk = (float*)dev.alloc((size_t)splitk_floats * 4, true);
-    const int splitk_tiles = ceil_div(widest, 128);
-    int* splitk_counters = (int*)dev.alloc((size_t)splitk_tiles * 4, true);
     const int meet_n = 1 << 16;
     int* meet = (int*)dev.alloc((size_t)meet_n * 4, true);
     int* flags = (int*)dev.alloc(2 * 4, true);           // [0] raised by a kernel whose wait ran out, [1] by a token id out of range
@@ -829,10 +823,6 @@ int main(int argc, char** argv) {
         step.residual = residual;
         step.plans = &plan;
         step.num_plans = 1;
-        step.splitk_scratch = splitk;
-        step.splitk_floats = splitk_floats;
-        step.splitk_counters = splitk_counters;
-        step.splitk_tiles = splitk_tiles;
         step.meet_counters = meet;
         step.meet_counters_n = meet_n;
         step.error_flag = flags;

@@ -1093,7 +1093,7 @@ def gemm_tcgen05_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ep
                                           _ptr(async_error_flag(a.device)), *_glu_args(glu), _stream()))
 
 
-DEPI_STORE_F32, DEPI_RESIDUAL, DEPI_SWIGLU, DEPI_ROPE_KV = 1, 2, 3, 4
+DEPI_STORE_F32, DEPI_RESIDUAL, DEPI_SWIGLU, DEPI_ROPE_KV, DEPI_STORE = 1, 2, 3, 4, 5
 
 
 def rope_table(positions: torch.Tensor, inv_freq: torch.Tensor, transposed: bool = False) -> torch.Tensor:
@@ -1112,10 +1112,8 @@ _splitk_retired = []     # meeting places that a larger one replaced: CUDA graph
 
 
 def reserve_splitk_scratch(device: torch.device, floats: int, tiles: int) -> None:
-    """Make sure the device has a zeroed meeting place of ``floats`` floats and ``tiles`` counters for
-    split-K contractions with fused epilogues.  Call it when a model is bound, never inside a step.
-    A meeting place that a larger one replaces is kept alive (and zero, as every launch leaves it): a graph
-    captured while it was current goes on adding into it."""
+    """A zeroed place of ``floats`` floats and ``tiles`` counters on the device (a larger one replaces a smaller, which is kept
+    alive).  The contractions of this library need none: their parts along K meet in shared memory."""
     key = torch.device(device).index or 0
     have = _splitk.get(key)
     if have is None or have[0].numel() < floats or have[1].numel() < tiles:
@@ -1148,7 +1146,8 @@ def gemm_decode(w: torch.Tensor, epilogue: int, M: int, *, a: Optional[torch.Ten
     Operand: ``a`` [M, K] bf16, or the float rows ``x[x_rows]`` (``x[:M]`` without ``x_rows``) to be
     RMS-normalised with ``norm_weight`` and ``eps`` inside the kernel.  Epilogues: DEPI_STORE_F32
     (``out`` float [M, N]), DEPI_RESIDUAL (adds into ``residual``), DEPI_SWIGLU (``out`` bf16 [M, N/2]),
-    DEPI_ROPE_KV (rotary by ``rope_table`` from :func:`rope_table`, ``q_out`` and the cache rows ``slot_mapping``)."""
+    DEPI_ROPE_KV (rotary by ``rope_table`` from :func:`rope_table`, ``q_out`` and the cache rows ``slot_mapping``).
+    ``split_k``: into how many parts K is cut; 0 lets the sizes and the device decide."""
     N, K = w.shape
     if w.dtype != torch.bfloat16:
         raise KernelError("gemm_decode takes bfloat16 weights")
@@ -1174,17 +1173,13 @@ def gemm_decode(w: torch.Tensor, epilogue: int, M: int, *, a: Optional[torch.Ten
             raise KernelError("gemm_decode: rope_table must be float32 [M, rotary_dim/2, 2]")
         if slot_mapping is not None and (k_cache is None or v_cache is None or k_cache.dtype != torch.bfloat16):
             raise KernelError("gemm_decode: the cache must be bfloat16")
-    scratch = splitk_scratch(w.device) if (split_k > 1 and epilogue in (DEPI_SWIGLU, DEPI_ROPE_KV)) else None
-    if scratch is not None and scratch[1].numel() < -(-N // 128):
-        scratch = None
     _check(lib().llb_gemm_decode(
         _ptr(w), _ptr(a), _ptr(x), _i32(x_rows, "x_rows"), _ptr(norm_weight),
         1 if (norm_weight is not None and norm_weight.dtype == torch.bfloat16) else 0, ctypes.c_float(eps),
         1 if norm else 0, _ptr(bias), _ptr(out), _ptr(residual), epilogue, M, N, K, split_k,
         _i32(slot_mapping, "slot_mapping"), _ptr(rope_table), rotary_dim,
         1 if interleaved else 0, num_heads, num_kv_heads, head_dim, _ptr(q_out), _ptr(k_cache), _ptr(v_cache),
-        _ptr(scratch[0]) if scratch else ctypes.c_void_p(0), ctypes.c_longlong(scratch[0].numel() if scratch else 0),
-        _ptr(scratch[1]) if scratch else ctypes.c_void_p(0), _ptr(async_error_flag(w.device)), _stream()))
+        _ptr(async_error_flag(w.device)), _stream()))
 
 
 def gemm_decode_scaled(w: torch.Tensor, epilogue: int, a: torch.Tensor, scale: float, bias: Optional[torch.Tensor] = None,
@@ -1214,15 +1209,22 @@ def gemm_decode_glu(w: torch.Tensor, a: torch.Tensor, bias: Optional[torch.Tenso
         raise KernelError("gemm_decode_glu: bfloat16 a [M,K], w [N,K] and out [M,N/2]")
     if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N):
         raise KernelError(f"gemm_decode_glu: bias must be float32 [{N}]")
-    scratch = splitk_scratch(w.device) if split_k > 1 else None
-    if scratch is not None and (scratch[1].numel() < -(-N // 128) or scratch[0].numel() < 64 * N):
-        scratch = None
-    if scratch is None:          # no meeting place was reserved for a contraction this wide: one piece
-        split_k = 1
-    _check(lib().llb_gemm_decode_glu(
-        _ptr(w), _ptr(a), _ptr(bias), _ptr(out), M, N, K, split_k,
-        _ptr(scratch[0]) if scratch else ctypes.c_void_p(0), ctypes.c_longlong(scratch[0].numel() if scratch else 0),
-        _ptr(scratch[1]) if scratch else ctypes.c_void_p(0), _ptr(async_error_flag(w.device)), *_glu_args(glu), _stream()))
+    _check(lib().llb_gemm_decode_glu(_ptr(w), _ptr(a), _ptr(bias), _ptr(out), DEPI_SWIGLU, M, N, K, split_k,
+                                     _ptr(async_error_flag(w.device)), *_glu_args(glu), _stream()))
+
+
+def gemm_decode_store(w: torch.Tensor, a: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, glu=None, split_k: int = 0) -> None:
+    """``out`` bf16 [M, N] = ``a`` bf16 [M, K] @ ``w`` bf16 [N, K]^T + ``bias`` for at most 64 rows, through the plain activation that ``glu``
+    names (``(ACT_SQUARED_RELU, ...)``)."""
+    N, K = w.shape
+    M = a.shape[0]
+    if w.dtype != torch.bfloat16 or a.dtype != torch.bfloat16 or tuple(a.shape) != (M, K) \
+            or out.dtype != torch.bfloat16 or tuple(out.shape) != (M, N):
+        raise KernelError("gemm_decode_store: bfloat16 a [M,K], w [N,K] and out [M,N]")
+    if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N):
+        raise KernelError(f"gemm_decode_store: bias must be float32 [{N}]")
+    _check(lib().llb_gemm_decode_glu(_ptr(w), _ptr(a), _ptr(bias), _ptr(out), DEPI_STORE, M, N, K, split_k,
+                                     _ptr(async_error_flag(w.device)), *_glu_args(glu), _stream()))
 
 
 def attention_tcgen05_supports(head_dim: int, page_size: int) -> bool:

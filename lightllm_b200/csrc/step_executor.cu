@@ -34,8 +34,7 @@ int llb_gemm_decode_supports(int M, int N, int K, int norm, int epilogue, int hd
 int llb_gemm_decode(const void* W, const void* a_bf16, const float* x, const int* x_rows, const void* norm_w, int norm_w_bf16,
                     float eps, int norm, const float* bias, void* out, float* residual, int epilogue, int M, int N, int K,
                     int split_k, const int* slot_mapping, const float* rope_table, int rotary_dim, int interleaved, int Hq,
-                    int Hkv, int hd, void* q_out, void* k_cache, void* v_cache, float* acc_scratch, long long scratch_floats,
-                    int* counters, int* error_flag, cudaStream_t stream);
+                    int Hkv, int hd, void* q_out, void* k_cache, void* v_cache, int* error_flag, cudaStream_t stream);
 int llb_gemm_simt(const void* A, int a_dtype, const void* W, const void* bias, int w_dtype, void* out, float* residual,
                   int epilogue, int M, int N, int K, void* scratch, long long scratch_bytes, int* error_flag, cudaStream_t stream);
 long long llb_gemm_simt_scratch_bytes(int a_dtype, int w_dtype, int M, int N, int K);
@@ -59,9 +58,8 @@ namespace {
 
 // The thresholds of the Python parts (parts/linear.py, parts/attention.py); a test runs both paths side by side.
 constexpr int DECODE_ROWS = 64;             // steps of at most this many rows use the fused decode contraction
-constexpr int FUSED_ROPE_MAX_ROWS = 16;     // up to here the projection's decode kernel rotates and writes the cache itself
-constexpr int PREFILL_ROPE_MIN_ROWS = 16;   // beyond, the tensor-core projection does (heads of 64 or 128)
-constexpr int DEPI_STORE_F32 = 1, DEPI_RESIDUAL = 2, DEPI_SWIGLU = 3, DEPI_ROPE_KV = 4;
+constexpr int PREFILL_ROPE_MIN_ROWS = 16;   // beyond, the tensor-core projection rotates and writes the cache (heads of 64 or 128)
+constexpr int DEPI_STORE_F32 = 1, DEPI_RESIDUAL = 2, DEPI_SWIGLU = 3, DEPI_ROPE_KV = 4, DEPI_STORE = 5;
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 inline int imin(int a, int b) { return a < b ? a : b; }
@@ -95,11 +93,6 @@ struct Exec {
 
     // ---- parts/linear.py ------------------------------------------------------------------------------------------
     int split_k_for(int N, int K) const { return imax(1, imin(ceil_div(K, 64), m.num_sms / ceil_div(N, 128))); }
-    int split_k_fused(int M, int N, int K) const {
-        const int tiles = ceil_div(N, 128);
-        if (M > 16 || tiles * 4 > m.num_sms) return 1;
-        return imax(1, imin(ceil_div(K, 64), m.num_sms / tiles));
-    }
     int split_k_wide(int M, int N, int K) const {
         const int tiles = ceil_div(M, 128) * ceil_div(N, N > 128 ? 256 : 128);
         if (tiles * 2 > m.num_sms) return 1;
@@ -108,25 +101,15 @@ struct Exec {
     bool decode_eligible(int M, int N, int K, int depi, int hd) const {
         return M <= DECODE_ROWS && bf16 && llb_gemm_decode_supports(M, N, K, 0, depi, hd);
     }
-    float* splitk_for(int N, int split, int depi) const {      // the meeting place of a split fused epilogue, if it is large enough
-        if (split > 1 && (depi == DEPI_SWIGLU || depi == DEPI_ROPE_KV) && s.splitk_scratch && s.splitk_tiles >= ceil_div(N, 128))
-            return s.splitk_scratch;
-        return nullptr;
-    }
 
     // out = x W^T (+ bias) with the epilogue; x [M, K] in the activation dtype
     int linear(const void* x, const void* w, const float* bias, int epi, void* out, float* residual, int M, int N, int K) {
         const int depi = epi == LLB_EPI_STORE_F32 ? DEPI_STORE_F32 : epi == LLB_EPI_RESIDUAL ? DEPI_RESIDUAL
-                         : epi == LLB_EPI_SWIGLU ? DEPI_SWIGLU : 0;
-        if (depi && decode_eligible(M, N, K, depi, 0)) {
-            int split = 1;
-            if (epi == LLB_EPI_RESIDUAL) split = split_k_for(N, K);
-            else if (epi == LLB_EPI_SWIGLU) split = split_k_fused(M, N, K);
-            float* sc = splitk_for(N, split, depi);
+                         : epi == LLB_EPI_SWIGLU ? DEPI_SWIGLU : DEPI_STORE;
+        if (decode_eligible(M, N, K, depi, 0)) {
             if (dry) return 0;
-            return llb_gemm_decode(w, x, nullptr, nullptr, nullptr, 0, 0.0f, 0, bias, out, residual, depi, M, N, K, split, nullptr,
-                                   nullptr, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr, sc, sc ? s.splitk_floats : 0,
-                                   sc ? s.splitk_counters : nullptr, s.error_flag, s.stream);
+            return llb_gemm_decode(w, x, nullptr, nullptr, nullptr, 0, 0.0f, 0, bias, out, residual, depi, M, N, K, 0, nullptr,
+                                   nullptr, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr, s.error_flag, s.stream);
         }
         if (bf16 && K % 8 == 0) {
             int split = M > 128 ? split_k_wide(M, N, K) : (epi == LLB_EPI_RESIDUAL ? split_k_for(N, K) : 1);
@@ -173,7 +156,7 @@ struct Exec {
     int projection_path(const LlbAttentionDesc& a) const {
         const int hd = a.head_dim, N = (a.num_heads + (a.writes ? 2 * a.num_kv_heads : 0)) * hd;
         const bool rotary = a.inv_freq != nullptr;
-        if (rotary && bf16 && s.T <= FUSED_ROPE_MAX_ROWS && decode_eligible(s.T, N, m.hidden, DEPI_ROPE_KV, hd)) return 1;
+        if (rotary && bf16 && decode_eligible(s.T, N, m.hidden, DEPI_ROPE_KV, hd)) return 1;
         if (rotary && bf16 && s.T > PREFILL_ROPE_MIN_ROWS && a.writes && (hd == 64 || hd == 128) && m.hidden % 8 == 0 &&
             a.rotary_dim == hd && !a.interleaved)
             return 2;
@@ -193,13 +176,10 @@ struct Exec {
         const int path = projection_path(a);
         if (path == 1) {
             // few rows: projection, bias, rotation and cache write in the decode contraction
-            const int split = split_k_fused(T, N, D);
-            float* sc = splitk_for(N, split, DEPI_ROPE_KV);
             if (!dry)
                 rc = llb_gemm_decode(a.w_qkv, x, nullptr, nullptr, nullptr, 0, 0.0f, 0, a.b_qkv, nullptr, nullptr, DEPI_ROPE_KV, T, N, D,
-                                     split, slots, a.rotary_dim ? table_of(a, false) : nullptr, a.rotary_dim, a.interleaved, hq, hkv,
-                                     hd, q, kc, vc, sc, sc ? s.splitk_floats : 0, sc ? s.splitk_counters : nullptr, s.error_flag,
-                                     s.stream);
+                                     0, slots, a.rotary_dim ? table_of(a, false) : nullptr, a.rotary_dim, a.interleaved, hq, hkv,
+                                     hd, q, kc, vc, s.error_flag, s.stream);
         } else if (path == 2) {
             // a long portion: the same in the epilogue of the tensor-core contraction
             if (!dry)

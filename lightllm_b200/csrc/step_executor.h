@@ -103,18 +103,14 @@ typedef struct {
     void* workspace;               // activations, tables and scratch of the step
     long long workspace_bytes;
     const LlbAttentionPlan* plans;
-    float* splitk_scratch;         // the zeroed meeting place of the fused decode contractions (or null)
-    long long splitk_floats;
-    int* splitk_counters;
     int* meet_counters;            // the zeroed counters of wide split contractions (or null)
     int* error_flag;               // raised by kernels whose waits ran out
     cudaStream_t stream;
-    int splitk_tiles, meet_counters_n;
+    int meet_counters_n;
     int T, S;
     int max_pages, page_size;
     int num_plans;
     int first_layer, last_layer;   // run entries [first, last)
-    int pad_;
 } LlbStepArgs;
 
 // Runs the run entries [first_layer, last_layer) over the step.  0, or a negative code with llb_last_error().

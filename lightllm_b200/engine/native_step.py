@@ -65,10 +65,9 @@ class AttentionPlan(ctypes.Structure):
 class StepArgs(ctypes.Structure):
     _fields_ = [("token_ids", _P), ("positions", _P), ("span_row", _P), ("span_len", _P), ("span_pos", _P),
                 ("block_tables", _P * MAX_GROUPS), ("slot_mapping", _P * MAX_GROUPS), ("residual", _P), ("workspace", _P),
-                ("workspace_bytes", _LL), ("plans", _P), ("splitk_scratch", _P), ("splitk_floats", _LL),
-                ("splitk_counters", _P), ("meet_counters", _P), ("error_flag", _P), ("stream", _P), ("splitk_tiles", _I),
-                ("meet_counters_n", _I), ("T", _I), ("S", _I), ("max_pages", _I), ("page_size", _I), ("num_plans", _I),
-                ("first_layer", _I), ("last_layer", _I), ("pad_", _I)]
+                ("workspace_bytes", _LL), ("plans", _P), ("meet_counters", _P),
+                ("error_flag", _P), ("stream", _P), ("meet_counters_n", _I), ("T", _I), ("S", _I), ("max_pages", _I), ("page_size", _I), ("num_plans", _I),
+                ("first_layer", _I), ("last_layer", _I)]
 
 
 _STRUCTS = (NormDesc, AttentionDesc, MlpDesc, LayerDesc, ModelDesc, TileList, AttentionPlan, StepArgs)
@@ -229,12 +228,6 @@ class NativeLayers:
             s.block_tables[g], s.slot_mapping[g] = bt.data_ptr(), sm.data_ptr()
         s.residual = residual.data_ptr()
         s.plans, s.num_plans = ctypes.addressof(self._plans), len(self._plan_keys)
-        sk = ops.splitk_scratch(self.device)
-        if sk is not None:
-            s.splitk_scratch, s.splitk_floats, s.splitk_counters, s.splitk_tiles = (sk[0].data_ptr(), sk[0].numel(),
-                                                                                   sk[1].data_ptr(), sk[1].numel())
-        else:
-            s.splitk_scratch, s.splitk_floats, s.splitk_counters, s.splitk_tiles = None, 0, None, 0
         s.meet_counters, s.meet_counters_n = self._meet.data_ptr(), self._meet.numel()
         s.error_flag = ops.async_error_flag(self.device).data_ptr()
         s.stream = ops.current_stream()

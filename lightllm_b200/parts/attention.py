@@ -19,7 +19,6 @@ _SMEM_BUDGET = 100 * 1024
 # portion masked): one block of the CUDA-core kernel walking a portion's keys takes hundreds of microseconds from a
 # few hundred keys on, an item of the tensor-core kernel about two per 128 keys.
 TENSOR_CORE_MIN_ROWS = 2
-FUSED_ROPE_MAX_ROWS = 16
 # Where the tensor-core kernels do not apply (float32, other head sizes): a portion of fewer than FEW_ROWS rows over
 # MANY_KEYS keys or more is walked row by row with each row's keys in pieces, not by one block per tile of rows.
 FEW_ROWS = 32
@@ -135,7 +134,6 @@ class AttentionMixer(Mixer):
         if self.out_bias:
             self.b_o = tensors[self._n("o", "bias")].float().contiguous()
         self.position.bind(tensors, dtype, device)
-        L.reserve_fused_scratch(device, self.w_qkv.shape[0])
 
     # ------------------------------------------------------------------------------------------
     accepts_lazy_norm = True
@@ -155,15 +153,13 @@ class AttentionMixer(Mixer):
         act_dtype = x.norm.out_dtype if lazy else x.dtype
         hq, hkv, hd = self.num_heads, self.num_kv_heads, self.head_dim
         w = self.w_qkv if cache.writes else self.w_qkv[: hq * hd]
-        # Beyond 16 rows the per-row loop of the rotary epilogue costs more than a separate rotation kernel
-        # (measured at 64 rows: 25 us fused, 14 us apart).
-        if T > FUSED_ROPE_MAX_ROWS or not L.decode_eligible(T, w, act_dtype, lazy, ops.DEPI_ROPE_KV, hd):
+        if not L.decode_eligible(T, w, act_dtype, lazy, ops.DEPI_ROPE_KV, hd):
             return None
         b = self.b_qkv if (cache.writes or self.b_qkv is None) else self.b_qkv[: hq * hd]
         inv_freq, rotary_dim, interleaved = table
         q = torch.empty((T, hq * hd), dtype=torch.bfloat16, device=w.device)
         operand = dict(x=x.residual, norm_weight=rms[0], eps=rms[1]) if lazy else dict(a=x)
-        ops.gemm_decode(w, ops.DEPI_ROPE_KV, T, bias=b, split_k=L.split_k_fused(T, w.shape[0], w.shape[1]),
+        ops.gemm_decode(w, ops.DEPI_ROPE_KV, T, bias=b, split_k=0,
                         slot_mapping=ctx.slot_mapping[cache.group] if cache.writes else None,
                         rope_table=self.position.step_table(ctx) if rotary_dim else None,
                         rotary_dim=rotary_dim, interleaved=interleaved, num_heads=hq, num_kv_heads=hkv, head_dim=hd,
@@ -366,7 +362,7 @@ class AttentionMixer(Mixer):
                                      ctx.block_tables[g], ctx.max_pages, ctx.page_size, self.num_heads,
                                      self.num_kv_heads, self.head_dim, window, self.scale, nsplit, None, sinks=self.sinks,
                                      cross=self.value_cross, softcap=self.softcap or 0.0, keep=self.keep_first,
-                                 slopes=self.slopes)
+                                     slopes=self.slopes)
             for tiles, bq, nsplit in simt:
                 self._simt(q, cache, out, tiles, common, bq, nsplit)
 

@@ -3,7 +3,9 @@
 ``y = x @ W^T`` with ``W`` stored ``[out, in]`` as in the checkpoint
 (src/engine/engine_server.cpp:1542-1544).  Which kernel runs depends on dtype and shape only:
 
-* float32 activations: the CUDA-core FFMA kernels (true 32-bit, no tensor cores);
+* float32 activations: the CUDA-core FFMA kernels, or for more rows and work the tensor cores on operands split into bf16
+  numbers that add up to them (32-bit accuracy either way, no TF32);
+* bfloat16 activations and weights, at most 64 rows: the decode contraction, K cut among the blocks of a cluster;
 * bfloat16 activations and weights, rows of 16-byte multiples, more than a few rows:
   the tcgen05 tensor-core kernel with TMEM accumulators;
 * everything else (few rows, odd inner sizes, float32 weights under bfloat16 activations):
@@ -59,16 +61,6 @@ def split_k_for(M: int, N: int, K: int) -> int:
     return max(1, min(kblocks, num_sms() // tiles))
 
 
-def split_k_fused(M: int, N: int, K: int) -> int:
-    """Splits for a decode contraction whose epilogue is fused (the splits meet in scratch).  Meeting
-    costs three more round trips to memory, so it only pays when the grid would otherwise leave most
-    SMs idle (the q/k/v projection: 9 blocks), and only for few rows, where the atomic adds are cheap."""
-    tiles, kblocks = -(-N // 128), -(-K // 64)
-    if M > 16 or tiles * 4 > num_sms():
-        return 1
-    return max(1, min(kblocks, num_sms() // tiles))
-
-
 def split_k_wide(M: int, N: int, K: int) -> int:
     """Splits for a contraction of more than 128 rows.  A block's time is its number of tensor-core
     instructions (K/16 per tile, whatever the tile's width), so when the tiles of 128 rows x 256 features
@@ -80,13 +72,7 @@ def split_k_wide(M: int, N: int, K: int) -> int:
     return max(1, min(num_sms() // tiles, -(-K // 64) // 16))
 
 
-def reserve_fused_scratch(device: torch.device, N: int) -> None:
-    """Called when a part with a fused decode contraction of N output features is bound."""
-    if torch.device(device).type == "cuda":
-        ops.reserve_splitk_scratch(device, DECODE_ROWS * N, -(-N // 128))
-
-
-_DECODE_EPI = {STORE_F32: ops.DEPI_STORE_F32, RESIDUAL: ops.DEPI_RESIDUAL, SWIGLU: ops.DEPI_SWIGLU}
+_DECODE_EPI = {STORE_F32: ops.DEPI_STORE_F32, RESIDUAL: ops.DEPI_RESIDUAL, SWIGLU: ops.DEPI_SWIGLU, STORE: ops.DEPI_STORE}
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, epilogue: int = STORE,
@@ -110,17 +96,15 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         glu = (ops.OUT_SCALE, scale, 0.0, 0.0)
 
     if epilogue in _DECODE_EPI and decode_eligible(M, w, x.dtype, False, _DECODE_EPI[epilogue]):
-        split_k = 1
-        if epilogue == RESIDUAL:
-            split_k = split_k_for(M, N, x.shape[1])
-        elif epilogue == SWIGLU:
-            split_k = split_k_fused(M, N, x.shape[1])
-        if epilogue == SWIGLU and glu is not None:
-            ops.gemm_decode_glu(w, x, bias, out, split_k, glu)
+        # (the kernel's launch cuts K as the sizes and the device suggest)
+        if epilogue == STORE:
+            ops.gemm_decode_store(w, x, bias, out, glu)
+        elif epilogue == SWIGLU and glu is not None:
+            ops.gemm_decode_glu(w, x, bias, out, 0, glu)
         elif scale != 1.0:
-            ops.gemm_decode_scaled(w, _DECODE_EPI[epilogue], x, scale, bias=bias, out=out, residual=residual, split_k=split_k)
+            ops.gemm_decode_scaled(w, _DECODE_EPI[epilogue], x, scale, bias=bias, out=out, residual=residual, split_k=0)
         else:
-            ops.gemm_decode(w, _DECODE_EPI[epilogue], M, a=x, bias=bias, out=out, residual=residual, split_k=split_k)
+            ops.gemm_decode(w, _DECODE_EPI[epilogue], M, a=x, bias=bias, out=out, residual=residual, split_k=0)
     elif tensor_core_eligible(x, w):
         if M > 128:
             split_k = split_k_wide(M, N, x.shape[1])
@@ -150,13 +134,12 @@ def linear_normed(lazy, w: torch.Tensor, bias: Optional[torch.Tensor], epilogue:
     """``linear`` on a LazyNorm input: the norm runs inside the contraction when the shape allows."""
     M, N = lazy.num_rows, w.shape[0]
     rms = lazy.fusable()
-    if rms is not None and epilogue in _DECODE_EPI and 0 < M <= FUSE_NORM_MAX_ROWS and w.shape[1] <= FUSE_NORM_MAX_COLS and \
+    if rms is not None and epilogue != STORE and 0 < M <= FUSE_NORM_MAX_ROWS and w.shape[1] <= FUSE_NORM_MAX_COLS and \
             decode_eligible(M, w, lazy.norm.out_dtype, True, _DECODE_EPI[epilogue]):
         cols = N // 2 if epilogue == SWIGLU else N
         out = torch.empty((M, cols), dtype=torch.float32 if epilogue == STORE_F32 else torch.bfloat16,
                           device=w.device)
         ops.gemm_decode(w, _DECODE_EPI[epilogue], M, x=lazy.residual, x_rows=lazy.rows, norm_weight=rms[0],
-                        eps=rms[1], bias=bias, out=out,
-                        split_k=split_k_fused(M, N, w.shape[1]) if epilogue == SWIGLU else 1)
+                        eps=rms[1], bias=bias, out=out, split_k=0)
         return out
     return linear(lazy.materialize(), w, bias, epilogue)

@@ -62,7 +62,6 @@ class GatedMLP(FeedForward):
         I, D = g.shape
         self.w_gate_up = torch.stack([g.to(wdt), u.to(wdt)], dim=1).reshape(2 * I, D).contiguous()
         self.w_down = tensors[self._n("down", "weight")]
-        L.reserve_fused_scratch(device, 2 * I)
         if self.bias:
             bg, bu = tensors[self._n("gate", "bias")].float(), tensors[self._n("up", "bias")].float()
             self.b_gate_up = torch.stack([bg, bu], dim=1).reshape(2 * I).contiguous()

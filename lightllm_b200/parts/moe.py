@@ -148,7 +148,6 @@ class RoutedExperts(FeedForward):
             wdt = torch.float32 if torch.float32 in (g.dtype, u.dtype) else g.dtype
             self.w_shared_gate_up = torch.stack([g.to(wdt), u.to(wdt)], dim=1).reshape(2 * self.shared["size"], D).contiguous()
             self.w_shared_down = tensors[self._s("down")]
-            L.reserve_fused_scratch(device, 2 * self.shared["size"])
         if E == 0:
             return
         gates, ups = [tensors[self._e(e, "gate")] for e in range(E)], [tensors[self._e(e, "up")] for e in range(E)]
@@ -162,7 +161,6 @@ class RoutedExperts(FeedForward):
         if wdt == torch.bfloat16 and dtype == torch.bfloat16 and self.top < self.outputs and D % 8 == 0 and I % 8 == 0:
             self.w_down_rows = torch.cat(downs, dim=0).contiguous()                     # [E * D, I]: expert by expert
             self._iota = torch.arange(max(E, self.top), dtype=torch.int32, device=device)          # each pair's own row, pair by pair
-        L.reserve_fused_scratch(device, E * 2 * I)
 
     def route(self, x):
         """(ids [T, top] int32, -1 for an identity expert; weights [T, top]; dense weights [T, experts]; the summed weights

@@ -209,6 +209,63 @@ def test_gemm_decode(ops, M, N, K, norm, epi):
         assert torch.allclose(got, ref, atol=tol * scale, rtol=0), f"max diff {float((got - ref).abs().max())}"
 
 
+# (tiles of features, blocks of 64 along K): one block alone, clusters of every size, several clusters into one residual, more tiles
+# than multiprocessors; rows at the edges of 16, 32 and 64 and fewer than a cluster's blocks
+@pytest.mark.parametrize("M", [1, 3, 16, 17, 31, 64])
+@pytest.mark.parametrize("N,K", [(126, 64), (127, 136), (384, 896), (1150, 4864), (2304, 200), (19200, 72)])
+@pytest.mark.parametrize("epi", ["store", "relu", "residual", "swiglu"])
+@pytest.mark.parametrize("split_k", [0, 2, 5, 8])
+def test_gemm_decode_clusters(ops, M, N, K, epi, split_k):
+    """The parts of K that meet in a cluster's shared memory, against float64."""
+    if epi == "swiglu" and N % 2:
+        N += 1
+    w, bias, a = rnd((N, K), torch.bfloat16, 70, 0.2), rnd((N,), torch.float32, 71), rnd((M, K), torch.bfloat16, 72, 2.0)
+    res = rnd((M, N), torch.float32, 73)
+    want = gemm_reference(a.cpu(), w, bias, {"residual": 2, "swiglu": 3}.get(epi, 1), res)
+    if epi == "residual":
+        got = res.clone()
+        ops.gemm_decode(w, ops.DEPI_RESIDUAL, M, a=a, bias=bias, residual=got, split_k=split_k)
+    elif epi == "swiglu":
+        got = torch.full((M, N // 2), float("nan"), dtype=torch.bfloat16, device=dev())
+        ops.gemm_decode_glu(w, a, bias, got, split_k, None)
+    else:
+        got = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=dev())
+        ops.gemm_decode_store(w, a, bias, got, (ops.ACT_SQUARED_RELU, 0.0, 0.0, 0.0) if epi == "relu" else None, split_k)
+        want = want.clamp(min=0.0) ** 2 if epi == "relu" else want
+    ops.check_async_errors(dev())
+    # float sums of exact products (2^-24 of the sum of magnitudes a product), a bf16 result (2^-9 of it); the gate multiplies both
+    size = a.abs().double().cpu() @ w.abs().double().cpu().t() + bias.abs().double().cpu() + 4.0
+    error = (K + 8) * 2.0 ** -24 * size
+    if epi == "relu":
+        error = 2 * error * (want.sqrt() + error)
+    if epi == "swiglu":
+        error = (error[:, 0::2] + error[:, 1::2]) * (size[:, 0::2] + size[:, 1::2]) * 1.2
+    bound = error + (0.0 if epi == "residual" else 2.0 ** -8 * want.abs() + 1e-6)
+    assert bool(((got.double().cpu() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M", [2, 17, 64])
+@pytest.mark.parametrize("split_k", [0, 3, 8])
+@pytest.mark.parametrize("hd,rd,inter,Hq,Hkv,K", [(64, 64, False, 14, 2, 896), (128, 128, False, 4, 1, 520), (32, 16, True, 6, 3, 136)])
+def test_gemm_decode_rope_clusters(ops, M, split_k, hd, rd, inter, Hq, Hkv, K):
+    """The rotary epilogue behind parts of K: the same as from one block alone, up to the order of the sums."""
+    N = (Hq + 2 * Hkv) * hd
+    w, bias, a = rnd((N, K), torch.bfloat16, 80, 0.1), rnd((N,), torch.float32, 81), rnd((M, K), torch.bfloat16, 82)
+    pos = torch.arange(M, dtype=torch.int32, device=dev()) * 37 + 5
+    inv = (10000.0 ** (-torch.arange(0, rd, 2, dtype=torch.float64) / rd)).float().to(dev())
+    slots = torch.randperm(200, generator=torch.Generator().manual_seed(83))[:M].to(torch.int32).to(dev())
+    table, outs = ops.rope_table(pos, inv), []
+    for split in (1, split_k):
+        kc, vc = (torch.full((200, Hkv, hd), 77.0, dtype=torch.bfloat16, device=dev()) for _ in range(2))
+        q = torch.full((M, Hq * hd), float("nan"), dtype=torch.bfloat16, device=dev())
+        ops.gemm_decode(w, ops.DEPI_ROPE_KV, M, a=a, bias=bias, slot_mapping=slots, split_k=split, rope_table=table, rotary_dim=rd,
+                        interleaved=inter, num_heads=Hq, num_kv_heads=Hkv, head_dim=hd, q_out=q, k_cache=kc, v_cache=vc)
+        outs.append((q, kc, vc))
+    ops.check_async_errors(dev())
+    for one, other in zip(*outs):          # two roundings to bf16 of sums that differ in their last bits
+        assert torch.allclose(one.float(), other.float(), rtol=2.0 ** -7, atol=2e-3)
+
+
 @pytest.mark.parametrize("M", [1, 8, 33])
 @pytest.mark.parametrize("hd,rd,inter,Hq,Hkv", [(64, 64, False, 14, 2), (128, 64, True, 3, 1), (32, 32, False, 6, 3),
                                                 (16, 16, False, 4, 2)])
