@@ -48,6 +48,7 @@ int llb_sample(const float* logits, int R, int V, long long stride, const float*
 int llb_paged_decode_mma_supports(int Hq, int Hkv, int hd);
 int llb_paged_decode_mma_cluster_splits();
 int llb_paged_decode_mma_resident(int hd);
+int llb_paged_decode_mma_fit(int hd, int nsplit, int pairs);
 int llb_attention_tcgen05_supports(int hd, int page_size);
 }
 
@@ -750,7 +751,8 @@ int main(int argc, char** argv) {
             int nsplit = std::max(1, std::min(std::max(1, ceil_div(2 * sms, (long long)nspans * cfg.kv_heads)), ceil_div(bound, 128)));
             if (bound <= CLUSTER_MERGE_MAX_KEYS) {
                 const int resident = blocks_per_sm * sms / (nspans * cfg.kv_heads);
-                nsplit = std::max(1, std::min(std::min(8, cluster_splits), std::min(resident, ceil_div(bound, 128))));
+                nsplit = llb_paged_decode_mma_fit(hd, std::max(1, std::min(std::min(8, cluster_splits), std::min(resident, ceil_div(bound, 128)))),
+                                                  nspans * cfg.kv_heads);
             }
             return nsplit;
         };
@@ -828,6 +830,7 @@ int main(int argc, char** argv) {
         step.error_flag = flags;
         step.stream = dev.stream;
         step.T = T;
+        step.fresh = 1;
         step.S = S;
         step.max_pages = P;
         step.page_size = PAGE;

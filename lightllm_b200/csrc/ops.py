@@ -1311,15 +1311,36 @@ def decode_mma_cluster_splits() -> int:
     return _cluster_splits
 
 
+_cluster_fit = {}
+
+
+def decode_mma_fit(head_dim: int, nsplit: int, pairs: int) -> int:
+    """The largest number of pieces up to ``nsplit`` whose clusters all find a place on the device at once for ``pairs``
+    (request, kv head) pairs."""
+    key = (head_dim, nsplit, pairs)
+    n = _cluster_fit.get(key)
+    if n is None:
+        if len(_cluster_fit) > 4096:
+            _cluster_fit.clear()
+        n = _cluster_fit[key] = int(lib().llb_paged_decode_mma_fit(head_dim, nsplit, pairs))
+    return n
+
+
+DECODE_EVEN_MAX = 64          # requests whose keys :func:`paged_decode_mma` cuts together
+
+
 def paged_decode_mma(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, out: torch.Tensor,
                      tile_span: torch.Tensor, tile_q0: torch.Tensor, num_tiles: int, span_row: torch.Tensor,
                      span_pos: torch.Tensor, block_table: torch.Tensor, max_pages: int, page_size: int,
                      num_heads: int, num_kv_heads: int, head_dim: int, window: int, scale: float,
                      nsplit: int = 1, scratch: Optional[torch.Tensor] = None,
                      sinks: Optional[torch.Tensor] = None, cross: int = 1, softcap: float = 0.0, keep: int = 0,
-                     slopes: Optional[torch.Tensor] = None) -> None:
+                     slopes: Optional[torch.Tensor] = None, fresh: int = 0) -> None:
     """Tensor-core decode attention: one query row per tile over its request's pages; bf16.  ``nsplit`` cuts
-    each request's keys; up to :func:`decode_mma_cluster_splits` the pieces are merged inside the kernel.
+    each request's keys; up to :func:`decode_mma_cluster_splits` the pieces are merged inside the kernel.  A negative one
+    cuts the keys of all requests together (at most :data:`DECODE_EVEN_MAX`) into ``-nsplit`` pieces of one length at most.
+    ``fresh`` > 0 says that all but a row's last ``fresh`` positions were in the cache before this step's first launch, so that
+    they may be read while the kernel before this one still runs.
     ``sinks``, ``v_cache is k_cache``, ``cross`` (crossed values), ``softcap``, ``keep``, ``slopes`` and a float32 ``out`` as
     :func:`paged_attention_tcgen05`."""
     _check_slopes(slopes, num_heads)
@@ -1330,8 +1351,9 @@ def paged_decode_mma(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
             raise KernelError("paged_decode_mma takes bfloat16 tensors")
     if out.dtype not in (torch.bfloat16, torch.float32) or out.numel() != q.shape[0] * num_heads * cross * head_dim:
         raise KernelError("decode attention: out is bfloat16 or float32 [T, heads, cross, head_dim]")
-    if nsplit > decode_mma_cluster_splits():
-        need = attention_scratch_floats(num_tiles, num_heads * cross, head_dim, 1, nsplit)
+    if nsplit < 0 or nsplit > decode_mma_cluster_splits():
+        need = -nsplit * num_heads * cross * (head_dim + 2) if nsplit < 0 else \
+            attention_scratch_floats(num_tiles, num_heads * cross, head_dim, 1, nsplit)
         if scratch is None or scratch.dtype != torch.float32 or scratch.numel() < need:
             raise KernelError(f"decode attention: nsplit={nsplit} needs {need} floats of scratch")
     _check(lib().llb_paged_decode_mma_biased(
@@ -1339,7 +1361,7 @@ def paged_decode_mma(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
         num_tiles, _i32(span_row, "span_row"), _i32(span_pos, "span_pos"), _i32(block_table, "block_table"),
         max_pages, page_size, num_heads, num_kv_heads, head_dim, window, ctypes.c_float(scale),
         ctypes.c_float(softcap or 0.0), nsplit,
-        _ptr(scratch), _ptr(sinks), cross, 1 if out.dtype == torch.float32 else 0, keep, _ptr(slopes), _stream()))
+        _ptr(scratch), _ptr(sinks), cross, 1 if out.dtype == torch.float32 else 0, keep, _ptr(slopes), fresh, _stream()))
 
 
 # Where the blocks that share a long row of logits meet (a 64-bit slot and a counter per row), per device.

@@ -14,7 +14,7 @@ int llb_paged_decode_mma_cluster_splits();
 int llb_paged_decode_mma(const void* q, const void* k_cache, const void* v_cache, void* out, const int* tile_span,
                          const int* tile_q0, int num_tiles, const int* span_row, const int* span_pos,
                          const int* block_table, int max_pages, int page_size, int Hq, int Hkv, int hd, int window,
-                         float scale, int nsplit, float* scratch, cudaStream_t stream);
+                         float scale, int nsplit, float* scratch, int fresh, cudaStream_t stream);
 int llb_paged_decode_mma_supports(int Hq, int Hkv, int hd);
 long long llb_attention_scratch_floats(int num_tiles, int Hq, int hd, int BQ, int nsplit);
 int llb_paged_attention(const void* q, const void* k_cache, const void* v_cache, void* out, int dtype, const int* tile_span,
@@ -208,12 +208,14 @@ struct Exec {
     }
     int decode_mma(const LlbAttentionDesc& a, const void* q, void* out, const LlbTileList& t, bool may_scratch) {
         float* scratch = nullptr;
-        if (may_scratch && t.nsplit > llb_paged_decode_mma_cluster_splits())
+        if (t.nsplit < 0)
+            scratch = (float*)take(-(long long)t.nsplit * a.num_heads * (a.head_dim + 2) * 4);
+        else if (may_scratch && t.nsplit > llb_paged_decode_mma_cluster_splits())
             scratch = (float*)take(llb_attention_scratch_floats(t.count, a.num_heads, a.head_dim, 1, t.nsplit) * 4);
         if (dry) return 0;
         return llb_paged_decode_mma(q, a.k_cache, a.v_cache, out, t.span, t.q0, t.count, s.span_row, s.span_pos,
                                     s.block_tables[a.group], s.max_pages, s.page_size, a.num_heads, a.num_kv_heads, a.head_dim,
-                                    a.window, a.scale, t.nsplit, scratch, s.stream);
+                                    a.window, a.scale, t.nsplit, scratch, s.fresh, s.stream);
     }
     int attend(const LlbAttentionDesc& a, const void* q, void* out) {
         const LlbAttentionPlan& p = s.plans[a.plan];

@@ -111,6 +111,7 @@ typedef struct {
     int max_pages, page_size;
     int num_plans;
     int first_layer, last_layer;   // run entries [first, last)
+    int fresh;                     // a row's last positions that this step may write (see llb_paged_decode_mma_biased)
 } LlbStepArgs;
 
 // Runs the run entries [first_layer, last_layer) over the step.  0, or a negative code with llb_last_error().

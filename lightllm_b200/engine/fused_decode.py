@@ -1,7 +1,7 @@
 """Decode steps through the persistent layer kernel (csrc/decode_layers.cu).
 
 A step in which every request brings one token (at most 64 of them) spends its time in the chain of dependent
-launches of a layer, not in the bytes it reads.  Where consecutive entries of the run list are the common block
+launches of a layer, not in the bytes it reads, where the layers are small.  Where consecutive entries of the run list are the common block
 
     h += attention(rmsnorm(h));  h += gated_mlp(rmsnorm(h))          (src/engine/engine_server.cpp:1530-1880)
 
@@ -23,16 +23,14 @@ from ..parts.norm import RMSNorm
 from ..parts.rotary import NoPositionEncoding, RotaryEmbedding
 
 MAX_ROWS = 64          # what the kernel takes
-# Up to this many rows the persistent kernel is faster than the layers launched kernel by kernel (measured on B200 at
-# the 0.5B sizes: 0.72 / 0.77 / 0.88 / 1.12 ms a step at 1 / 8 / 16 / 32 rows against 0.80 / 0.90 / 1.00 / 1.17; at 64 rows
-# 1.66 against 1.54, where the attention's keys and the operands of 64 rows outweigh the saved launches).
+# Where the persistent kernel is faster than the layers launched kernel by kernel (each kernel set up while the one before it runs):
+# layers of a few megabytes of weights, of which nothing but the chain of stages is left, under two rows and more.  Measured on
+# B200, ms a step of 24 layers, persistent / kernel by kernel: width 256 (2 MB a layer) 0.56 / 0.50 at one row, 0.55 / 0.61 at four,
+# 0.69 / 0.81 at 32; width 512 (6 MB) 0.61 / 0.55, 0.58 / 0.58, 0.72 / 0.74; width 768 (15 MB) 0.64 / 0.59, 0.62 / 0.67, 0.88 / 0.85, eight
+# rows 0.71 / 0.68; the 0.5B sizes (30 MB) 0.73 / 0.67, 0.73 / 0.72, 0.97 / 0.95; the 1.5B sizes (93 MB, 28 layers) 1.36 / 1.20, 1.38 / 1.23, 2.10 / 1.56.
 DEFAULT_ROWS = 32
-# The kernel pays where a layer is paced by its chain of stages, not by its bytes: up to this many bytes of weights a
-# layer.  Measured: 30 MB a layer (0.5B sizes) 0.72 ms a step at one row against 0.80 launched kernel by kernel; 93 MB
-# (1.5B) 1.36 against 1.33 at one row and 1.57 against 1.81 at eight; 404 MB (7B) 4.5 against 3.1: there the separate
-# kernels stream their weights at 0.7 of the memory's bandwidth, which one block per multiprocessor walking through
-# build, multiply and drain does not reach.
-MAX_LAYER_BYTES = 128 << 20
+MIN_ROWS = 2
+MAX_LAYER_BYTES = 8 << 20
 
 
 def _layer_facts(block, view):
@@ -127,7 +125,7 @@ class FusedDecode:
     def takes(self, ctx) -> bool:
         # (one row a request: the kernel's attention stage makes a row's new key and value itself, beside the rows that
         # read the cache, so the rows of a step described row by row, which share requests, go kernel by kernel)
-        return (self.enabled and ctx.decode_only and not ctx.rowwise and ctx.T <= self.max_rows
+        return (self.enabled and ctx.decode_only and not ctx.rowwise and MIN_ROWS <= ctx.T <= self.max_rows
                 and len(ctx.block_tables) <= ops.MAX_FUSED_GROUPS)
 
     def segment_at(self, run_index: int) -> Optional[Segment]:

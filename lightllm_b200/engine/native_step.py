@@ -67,7 +67,7 @@ class StepArgs(ctypes.Structure):
                 ("block_tables", _P * MAX_GROUPS), ("slot_mapping", _P * MAX_GROUPS), ("residual", _P), ("workspace", _P),
                 ("workspace_bytes", _LL), ("plans", _P), ("meet_counters", _P),
                 ("error_flag", _P), ("stream", _P), ("meet_counters_n", _I), ("T", _I), ("S", _I), ("max_pages", _I), ("page_size", _I), ("num_plans", _I),
-                ("first_layer", _I), ("last_layer", _I)]
+                ("first_layer", _I), ("last_layer", _I), ("fresh", _I)]
 
 
 _STRUCTS = (NormDesc, AttentionDesc, MlpDesc, LayerDesc, ModelDesc, TileList, AttentionPlan, StepArgs)
@@ -232,7 +232,7 @@ class NativeLayers:
         s.error_flag = ops.async_error_flag(self.device).data_ptr()
         s.stream = ops.current_stream()
         s.T, s.S, s.max_pages, s.page_size = ctx.T, ctx.num_spans, ctx.max_pages, ctx.page_size
-        s.first_layer, s.last_layer = first, last
+        s.first_layer, s.last_layer, s.fresh = first, last, ctx.fresh_positions
         s.workspace, s.workspace_bytes = None, 0
         need = lib.llb_step_workspace_need(ctypes.addressof(self._model), ctypes.addressof(s))
         if need < 0:

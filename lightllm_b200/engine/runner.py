@@ -268,6 +268,9 @@ class ModelRunner:
         ctx.max_pages, ctx.page_size = P, ps
         ctx.decode_only = all(s.length == 1 for s in spans)
         ctx.rowwise = rowwise
+        # the last positions of a row that attends alone which this step itself may write: its own, or in a step described row by
+        # row those of its whole portion
+        ctx.fresh_positions = self.ROWWISE_MAX_ROWS if rowwise else 1
         ctx.max_context = max_context
         ctx.dtype, ctx.device = self.model.dtype, self.device
         ctx.cache, ctx.err = cache, self.err

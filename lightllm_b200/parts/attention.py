@@ -4,6 +4,7 @@ from __future__ import annotations
 import math
 from typing import Dict, List, Optional
 
+import numpy as np
 import torch
 
 from ..cache import CacheSpec, KVSpec
@@ -23,6 +24,8 @@ TENSOR_CORE_MIN_ROWS = 2
 # MANY_KEYS keys or more is walked row by row with each row's keys in pieces, not by one block per tile of rows.
 FEW_ROWS = 32
 MANY_KEYS = 512
+# Requests of different lengths: how many keys longer than an even piece the longest one's piece may be (the merge's 2.2 to 2.8 us).
+EVEN_GAIN_KEYS = {64: 160, 128: 112}
 # Up to this many keys per request the decode attention's pieces are merged inside the kernel.
 CLUSTER_MERGE_MAX_KEYS = 8192
 # From this many rows on, heads of 64 or 128 get their rotation and cache write in the projection's tensor-core epilogue.
@@ -259,11 +262,36 @@ class AttentionMixer(Mixer):
                 resident = (ops.decode_mma_resident(self.head_dim) * L.num_sms(ctx.device)
                             // (S * self.num_kv_heads * cross))
                 nsplit = max(1, min(8, ops.decode_mma_cluster_splits(), resident, -(-span // 128)))
+                nsplit = ops.decode_mma_fit(self.head_dim, nsplit, S * self.num_kv_heads * cross)
+            if mma:
+                nsplit = self._even_pieces(ctx, range(S), nsplit)
             plan = ("decode_mma" if mma else "decode_simt", ctx.tiles(1), nsplit)
         else:
             plan = self._plan_mixed(ctx, bf16, window)
         ctx.memo[key] = plan
         return plan
+
+    def _even_pieces(self, ctx, which, nsplit: int) -> int:
+        """``nsplit`` pieces a request, or minus the number of pieces of one length over all requests: a block takes 20 to 27 ns a key,
+        so where the longest request's piece is longer than an even one by EVEN_GAIN_KEYS, the merge of the even ones, a launch
+        of its own, is paid for."""
+        n = len(which)
+        if n < 2 or n > ops.DECODE_EVEN_MAX:
+            return nsplit
+        window = self.kernel_window()
+        starts = np.fromiter((ctx.spans[i].start for i in which), dtype=np.int64, count=n)
+        keys = starts + 1
+        if window > 0:
+            keys = np.minimum(keys, window + self.keep_first)
+        elif window < 0:
+            keys = np.minimum(keys, starts % -window + 1 + self.keep_first)
+        resident = ops.decode_mma_resident(self.head_dim) * L.num_sms(ctx.device) // (self.num_kv_heads * self.value_cross)
+        pieces = max(n, min(resident, n + 128))
+        even = max(64, -(-int(keys.sum()) // pieces))
+        if -(-int(keys.max()) // nsplit) < even + EVEN_GAIN_KEYS[self.head_dim]:
+            return nsplit
+        ctx.shape_key.append(("even", pieces))
+        return -pieces
 
     def _plan_mixed(self, ctx, bf16: bool, window: int):
         """A step with portions of prompts, maybe beside decoded tokens.  Each span goes where its shape is served best:
@@ -299,7 +327,8 @@ class AttentionMixer(Mixer):
             resident = (ops.decode_mma_resident(self.head_dim) * L.num_sms(ctx.device)
                         // (len(single) * self.num_kv_heads * self.value_cross))
             nsplit = max(1, min(8, ops.decode_mma_cluster_splits(), resident, -(-span // 128)))
-            decode = (ctx.tiles(1, select=tuple(single)), nsplit)
+            nsplit = ops.decode_mma_fit(self.head_dim, nsplit, len(single) * self.num_kv_heads * self.value_cross)
+            decode = (ctx.tiles(1, select=tuple(single)), self._even_pieces(ctx, single, nsplit))
         simt = []
         if rows:         # few rows over many keys: row by row, each row's keys in pieces
             simt.append((ctx.tiles(1, select=tuple(rows)), 1, max(2, min(16, -(-rows_keys // 256)))))
@@ -338,7 +367,10 @@ class AttentionMixer(Mixer):
         if plan[0] == "decode_mma":
             (tile_span, tile_q0, ntiles), nsplit = plan[1], plan[2]
             scratch = None
-            if nsplit > ops.decode_mma_cluster_splits():
+            if nsplit < 0:
+                scratch = torch.empty(-nsplit * self.num_heads * self.value_cross * (self.head_dim + 2), dtype=torch.float32,
+                                      device=q.device)
+            elif nsplit > ops.decode_mma_cluster_splits():
                 scratch = torch.empty(ops.attention_scratch_floats(ntiles, self.num_heads * self.value_cross,
                                                                    self.head_dim, 1, nsplit),
                                       dtype=torch.float32, device=q.device)
@@ -346,7 +378,7 @@ class AttentionMixer(Mixer):
                                  ctx.block_tables[g], ctx.max_pages, ctx.page_size, self.num_heads,
                                  self.num_kv_heads, self.head_dim, window, self.scale, nsplit, scratch, sinks=self.sinks,
                                  cross=self.value_cross, softcap=self.softcap or 0.0, keep=self.keep_first,
-                                 slopes=self.slopes)
+                                 slopes=self.slopes, fresh=ctx.fresh_positions)
         elif plan[0] == "decode_simt":
             self._simt(q, cache, out, plan[1], common, 1, plan[2])
         else:
@@ -358,11 +390,13 @@ class AttentionMixer(Mixer):
                                  slopes=self.slopes)
             if decode is not None:
                 (tile_span, tile_q0, ntiles), nsplit = decode
+                scratch = None if nsplit > 0 else torch.empty(-nsplit * self.num_heads * self.value_cross * (self.head_dim + 2),
+                                                              dtype=torch.float32, device=q.device)
                 ops.paged_decode_mma(q, cache.k, v_plane, out, tile_span, tile_q0, ntiles, ctx.span_row, ctx.span_pos,
                                      ctx.block_tables[g], ctx.max_pages, ctx.page_size, self.num_heads,
-                                     self.num_kv_heads, self.head_dim, window, self.scale, nsplit, None, sinks=self.sinks,
+                                     self.num_kv_heads, self.head_dim, window, self.scale, nsplit, scratch, sinks=self.sinks,
                                      cross=self.value_cross, softcap=self.softcap or 0.0, keep=self.keep_first,
-                                     slopes=self.slopes)
+                                     slopes=self.slopes, fresh=ctx.fresh_positions)
             for tiles, bq, nsplit in simt:
                 self._simt(q, cache, out, tiles, common, bq, nsplit)
 

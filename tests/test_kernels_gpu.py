@@ -623,6 +623,29 @@ def test_paged_decode_mma(ops, case, nsplit, spike):
     assert torch.allclose(got, ref, atol=2e-2, rtol=2e-2), f"max diff {float((got - ref).abs().max())}"
 
 
+# one request, as many as are cut together, lengths that fill pieces exactly, pieces more and fewer than the keys allow
+@pytest.mark.parametrize("case", [MMA_DECODE_CASES[0], MMA_DECODE_CASES[1], MMA_DECODE_CASES[2], MMA_DECODE_CASES[4],
+                                  (14, 2, 64, 16, [127, 128, 255, 256, 511, 0], None), (12, 2, 128, 16, [63, 64, 4000, 65, 1, 900], None),
+                                  (4, 2, 64, 16, [(37 * i * i) % 1500 for i in range(64)], None), (28, 4, 128, 16, [2000, 3, 700], 300)])
+@pytest.mark.parametrize("more", [0, 1, 17, 140])
+def test_paged_decode_mma_pieces_of_one_length(ops, case, more):
+    Hq, Hkv, hd, page, starts, window = case
+    lens, pieces = [1] * len(starts), len(starts) + more
+    s = paged_setup(torch.bfloat16, lens, starts, Hq, Hkv, hd, page, seed=26, spike=True)
+    ts, tq, nt = tiles_for(lens, 1)
+    out = torch.full((s["rows"], Hq * hd), float("nan"), dtype=torch.bfloat16, device=dev())
+    scratch = torch.full((pieces * Hq * (hd + 2),), float("nan"), device=dev())
+    ops.paged_decode_mma(s["q"], s["kc"], s["vc"], out, ts, tq, nt, s["span_row"], s["span_pos"], s["bt"],
+                         s["max_pages"], page, Hq, Hkv, hd, window or 0, 1.0 / math.sqrt(hd), -pieces, scratch)
+    ref = attention_reference(s["full"], lens, starts, hd, window).reshape(s["rows"], Hq * hd)
+    got = out.float().cpu()
+    assert not torch.isnan(got).any()
+    assert torch.allclose(got, ref, atol=2e-2, rtol=2e-2), f"max diff {float((got - ref).abs().max())}"
+    with pytest.raises(ops.KernelError):          # fewer pieces than requests
+        ops.paged_decode_mma(s["q"], s["kc"], s["vc"], out, ts, tq, nt, s["span_row"], s["span_pos"], s["bt"],
+                             s["max_pages"], page, Hq, Hkv, hd, window or 0, 1.0 / math.sqrt(hd), 1 - nt if nt > 1 else 0, scratch)
+
+
 @pytest.mark.parametrize("V", [151937, 16384, 1003])      # long rows are shared among blocks, short ones are not
 def test_argmax_lowest_index_on_ties(ops, V):
     x = rnd((9, V), torch.float32, 30)
