@@ -58,6 +58,7 @@ struct GemmParams {
     int num_kb;             // K blocks in all
     int kb_per_split;       // K blocks per grid.z slice (per split of the persistent kernel)
     int splits;             // persistent kernel: work items per tile along K
+    int width;              // features of a pair's tile (a multiple of 32, at most 256)
     int direct;             // residual epilogue with splits: every piece adds its part to the residual itself (TMA
                             // reduce-add), nothing meets in `partials`
     float* partials;        // [items, tile width, 128] float: the splits' accumulators meet here
@@ -400,50 +401,47 @@ __device__ __forceinline__ void staged_chunk(const GemmParams& p, const CUtensor
     }
 }
 
-// Rotary epilogue of one warp: token rows row0 .. row0+31 (one per lane) and the 64 output features nb .. nb+63 of q,
-// k or v (src/ops/rope.cu:54-59 on every pair; cache rows as src/kv_cache/paged_attention.cu:1150-1163).  With heads
-// of 64 these are one whole head and both members of every pair (j, j + 32) are here; with heads of 128 they are half
-// of a head, the pairs are (j, j + 64), and the other members come in `p0`, `p1` (the same columns of the head's other
-// half).  The (cos, sin) table is laid out [pair][token], so the lanes of a warp read neighbouring entries.  q leaves
-// through the warp's staging tile and one TMA store (64 bf16 are one 128-byte row of it) when `staged`; k and v go
+// Rotary epilogue of one warp: token rows row0 .. row0+31 (one per lane) and 32 pairs of output features, nb + j and nb + HD/2 + j, of
+// q, k or v (src/ops/rope.cu:54-59 on every pair; cache rows as src/kv_cache/paged_attention.cu:1150-1163).  With heads
+// of 64 these are one whole head, with heads of 128 half of one: both members of a pair are here, so every accumulator and every
+// (cos, sin) is read once.  (Heads of 128 by 64 neighbouring features, with the partners read beside them, took twice the reads
+// of both: 2,030 rows x 1,536 with 12 / 2 heads 27.9 us, 23.8 so and 17.8 on pair tiles.)  The (cos, sin) table is laid out [pair][token], so the lanes of a warp read neighbouring entries.  q
+// leaves through the warp's staging tile and TMA stores when `staged` (64 bf16 are one 128-byte row of it, or two of 64 bytes); k and v go
 // straight to their cache rows, which lie wherever the pages are.
 template <int HD>
 __device__ __forceinline__ void epilogue_rope_warp(const GemmParams& p, const CUtensorMap* map_q, uint8_t* stage,
                                                    bool staged, int lane, int row0, int nb, const uint32_t (&r0)[32],
-                                                   const uint32_t (&r1)[32], const uint32_t (&p0)[32],
-                                                   const uint32_t (&p1)[32]) {
+                                                   const uint32_t (&r1)[32]) {
     if (nb >= p.N) return;                       // uniform over the warp
+    constexpr int GAP = HD / 2;
     const int m = row0 + lane;
     const bool in_m = m < p.M;
     const int q_end = p.Hq * HD, k_end = q_end + p.Hkv * HD;
-    const bool second_half = HD == 128 && (nb & 64) != 0;      // these columns are the pairs' second members
     float a[32], b[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
         a[j] = __uint_as_float(r0[j]);
         b[j] = __uint_as_float(r1[j]);
-        if (p.bias) { a[j] += p.bias[nb + j]; b[j] += p.bias[nb + 32 + j]; }
+    }
+    if (p.bias && ((uintptr_t)p.bias & 15) == 0) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+            const float4 u = __ldg(reinterpret_cast<const float4*>(p.bias + nb + j)), v = __ldg(reinterpret_cast<const float4*>(p.bias + nb + GAP + j));
+            a[j] += u.x; a[j + 1] += u.y; a[j + 2] += u.z; a[j + 3] += u.w;
+            b[j] += v.x; b[j + 1] += v.y; b[j + 2] += v.z; b[j + 3] += v.w;
+        }
+    } else if (p.bias) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) { a[j] += p.bias[nb + j]; b[j] += p.bias[nb + GAP + j]; }
     }
     if (nb < k_end && in_m) {
-        const float2* cs = p.rope_table + m;
-        if (HD == 64) {
+        const float2* cs = p.rope_table + (size_t)(nb % GAP) * p.M + m;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const float2 t = cs[(size_t)j * p.M];
-                const float x = a[j], y = b[j];
-                a[j] = x * t.x - y * t.y;
-                b[j] = y * t.x + x * t.y;
-            }
-        } else {
-            const int nbp = second_half ? nb - 64 : nb + 64;      // where the partners' bias lies
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                float pa = __uint_as_float(p0[j]), pb = __uint_as_float(p1[j]);
-                if (p.bias) { pa += p.bias[nbp + j]; pb += p.bias[nbp + 32 + j]; }
-                const float2 ta = cs[(size_t)j * p.M], tb = cs[(size_t)(32 + j) * p.M];
-                a[j] = second_half ? a[j] * ta.x + pa * ta.y : a[j] * ta.x - pa * ta.y;
-                b[j] = second_half ? b[j] * tb.x + pb * tb.y : b[j] * tb.x - pb * tb.y;
-            }
+        for (int j = 0; j < 32; ++j) {
+            const float2 t = cs[(size_t)j * p.M];
+            const float x = a[j], y = b[j];
+            a[j] = x * t.x - y * t.y;
+            b[j] = y * t.x + x * t.y;
         }
     }
     uint32_t wa[16], wb[16];
@@ -457,16 +455,20 @@ __device__ __forceinline__ void epilogue_rope_warp(const GemmParams& p, const CU
     if (nb < q_end && staged) {
         if (lane == 0) tma_store_wait_read();
         __syncwarp();
-        uint8_t* row = stage + lane * 128;
+        // heads of 64: rows of 128 bytes, the 128-byte swizzle; of 128: two tiles of 64-byte rows, the 64-byte swizzle
+        uint8_t* row = stage + lane * (HD == 64 ? 128 : 64);
+        const int turn = HD == 64 ? lane & 7 : (lane >> 1) & 3;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            *reinterpret_cast<uint4*>(row + ((c ^ (lane & 7)) * 16)) = make_uint4(wa[4 * c], wa[4 * c + 1], wa[4 * c + 2], wa[4 * c + 3]);
-            *reinterpret_cast<uint4*>(row + (((4 + c) ^ (lane & 7)) * 16)) = make_uint4(wb[4 * c], wb[4 * c + 1], wb[4 * c + 2], wb[4 * c + 3]);
+            *reinterpret_cast<uint4*>(row + ((c ^ turn) * 16)) = make_uint4(wa[4 * c], wa[4 * c + 1], wa[4 * c + 2], wa[4 * c + 3]);
+            *reinterpret_cast<uint4*>(row + (HD == 64 ? ((4 + c) ^ turn) * 16 : 2048 + (c ^ turn) * 16)) =
+                make_uint4(wb[4 * c], wb[4 * c + 1], wb[4 * c + 2], wb[4 * c + 3]);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0 && row0 < p.M) {
             tma_store_2d(map_q, smem_u32(stage), nb, row0);
+            if (HD == 128) tma_store_2d(map_q, smem_u32(stage) + 2048, nb + GAP, row0);
             tma_store_commit();
         }
         return;
@@ -484,7 +486,7 @@ __device__ __forceinline__ void epilogue_rope_warp(const GemmParams& p, const CU
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         *reinterpret_cast<uint4*>(dst + 8 * c) = make_uint4(wa[4 * c], wa[4 * c + 1], wa[4 * c + 2], wa[4 * c + 3]);
-        *reinterpret_cast<uint4*>(dst + 32 + 8 * c) = make_uint4(wb[4 * c], wb[4 * c + 1], wb[4 * c + 2], wb[4 * c + 3]);
+        *reinterpret_cast<uint4*>(dst + GAP + 8 * c) = make_uint4(wb[4 * c], wb[4 * c + 1], wb[4 * c + 2], wb[4 * c + 3]);
     }
 }
 
@@ -525,7 +527,8 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const 
     const int first_item = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
     const int item_stride = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
     const int m_tiles = (p.M + ROWS_PER_TILE - 1) / ROWS_PER_TILE;
-    const int n_tiles = (p.N + P_BN - 1) / P_BN;
+    const int width = PAIR ? p.width : P_BN;                        // features of a tile
+    const int n_tiles = (p.N + width - 1) / width;
     const int num_tiles = m_tiles * n_tiles;
     const int nkb = p.num_kb;
     const int splits = p.splits;
@@ -566,7 +569,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const 
             for (int w = first_item; w < num_items; w += item_stride) {
                 const int t = w / splits, ks = w - t * splits;
                 const int a_row0 = (t % m_tiles) * ROWS_PER_TILE + (int)rank * TILE_M;
-                int b_row0 = (t / m_tiles) * P_BN + (PAIR ? (int)rank * (P_BN / 2) : 0);
+                int b_row0 = (t / m_tiles) * width + (PAIR ? (int)rank * (width / 2) : 0);
                 if (!PAIR && p.tile_group) b_row0 += p.tile_group[t % m_tiles] * p.N;
                 const int kb0 = ks * p.kb_per_split, kb1 = min(nkb, kb0 + p.kb_per_split);
                 bool ok = true;
@@ -576,7 +579,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const 
                     if (!ok) break;
                     if (PAIR) {
                         const int nk = min(KPS, kb1 - kb);
-                        if (rank == 0) mbar_expect_tx(&full_bar[s], nk * 2 * (A_BYTES + B_BYTES));
+                        if (rank == 0) mbar_expect_tx(&full_bar[s], nk * (2 * A_BYTES + (uint32_t)width * TILE_K * 2));
                         for (int j = 0; j < nk; ++j) {
                             tma_load_2d_pair(a_tiles + (s * KPS + j) * A_BYTES, &map_a, (kb + j) * TILE_K, a_row0, full_of_first + s * 8);
                             tma_load_2d_pair(b_tiles + (s * KPS + j) * B_BYTES, &map_b, (kb + j) * TILE_K, b_row0, full_of_first + s * 8);
@@ -597,7 +600,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const 
             // the loop carries what it needs in registers: the stage's two operand descriptors (advanced by
             // constants; the address field of a descriptor is the shared-memory address / 16), the addresses of its
             // barriers, its phase bit.
-            constexpr uint32_t idesc = idesc_bf16(ROWS_PER_TILE, P_BN);
+            const uint32_t idesc = idesc_bf16(ROWS_PER_TILE, width);
             constexpr uint64_t A_STEP = A_BYTES >> 4, B_STEP = B_BYTES >> 4, K_STEP = (UMMA_K * 2) >> 4;
             const uint64_t da0 = desc_kmajor(smem_u32(a_tiles)), db0 = desc_kmajor(smem_u32(b_tiles));
             const uint32_t full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]);
@@ -663,7 +666,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const 
         for (int w = first_item; w < num_items; w += item_stride, ++local) {
             const int t = w / splits;
             const int buf = local & 1;
-            const int a_row0 = (t % m_tiles) * ROWS_PER_TILE + (int)rank * TILE_M, b_row0 = (t / m_tiles) * P_BN;
+            const int a_row0 = (t % m_tiles) * ROWS_PER_TILE + (int)rank * TILE_M, b_row0 = (t / m_tiles) * width;
             if (!mbar_wait(&acc_full[buf], (local >> 1) & 1, abort_flag)) break;      // uniform over the warp
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const bool direct = EPI == LLB_EPI_RESIDUAL && p.direct != 0;      // uniform over the grid
@@ -778,36 +781,30 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const 
                 continue;
             }
             if (epi_is_rope(EPI)) {
-                // 64 columns at a time: a head of 64 with both members of every rotary pair, or half of a head of 128
+                // 32 pairs at a time: heads of 64 are shared out between the halves, heads of 128 are halved
+                constexpr bool WIDE = EPI == EPI_ROPE128;
 #pragma unroll 1
-                for (int c0 = half * (P_BN / 2); c0 < (half + 1) * (P_BN / 2); c0 += 64) {
+                for (int c = 0; c < P_BN / 2; c += 64) {
+                    const int c0 = WIDE ? c * 2 + half * 32 : half * (P_BN / 2) + c;
                     uint32_t r0[32], r1[32];
                     const uint32_t ta = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P_BN + c0);
                     tmem_ld32_nowait(ta, r0);
-                    tmem_ld32_nowait(ta + 32, r1);
-                    if (EPI == EPI_ROPE128) {      // the pairs' other members: the same columns of the head's other half (the tile is one head)
-                        uint32_t p0[32], p1[32];
-                        const uint32_t tp = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P_BN + (c0 ^ 64));
-                        tmem_ld32_nowait(tp, p0);
-                        tmem_ld32_nowait(tp + 32, p1);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        epilogue_rope_warp<128>(p, &map_out, my_stage, p.tma_out != 0, lane, a_row0 + quarter * 32, b_row0 + c0,
-                                                r0, r1, p0, p1);
-                    } else {
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        epilogue_rope_warp<64>(p, &map_out, my_stage, p.tma_out != 0, lane, a_row0 + quarter * 32, b_row0 + c0,
-                                               r0, r1, r0, r1);
-                    }
+                    tmem_ld32_nowait(ta + (WIDE ? 64 : 32), r1);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    epilogue_rope_warp<(WIDE ? 128 : 64)>(p, &map_out, my_stage, p.tma_out != 0, lane, a_row0 + quarter * 32, b_row0 + c0, r0, r1);
                 }
             } else {
+                // (a narrower tile's halves are whole staged rows too: of 32 columns, see pair_width)
+                const int middle = PAIR ? (width / 2 + 31) / 32 * 32 : P_BN / 2;
+                const int begin = half * middle, end = half ? width : middle;
 #pragma unroll 1
-                for (int c0 = half * (P_BN / 2); c0 < (half + 1) * (P_BN / 2); c0 += 32) {
+                for (int c0 = begin; c0 < end; c0 += 32) {
                     uint32_t r[32];
                     tmem_ld32_nowait(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P_BN + c0), r);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (staged)
                         staged_chunk<SEPI>(p, &map_out, my_stage, lane, a_row0 + quarter * 32, b_row0 + c0,
-                                           ((c0 - half * (P_BN / 2)) >> 5) % StagedOut<SEPI>::PIECES, r);
+                                           ((c0 - begin) >> 5) % StagedOut<SEPI>::PIECES, r);
                     else
                         epilogue_row<SEPI, 32>(p, a_row0 + row, b_row0 + c0, r);
                 }
@@ -914,7 +911,7 @@ int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mb, const CUtens
         cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
         configured = true;
     }
-    const int tiles = llb_ceil_div(p.M, PAIR ? 2 * TILE_M : TILE_M) * llb_ceil_div(p.N, P_BN) * p.splits;
+    const int tiles = llb_ceil_div(p.M, PAIR ? 2 * TILE_M : TILE_M) * llb_ceil_div(p.N, PAIR ? p.width : P_BN) * p.splits;
     const int units = PAIR ? num_sms / 2 : num_sms;              // blocks, or pairs of blocks
     const int grid = (tiles < units ? tiles : units) * (PAIR ? 2 : 1);
     cudaLaunchConfig_t cfg = {};
@@ -957,6 +954,27 @@ int pair_min_features() {
         if (n < 256) n = 256;
     }
     return n;
+}
+
+// The width of a pair's tiles.  The pairs take the tiles in rounds, and 256 features a tile may leave the last round nearly empty (2,048 x
+// 9,728: 304 tiles for 74 pairs) or pairs without any (2,048 x 1,536: 48): the width with the least rounds x (width + 48), a tile's
+// time beside the widest's being what its columns and a fixed part say.  Narrower ones only under the epilogues whose staged rows are 32
+// columns: the gated activation's are 128, and with the rest of a tile of 224 in direct stores 2,048 x 9,728 x 896 took 54.0 us
+// instead of 44.6.  Measured (256 -> chosen, us): 2,030 x 1,536 x 8,960 52.7 -> 49.7 at 192 (a narrower tile is bound by what a
+// multiprocessor gets from L2), 2,030 x 1,536 x 1,536 15.4 -> 14.2, 600 x 1,536 x 1,536 14.7 -> 12.5, 2,100 x 3,584 x 18,944 222 -> 218 at 224.
+int pair_width(int epi, int M, int N, int num_sms) {
+    const int m_tiles = llb_ceil_div(M, 2 * TILE_M), units = num_sms / 2;
+    int best = 256;
+    long long least = -1;
+    for (int w = 256; w >= 128; w -= 32) {
+        if (w != 256 && epi != LLB_EPI_RESIDUAL && epi != LLB_EPI_STORE_F32) break;
+        const long long cost = (long long)llb_ceil_div(m_tiles * llb_ceil_div(N, w), units) * (w + 48);
+        if (least < 0 || cost < least) {
+            least = cost;
+            best = w;
+        }
+    }
+    return best;
 }
 
 template <int P_BN, bool PAIR = false>
@@ -1070,7 +1088,11 @@ LLB_EXPORT int llb_gemm_tcgen05_glu(const void* A, const void* W, const float* b
     // Many rows and many features: pairs of CTAs on tiles of 256 x 256, each CTA loading its own rows and half of
     // the weights' tile.
     if (split_k == 1 && N >= pair_min_features() && M >= 512 && pair_tiles_enabled()) {
-        if ((rc = make_map(W, N, K, 128, &mb))) return rc;
+        int dev = 0, num_sms = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+        p.width = pair_width(epilogue, M, N, num_sms);
+        if ((rc = make_map(W, N, K, p.width / 2, &mb))) return rc;
         return dispatch_persistent<256, true>(epilogue, ma, mb, p, stream);
     }
     // The wide tile wins wherever its padding of N costs little, and always when K is split (few tiles are what
@@ -1162,25 +1184,26 @@ LLB_EXPORT int llb_gemm_tcgen05_rope(const void* A, const void* W, const float* 
     int rc;
     if ((rc = make_map(A, M, K, TILE_M, &ma))) return rc;
     if ((rc = make_map(W, N, K, 128, &mb))) return rc;
-    // q leaves through TMA stores of 64 bf16 x 32 rows (its row pitch, Hq * hd * 2 bytes, always allows it)
+    // q leaves through TMA stores of 64 (heads of 128: 32) bf16 x 32 rows (its row pitch, Hq * hd * 2 bytes, always allows it)
     CUtensorMap mq = ma;
     {
         t5::EncodeTiledFn fn = t5::encode_tiled_fn();
         if (!fn) return llb_fail("gemm_tcgen05_rope: cuTensorMapEncodeTiled is not available from the driver");
         cuuint64_t dims[2] = {(cuuint64_t)Hq * hd, (cuuint64_t)M};
         cuuint64_t strides[1] = {(cuuint64_t)Hq * hd * 2};
-        cuuint32_t box[2] = {64u, 32u};
+        cuuint32_t box[2] = {hd == 64 ? 64u : 32u, 32u};
         cuuint32_t estr[2] = {1, 1};
         CUresult r = fn(&mq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, q_out, dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, hd == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return llb_fail("gemm_tcgen05_rope: cuTensorMapEncodeTiled (q) failed with code %d", (int)r);
         p.tma_out = 1;
     }
     // Many rows and features: pair tiles, as the plain contraction takes them (each CTA loads 128 of the tile's 256 weight
-    // rows, which is the box of `mb` already).  Measured at 2,048 rows: 4,608 features (the 7B sizes) 25.0 ms a prefill step
-    // against 26.1; 2,048 features (1.5B) and 1,152 (0.5B) gain nothing, so the rule starts at 4,096.
-    if (M >= 512 && N >= 4 * pair_min_features() && pair_tiles_enabled())
+    // rows, which is the box of `mb` already).  Measured at 2,030 rows: 2,048 features (the 1.5B sizes) 17.8 us against 23.8,
+    // 4,608 (7B) 25.0 ms a prefill step of 2,048 rows against 26.1; 1,152 features (0.5B) fill 144 multiprocessors as they are.
+    p.width = 256;
+    if (M >= 512 && N >= 2 * pair_min_features() && pair_tiles_enabled())
         return hd == 128 ? launch_persistent<EPI_ROPE128, 256, true>(ma, mb, mq, p, stream)
                          : launch_persistent<EPI_ROPE64, 256, true>(ma, mb, mq, p, stream);
     return hd == 128 ? launch_persistent<EPI_ROPE128, 128>(ma, mb, mq, p, stream)

@@ -165,6 +165,22 @@ def test_gemm_tcgen05(ops, M, N, K, epi):
             assert int(ops._meet_counters[dev().index or 0].abs().max()) == 0
 
 
+# tiles of 192, 224, 160 and 128 features a pair; the last tile whole and ragged, its last rows missing
+@pytest.mark.parametrize("M,N,K", [(2030, 1536, 72), (2100, 3584, 200), (1025, 2400, 136), (530, 5000, 64), (2048, 9728, 136), (2300, 1290, 64)])
+@pytest.mark.parametrize("epi", [1, 2])
+@pytest.mark.parametrize("bias_on", [True, False])
+def test_gemm_tcgen05_pair_widths(ops, M, N, K, epi, bias_on):
+    a, w = rnd((M, K), torch.bfloat16, 44), rnd((N, K), torch.bfloat16, 45, 0.2)
+    bias = rnd((N,), torch.float32, 46) if bias_on else None
+    got = rnd((M, N), torch.float32, 47) if epi == 2 else torch.full((M, N), float("nan"), device=dev())
+    ref = gemm_reference(a, w, bias, epi, got)
+    ops.gemm_tcgen05(a, w, bias, epi, None if epi == 2 else got, got if epi == 2 else None)
+    ops.check_async_errors(dev())
+    got, tol = got.double().cpu(), 1e-5 * math.sqrt(K)
+    assert not torch.isnan(got).any()
+    assert torch.allclose(got, ref, atol=tol * max(1.0, float(ref.abs().max())), rtol=0), f"max diff {float((got - ref).abs().max())}"
+
+
 DECODE_SHAPES = [(1, 1152, 896), (8, 9728, 896), (13, 896, 4864), (16, 130, 64), (17, 200, 136), (40, 1000, 96),
                  (64, 384, 192)]
 
