@@ -32,16 +32,27 @@ using namespace t5;
 
 // SiLU for the bf16 epilogues: the fast exponential and division are far inside bf16's rounding.
 __device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
-// The GLU epilogue's activation on a (gate, up) pair: SiLU with the fast or the exact exponential, or what glu.kind names.
-template <bool FAST>
-__device__ __forceinline__ float glu_pair(const LlbGluArgs& glu, float g, float u) {
-    if (glu.kind == LLB_GLU_SILU) return (FAST ? silu_fast(g) : llb_silu(g)) * u;
-    if (FAST && glu.kind == LLB_GLU_CLAMPED_SWISH) {          // the clamped gate with the fast exponential and division
-        g = fminf(g, glu.limit);
-        u = fminf(fmaxf(u, -glu.limit), glu.limit);
-        return __fdividef(g, 1.0f + __expf(-glu.alpha * g)) * (u + glu.up_shift);
+
+// The outputs of neighbouring accumulators, two each.  The activation is chosen once: chosen pair by pair, every pair was a branch of its own
+// whose exponential and division nothing overlapped, and with all of them unrolled 16 times the code did not stay in the instruction
+// cache (a tile of 128 x 256 took the epilogue twice its products' time at K = 896).  us: 2,048 x 9,728 x 896 44.6 -> 31.7 (1,125 TFLOP/s),
+// 4,096 x 9,728 x 896 84 -> 57, 2,030 x 17,920 x 1,536 85.4 -> 83.4 (its products pace it).
+template <bool FAST, int N>
+__device__ __forceinline__ void glu_row(const LlbGluArgs& glu, const float (&v)[2 * N], float (&out)[N]) {
+    if (glu.kind == LLB_GLU_SILU) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) out[j] = (FAST ? silu_fast(v[2 * j]) : llb_silu(v[2 * j])) * v[2 * j + 1];
+    } else if (FAST && glu.kind == LLB_GLU_CLAMPED_SWISH) {
+        const float alpha = glu.alpha, limit = glu.limit, shift = glu.up_shift;
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const float g = fminf(v[2 * j], limit), u = fminf(fmaxf(v[2 * j + 1], -limit), limit);
+            out[j] = __fdividef(g, 1.0f + __expf(-alpha * g)) * (u + shift);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; ++j) out[j] = llb_glu(v[2 * j], v[2 * j + 1], glu.kind, glu.alpha, glu.limit, glu.up_shift);
     }
-    return llb_glu(g, u, glu.kind, glu.alpha, glu.limit, glu.up_shift);
 }
 
 constexpr int TILE_M = 128;       // rows of the A role = TMEM lanes
@@ -100,23 +111,24 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, int m, int nb,
         }
         if (EPI == LLB_EPI_SWIGLU) {
             __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)m * (p.N / 2) + (nb >> 1);
+            float y[CHUNK / 2];
             if (full && (p.N % 16) == 0) {     // 16-byte stores of 8 outputs
+                glu_row<true, CHUNK / 2>(p.glu, v, y);
 #pragma unroll
-                for (int j = 0; j < CHUNK; j += 16) {
+                for (int j = 0; j < CHUNK / 2; j += 8) {
                     uint32_t w[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        const __nv_bfloat162 h = __floats2bfloat162_rn(
-                            glu_pair<true>(p.glu, v[j + 4 * e], v[j + 4 * e + 1]),
-                            glu_pair<true>(p.glu, v[j + 4 * e + 2], v[j + 4 * e + 3]));
+                        const __nv_bfloat162 h = __floats2bfloat162_rn(y[j + 2 * e], y[j + 2 * e + 1]);
                         w[e] = *reinterpret_cast<const uint32_t*>(&h);
                     }
-                    *reinterpret_cast<uint4*>(o + (j >> 1)) = make_uint4(w[0], w[1], w[2], w[3]);
+                    *reinterpret_cast<uint4*>(o + j) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
             } else {
+                glu_row<false, CHUNK / 2>(p.glu, v, y);
 #pragma unroll
-                for (int j = 0; j < CHUNK; j += 2)
-                    if (nb + j + 1 < p.N) o[j >> 1] = __float2bfloat16_rn(glu_pair<false>(p.glu, v[j], v[j + 1]));
+                for (int j = 0; j < CHUNK / 2; ++j)
+                    if (nb + 2 * j + 1 < p.N) o[j] = __float2bfloat16_rn(y[j]);
             }
         } else if (EPI == LLB_EPI_STORE) {
             if (p.glu.kind == LLB_ACT_SQUARED_RELU) {
@@ -286,7 +298,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 const float other = __shfl_xor_sync(0xffffffffu, v, 1);   // gate in even rows, up in odd
                                 if ((lane & 1) == 0 && m < p.M && n + 1 < p.N)
                                     ((__nv_bfloat16*)p.out)[(size_t)m * (p.N / 2) + (n >> 1)] =
-                                        __float2bfloat16_rn(glu_pair<false>(p.glu, v, other));
+                                        __float2bfloat16_rn(llb_glu(v, other, p.glu.kind, p.glu.alpha, p.glu.limit, p.glu.up_shift));
                             } else if (m < p.M && n < p.N) {
                                 const size_t idx = (size_t)m * p.N + n;
                                 if (EPI == LLB_EPI_STORE_F32 || EPI == LLB_EPI_RESIDUAL) v *= llb_out_scale(p.glu);
@@ -374,13 +386,14 @@ __device__ __forceinline__ void staged_chunk(const GemmParams& p, const CUtensor
             *reinterpret_cast<uint4*>(row + (((piece * CHUNKS + c) ^ (lane & 7)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
     } else {      // SiLU(gate) * up on interleaved features: 32 accumulator columns give 16 outputs
+        float y[16];
+        glu_row<true, 16>(p.glu, v, y);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             uint32_t w[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int j = 16 * c + 4 * e;
-                const __nv_bfloat162 h = __floats2bfloat162_rn(glu_pair<true>(p.glu, v[j], v[j + 1]), glu_pair<true>(p.glu, v[j + 2], v[j + 3]));
+                const __nv_bfloat162 h = __floats2bfloat162_rn(y[8 * c + 2 * e], y[8 * c + 2 * e + 1]);
                 w[e] = *reinterpret_cast<const uint32_t*>(&h);
             }
             *reinterpret_cast<uint4*>(row + (((piece * CHUNKS + c) ^ (lane & 7)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
