@@ -38,6 +38,7 @@ struct AttnParams {
     const int* span_pos;
     const int* block_table;
     int max_pages, page_size, Hq, Hkv, hd, window, BQ, nsplit;
+    int key_groups;    // of warps that share a block's keys (tiles of rows in 32 bits)
     int share;            // groups of query heads that read one kv head of the cache: `Hkv` counts the groups, Hkv / share the cache's
                           // heads (1 unless a group's rows would not fit in shared memory; a divisor of the heads a kv head)
     int hdv;              // width of a value row and of an output row (hd for ordinary attention)
@@ -518,19 +519,30 @@ size_t attention_smem_bytes(int BQ, int G, int hd, int hdv) {
 // kv head and walks their keys 64 at a time.  Scores and P V are register tiles (4 queries x 4 keys, 4 queries x 4
 // dimensions a thread, 16-byte shared loads), so the FFMA pipe and not the shared memory paces it; the kernel above spends a
 // shared load on every product (24 layers of a 389-token prompt at 14 / 2 heads of 64: 890 -> 62 us a layer).  Row maxima and sums are exchanged between the 16 threads that share a query row.
+// Groups of four warps share the queries and take the tiles of keys in turn; what they found is merged at the end.  One group alone walks
+// all of a long row's tiles with one warp a scheduler, and what paces a tile then is its own chain: two loads one behind the other,
+// some 4,000 instructions.  us at 14 / 2 heads of 64, one group -> four: a prompt of 150 26.9 -> 15.8, of 389 62 -> 30.5; two: of 1,000
+// 178 -> 103; but 30 prompts of 30 tokens 15.5 -> 21.6 (one group stays).
 constexpr int TQ = 32, TKEYS = 64, TP = TKEYS + 4;
-template <int HD> constexpr size_t tile_f32_smem() { return sizeof(float) * ((size_t)TQ * (HD + 4) + TKEYS * (HD + 4) + TKEYS * HD + TQ * TP); }
+constexpr int GROUP_THREADS = 128;
+template <int HD> constexpr int tile_f32_group() { return TKEYS * (HD + 4) + TKEYS * HD + TQ * TP; }          // floats
+template <int HD, int GROUPS> constexpr size_t tile_f32_smem() { return sizeof(float) * ((size_t)TQ * (HD + 4) + GROUPS * tile_f32_group<HD>()); }
+__device__ __forceinline__ void group_sync(int group) {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(GROUP_THREADS) : "memory");
+}
 
-template <int HD>
-__global__ void __launch_bounds__(128) paged_attention_tile_f32_kernel(AttnParams p, int chunks, int per) {
+template <int HD, int GROUPS>
+__global__ void __launch_bounds__(GROUPS * GROUP_THREADS) paged_attention_tile_f32_kernel(AttnParams p, int chunks, int per) {
     extern __shared__ __align__(16) float smem[];
     constexpr int LD = HD + 4, ND = HD / 64;
     float* Qs = smem;                        // [TQ][LD]
-    float* Ks = Qs + TQ * LD;                // [TKEYS][LD]
+    const int group = threadIdx.x / GROUP_THREADS, tid = threadIdx.x % GROUP_THREADS;
+    float* Ks = Qs + TQ * LD + group * tile_f32_group<HD>();          // [TKEYS][LD]
     float* Vs = Ks + TKEYS * LD;             // [TKEYS][HD]
     float* Ps = Vs + TKEYS * HD;             // [TQ][TP]
-    const int tile = gridDim.x - 1 - blockIdx.x;          // later tiles of a span have more keys: they start first
-    const int kvh = blockIdx.y / chunks, chunk = blockIdx.y % chunks;
+    // Later tiles of a span have more keys: all blocks of theirs start first, so that a multiprocessor's second block is a short one
+    const int per_tile = p.Hkv * chunks, tile = (int)((gridDim.x - 1 - blockIdx.x) / per_tile), part = (gridDim.x - 1 - blockIdx.x) % per_tile;
+    const int kvh = part / chunks, chunk = part % chunks;
     const int G = p.Hq / p.Hkv;
     const int span = p.tile_span[tile], q0 = p.tile_q0[tile];
     const int row0 = p.span_row[span] + q0, pos0 = p.span_pos[span] + q0;
@@ -544,8 +556,8 @@ __global__ void __launch_bounds__(128) paged_attention_tile_f32_kernel(AttnParam
     const int r_lo = v_lo / G, r_hi = (v_lo + nv - 1) / G;
     const LlbKeys keys = llb_keys(llb_first_visible(pos0 + r_lo, p.window), pos0 + r_hi + 1, p.keep);
 
-    const int tid = threadIdx.x, tq = tid >> 4, tl = tid & 15;
-    for (int i = tid; i < TQ * (HD / 4); i += 128) {
+    const int tq = tid >> 4, tl = tid & 15;
+    for (int i = threadIdx.x; i < TQ * (HD / 4); i += GROUPS * GROUP_THREADS) {
         const int v = i / (HD / 4), d = (i % (HD / 4)) * 4;
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
         if (v < nv) {
@@ -566,8 +578,9 @@ __global__ void __launch_bounds__(128) paged_attention_tile_f32_kernel(AttnParam
 #pragma unroll
         for (int d = 0; d < 4 * ND; ++d) o[i][d] = 0.0f;
     }
-    for (int kb = 0; kb < keys.count; kb += TKEYS) {
-        __syncthreads();          // the last tile has been read (and the queries are there)
+    __syncthreads();              // the queries are there
+    for (int kb = group * TKEYS; kb < keys.count; kb += GROUPS * TKEYS) {
+        group_sync(group);        // the group's last tile has been read
         for (int i = tid; i < TKEYS * (HD / 4); i += 128) {
             const int j = i / (HD / 4), d = (i % (HD / 4)) * 4;
             float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f), v4 = k4;
@@ -580,7 +593,7 @@ __global__ void __launch_bounds__(128) paged_attention_tile_f32_kernel(AttnParam
             *reinterpret_cast<float4*>(Ks + j * LD + d) = k4;
             *reinterpret_cast<float4*>(Vs + j * HD + d) = v4;
         }
-        __syncthreads();
+        group_sync(group);
         float s[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -658,6 +671,36 @@ __global__ void __launch_bounds__(128) paged_attention_tile_f32_kernel(AttnParam
         }
         __syncwarp();
     }
+    // group 0 adds what the others leave in their own tiles' place: [4 rows][2 + 4 ND values][128 threads]
+    constexpr int LEFT = 2 + 4 * ND;
+    static_assert(4 * LEFT * GROUP_THREADS <= tile_f32_group<HD>(), "the sums of one group over its tiles");
+    if (group > 0) {
+        float* left = Ks + tid;
+        group_sync(group);        // every warp of the group has read its last tile
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            left[(i * LEFT) * GROUP_THREADS] = m[i];
+            left[(i * LEFT + 1) * GROUP_THREADS] = l[i];
+#pragma unroll
+            for (int d = 0; d < 4 * ND; ++d) left[(i * LEFT + 2 + d) * GROUP_THREADS] = o[i][d];
+        }
+    }
+    __syncthreads();
+    if (group > 0) return;
+#pragma unroll 1
+    for (int other = 1; other < GROUPS; ++other) {
+        const float* left = Ks + other * tile_f32_group<HD>() + tid;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float m1 = left[(i * LEFT) * GROUP_THREADS];
+            if (m1 == -INFINITY) continue;          // no visible key among the group's
+            const float top = fmaxf(m[i], m1), keep = expf(m[i] - top), add = expf(m1 - top);
+            l[i] = l[i] * keep + left[(i * LEFT + 1) * GROUP_THREADS] * add;
+            m[i] = top;
+#pragma unroll
+            for (int d = 0; d < 4 * ND; ++d) o[i][d] = o[i][d] * keep + left[(i * LEFT + 2 + d) * GROUP_THREADS] * add;
+        }
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int v = tq + 8 * i;
@@ -683,27 +726,38 @@ bool tile_f32_eligible(const AttnParams& p) {
            (((uintptr_t)p.q | (uintptr_t)p.k_cache | (uintptr_t)p.v_cache | (uintptr_t)p.out) % 16) == 0;
 }
 
-template <int HD>
+template <int HD, int GROUPS>
 int launch_tile_f32(const AttnParams& p, int num_tiles, cudaStream_t stream) {
+    constexpr size_t smem = tile_f32_smem<HD, GROUPS>();
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(paged_attention_tile_f32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)tile_f32_smem<HD>());
+        const cudaError_t e = cudaFuncSetAttribute(paged_attention_tile_f32_kernel<HD, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)smem);
         if (e != cudaSuccess) return llb_fail("attention: cannot opt in to shared memory: %s", cudaGetErrorString(e));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
     const int vectors = p.BQ * (p.Hq / p.Hkv), chunks = llb_ceil_div(vectors, TQ);
-    paged_attention_tile_f32_kernel<HD><<<dim3(num_tiles, p.Hkv * chunks), 128, tile_f32_smem<HD>(), stream>>>(
+    paged_attention_tile_f32_kernel<HD, GROUPS><<<num_tiles * p.Hkv * chunks, GROUPS * GROUP_THREADS, smem, stream>>>(
         p, chunks, llb_ceil_div(vectors, chunks));
     return llb_check_launch("paged_attention_tile_f32");
 }
 
+// As many groups as the caller asks for (who knows how long the rows are: a block of few keys keeps one group busy, and blocks of
+// several groups take the place of more blocks), two at most for heads of 128.
+int dispatch_tile_f32(const AttnParams& p, int num_tiles, cudaStream_t stream) {
+    if (p.hd != 64) return p.key_groups > 1 ? launch_tile_f32<128, 2>(p, num_tiles, stream) : launch_tile_f32<128, 1>(p, num_tiles, stream);
+    if (p.key_groups == 4) return launch_tile_f32<64, 4>(p, num_tiles, stream);
+    return p.key_groups == 2 ? launch_tile_f32<64, 2>(p, num_tiles, stream) : launch_tile_f32<64, 1>(p, num_tiles, stream);
+}
+
 template <typename T>
 int launch_attention(AttnParams p, int num_tiles, cudaStream_t stream) {
-    if (tile_f32_eligible<T>(p) && !decode_eligible<T>(p))
-        return p.hd == 64 ? launch_tile_f32<64>(p, num_tiles, stream) : launch_tile_f32<128>(p, num_tiles, stream);
+    // (blocks are numbered in one dimension)
+    if (tile_f32_eligible<T>(p) && !decode_eligible<T>(p) &&
+        (long long)num_tiles * p.Hkv * llb_ceil_div(p.BQ * (p.Hq / p.Hkv), TQ) < (1ll << 31))
+        return dispatch_tile_f32(p, num_tiles, stream);
     // many heads over wide rows: as many blocks share a kv head as it takes for one block's heads to fit
     const int heads = p.Hq / p.Hkv;
     while (p.share < heads && attention_smem_bytes(p.BQ, heads / p.share, p.hd, p.hdv) > 200 * 1024)
@@ -761,7 +815,8 @@ LLB_EXPORT long long llb_attention_scratch_floats(int num_tiles, int Hq, int hd,
 // tile_span, tile_q0 [num_tiles]; span_row, span_len, span_pos [S]; block_table [S, max_pages].
 // window: > 0 the latest keys, < 0 the query's own block of -window positions, 0 every earlier key (llb_first_visible).  sinks [Hq] float or null: exp(sinks[h]) is added once to head h's
 // softmax denominator (a logit without key or value, not scaled).  scratch: num_tiles*Hq*BQ*nsplit*(hdv+2) floats
-// when nsplit > 1, else unused.
+// when nsplit > 1, else unused.  nsplit = -2 or -4: one piece, and where the tiles of rows in 32 bits serve the call, so many groups of
+// warps of a block share its keys.
 // v_shared != 0: v_cache is [slots, hdv] and every query head reads the whole row (out [T, Hq, hdv]): the products of a
 // head's softmax weights with the values of ALL kv heads, for mixers that combine heads' weights after the softmax.
 // out_f32 != 0: out is float whatever `dtype` says.
@@ -780,6 +835,8 @@ LLB_EXPORT int llb_paged_attention_biased(const void* q, const void* k_cache, co
     LLB_REQUIRE(num_tiles > 0 && Hq > 0 && Hkv > 0 && hd > 0 && hdv > 0 && page_size > 0 && max_pages > 0 && BQ > 0,
                 "attention: bad sizes");
     LLB_REQUIRE(Hq % Hkv == 0, "attention: %d query heads are not a multiple of %d kv heads", Hq, Hkv);
+    const int groups = nsplit == -4 ? 4 : nsplit == -2 ? 2 : 1;
+    if (groups > 1) nsplit = 1;
     LLB_REQUIRE(nsplit >= 1 && nsplit <= MERGE_MAX_SPLITS && Hkv <= 65535,
                 "attention: split count %d is outside 1..%d", nsplit, MERGE_MAX_SPLITS);
     LLB_REQUIRE(nsplit == 1 || scratch != nullptr, "attention: nsplit=%d needs scratch", nsplit);
@@ -788,7 +845,7 @@ LLB_EXPORT int llb_paged_attention_biased(const void* q, const void* k_cache, co
     p.tile_span = tile_span; p.tile_q0 = tile_q0;
     p.span_row = span_row; p.span_len = span_len; p.span_pos = span_pos; p.block_table = block_table;
     p.max_pages = max_pages; p.page_size = page_size; p.Hq = Hq; p.Hkv = Hkv; p.hd = hd;
-    p.window = window; p.BQ = BQ; p.nsplit = nsplit; p.scale = scale;
+    p.window = window; p.BQ = BQ; p.nsplit = nsplit; p.key_groups = groups; p.scale = scale;
     p.softcap = softcap > 0.0f ? softcap : 0.0f;
     p.hdv = hdv; p.vrow = vrow; p.sinks = sinks; p.share = 1;
     LLB_REQUIRE(vrow >= hdv, "attention: value rows of %d numbers, %d apart", hdv, vrow);

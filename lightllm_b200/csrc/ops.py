@@ -265,7 +265,8 @@ def paged_attention_simt(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
     not capped).  ``v_stride``: numbers from one value row to the next when it is not ``v_head_dim`` (values that are the
     first ``v_head_dim`` numbers of the key rows: ``head_dim``).  ``keep``: the first ``keep`` positions stay visible whatever
     the window says.  ``slopes`` float32 [num_heads]: ``slopes[h] * (query position - key position)`` is taken off head h's
-    scores after the cap."""
+    scores after the cap.  ``nsplit`` of -2 or -4: one piece, whose keys that many groups of a block's warps share where the
+    tiled 32-bit kernel serves the call."""
     hdv = head_dim if v_head_dim is None else v_head_dim
     if k_cache.dtype != q.dtype or v_cache.dtype != q.dtype or out.dtype not in (q.dtype, torch.float32):
         raise KernelError("attention: q and the caches must share a dtype, out has it or is float32")

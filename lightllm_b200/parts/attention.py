@@ -293,6 +293,30 @@ class AttentionMixer(Mixer):
         ctx.shape_key.append(("even", pieces))
         return -pieces
 
+    def _key_groups(self, ctx, which, bq: int, window: int) -> int:
+        """Into how many groups the tiled 32-bit kernel deals the keys of its blocks, as a negative split count (1: not).  Groups shorten
+        a block and take the place of other blocks, so they are for few blocks, or for rows of several tiles of 64 keys."""
+        if ctx.dtype != torch.float32 or self.head_dim not in (64, 128) or self.v_head_dim != self.head_dim:
+            return 1
+        lengths = np.array([ctx.spans[i].length for i in which], dtype=np.int64)
+        ends = np.array([ctx.spans[i].start for i in which], dtype=np.int64) + lengths
+        tiles = -(-lengths // bq)
+        if window:
+            ends = np.minimum(ends, abs(window) + self.keep_first + bq)
+        if ends.max() <= 128:
+            return 1
+        keys = ends if window else ends - lengths / 2          # of a span's average tile, about
+        rounds = float((tiles * np.maximum(1.0, keys / 64)).sum() / tiles.sum())
+        sms = L.num_sms(ctx.device)
+        blocks = int(tiles.sum()) * self.num_kv_heads * -(-bq * (self.num_heads // self.num_kv_heads) // 32)
+        groups = 1
+        if blocks <= sms or (blocks <= sms * 3 // 2 and rounds >= 2.3):
+            groups = 4
+        elif rounds >= 3.0:
+            groups = 2
+        ctx.shape_key.append(("key_groups", groups))
+        return -groups if groups > 1 else 1
+
     def _plan_mixed(self, ctx, bf16: bool, window: int):
         """A step with portions of prompts, maybe beside decoded tokens.  Each span goes where its shape is served best:
         portions of two rows or more to the tensor-core kernel in tiles of 128 rows;
@@ -334,7 +358,7 @@ class AttentionMixer(Mixer):
             simt.append((ctx.tiles(1, select=tuple(rows)), 1, max(2, min(16, -(-rows_keys // 256)))))
         if rest:
             bq = self.tile_height()
-            simt.append((ctx.tiles(bq, select=tuple(rest)), bq, 1))
+            simt.append((ctx.tiles(bq, select=tuple(rest)), bq, self._key_groups(ctx, rest, bq, window)))
         return ("mixed", items, decode, simt)
 
     @property

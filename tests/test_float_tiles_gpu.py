@@ -61,6 +61,25 @@ def test_float_contraction_of_what_bf16_does_not_hold(ops, M, N, K):  # noqa: F8
     assert bool(beyond.all())          # sums that pass the largest float on the way are infinite or NaN, as with FFMA
 
 
+@pytest.mark.parametrize("Hq,Hkv,hd", [(14, 2, 64), (3, 3, 128), (12, 2, 128)])
+@pytest.mark.parametrize("window", [None, 70])
+@pytest.mark.parametrize("groups", [2, 4])
+def test_float_attention_by_groups(ops, Hq, Hkv, hd, window, groups):  # noqa: F811
+    """Groups of warps that share a block's keys: fewer tiles of keys than groups, as many, and more; windows that leave groups without."""
+    lens, starts = [1, 16, 67, 33, 20], [0, 63, 0, 130, 440]
+    s = paged_setup(torch.float32, lens, starts, Hq, Hkv, hd, 16, 13)
+    ts, tq, nt = tiles_for(lens, 16)
+    outs = []
+    for nsplit in (1, -groups):
+        out = torch.full((s["rows"], Hq * hd), float("nan"), device=dev())
+        ops.paged_attention_simt(s["q"], s["kc"], s["vc"], out, ts, tq, nt, s["span_row"], s["span_len"], s["span_pos"], s["bt"],
+                                 s["max_pages"], 16, Hq, Hkv, hd, window or 0, hd ** -0.5, 16, nsplit)
+        outs.append(out.cpu())
+    ref = attention_reference(s["full"], lens, starts, hd, window).reshape(s["rows"], Hq * hd)
+    assert not torch.isnan(outs[1]).any()
+    assert torch.allclose(outs[1], ref, atol=2e-5, rtol=2e-5) and torch.allclose(outs[0], outs[1], atol=2e-6, rtol=2e-6)
+
+
 @pytest.mark.parametrize("Hq,Hkv,hd", [(14, 2, 64), (3, 3, 128), (9, 1, 64), (12, 2, 128)])
 @pytest.mark.parametrize("window", [None, 33])
 @pytest.mark.parametrize("bq", [16, 5])
