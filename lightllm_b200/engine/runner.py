@@ -394,13 +394,22 @@ class ModelRunner:
             return logits
         return logits.index_select(0, ctx.select_rows)
 
+    @staticmethod
+    def graph_key(ctx: StepContext) -> tuple:
+        """What the launches of a step depend on: steps of one key may share a CUDA graph.  A decoding batch and a step described
+        row by row can agree in every count, and must not share one: row by row, several rows may be one request's, so the
+        persistent layer kernel does not take them, and the decode attention may not read a row's latest positions
+        (``fresh_positions``) before the kernel that writes them has completed."""
+        return (ctx.T, ctx.num_spans, ctx.num_want, ctx.max_pages, ctx.decode_only, ctx.rowwise, ctx.fresh_positions,
+                tuple(ctx.shape_key))
+
     def _forward_graphed(self, ctx: StepContext) -> Optional[torch.Tensor]:
         """A step through a CUDA graph.  The metadata buffer has equal addresses for equal counts, so a
         graph captured for (tokens, requests, wanted rows, block-table width, sizes of the staged index
         arrays and what else the parts named) serves every later step of that shape; only the metadata
         copy stays outside."""
         from ..csrc import ops
-        key = (ctx.T, ctx.num_spans, ctx.num_want, ctx.max_pages, ctx.decode_only, tuple(ctx.shape_key))
+        key = self.graph_key(ctx)
         hit = self._graphs.get(key)
         if hit is not None:
             self._graphs[key] = self._graphs.pop(key)          # most recently used last

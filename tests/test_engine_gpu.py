@@ -453,6 +453,46 @@ def test_small_mixed_steps_described_row_by_row(tmp_path, monkeypatch, name, dty
     assert worst <= tol, worst
 
 
+@pytest.mark.parametrize("fused", ["0", "1"])
+@pytest.mark.parametrize("name", ["D", "E"])
+def test_a_step_row_by_row_after_decoding_batches_of_as_many_rows(tmp_path, monkeypatch, name, fused):
+    """Batches of eight tokens run from their graph; then steps of two tokens and a portion of six (eight rows, row by row), whose
+    rows read what the rows before them wrote in the same step, follow the plain implementation, and so do batches after them."""
+    monkeypatch.setenv("LLB_FUSED_DECODE", fused)
+    d = model_dir(tmp_path, name, seed=33, store="bfloat16", edit=sharpen(3.0))
+    cfg, w = P.read_model_dir(d)
+    rng = random.Random(34)
+    page = PAGE_SIZE[name]
+    seqs = {i: [rng.randrange(cfg["vocab_size"]) for _ in range(140)] for i in range(8)}
+    ref = {i: P.plain_forward(cfg, w, s) for i, s in seqs.items()}
+    core = EngineCore(d, EngineOptions(dtype="bfloat16", max_seq_len=256, max_batch_tokens=1024, page_size=page,
+                                       num_pages=9 * (-(-144 // page) + 1), max_seqs=8))
+    at, worst = {}, 0.0
+    for i in seqs:
+        core.open(i)
+        at[i] = 0
+
+    def step(parts):
+        nonlocal worst
+        out = core.step([StepEntry(i, seqs[i][at[i]: at[i] + n], [n - 1]) for i, n in parts])
+        for k, (i, n) in enumerate(parts):
+            at[i] += n
+            worst = max(worst, float((out[k].float().cpu() - ref[i][at[i] - 1]).abs().max()))
+        return core.runner.last_ctx
+
+    step([(i, 100) for i in seqs])
+    for _ in range(4):
+        assert not step([(i, 1) for i in seqs]).rowwise
+    assert core.runner.graph_replays > 0
+    for k in range(4):
+        ctx = step([(k, 1), ((k + 1) % 8, 1), ((k + 2) % 8, 6)])
+        assert ctx.rowwise and ctx.T == 8
+    for _ in range(2):
+        assert not step([(i, 1) for i in seqs]).rowwise
+    core.runner.check_device_errors()
+    assert worst <= atol_for(name + " sharp", "bfloat16", ref), worst
+
+
 def test_token_ids_taken_from_the_device(tmp_path):
     """``step(entries, device_tokens)`` reads the step's ids from a device tensor (the entries only give the counts):
     a decoding batch, and a small mixed step that is described row by row and padded, where the padding has to

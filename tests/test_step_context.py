@@ -145,3 +145,34 @@ def test_a_mixed_step_described_row_by_row():
     assert len(rows) == 16                                   # already a multiple of the bucket: no padding
     rows, _ = rows_as_spans([Span("a", 0, 10, 61, 0)], 8, 62)
     assert len(rows) == 62 and all(r.start == 70 for r in rows[61:])      # the bucket stops at the row limit
+
+
+def test_a_decoding_batch_and_a_step_row_by_row_share_no_graph():
+    """Eight requests of one token, and two tokens beside a portion of six, have equal counts once the second is described row by row.
+    The first one's graph reads a row's latest positions early, or runs the persistent kernel, and must not serve the second."""
+    from types import SimpleNamespace
+    from lightllm_b200.engine.runner import ModelRunner
+    captured = []
+
+    class Graph:
+        def __init__(self, ctx):
+            self.rowwise = ctx.rowwise
+
+        def replay(self):
+            captured.append(self.rowwise)
+
+    runner = SimpleNamespace(_graphs={}, _graph_seen={}, max_graphs=4, graph_replays=0, graph_launches=0,
+                             MIXED_CAPTURE_AFTER=ModelRunner.MIXED_CAPTURE_AFTER, forward=lambda ctx: None,
+                             _picked=lambda ctx, logits: logits, _capture=lambda ctx: (Graph(ctx), None),
+                             graph_key=getattr(ModelRunner, "graph_key", None))
+
+    def step(rowwise):
+        ctx = context([(90 + i, 1, i) for i in range(8)])
+        ctx.T, ctx.num_want, ctx.max_pages, ctx.decode_only = 8, 8, 32, True
+        ctx.rowwise, ctx.fresh_positions = rowwise, ModelRunner.ROWWISE_MAX_ROWS if rowwise else 1
+        ctx.tiles(1)
+        ModelRunner._forward_graphed(runner, ctx)
+
+    for rowwise in (False, False, True, True, False, True):
+        step(rowwise)
+    assert captured == [False, True, False, True]          # each from its second sight on, from a graph of its own kind
