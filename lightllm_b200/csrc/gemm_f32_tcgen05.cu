@@ -4,7 +4,7 @@
 // calls cublasSgemm, src/ops/gemm.cu:92-97).  The tensor cores multiply bf16 exactly but take no floats, and they cut off what
 // does not fit a float after every instruction instead of rounding it.  So
 //   * every operand is the sum of three bf16 numbers, x = x1 + x2 + x3 (each rounded to nearest from what is left, which is
-//     exact for a float's 24 bits).  The weights are split on the way into shared memory, so no copy of them is kept; the
+//     exact for a float's 24 bits, see UP).  The weights are split on the way into shared memory, so no copy of them is kept; the
 //     tokens, which every tile of features reads, by a kernel before this one (split in every block they took most of its
 //     instructions: 1,670 issue cycles a slice of 32 columns beside 900 of products);
 //   * of the nine products the six that matter are computed: x1 w1 into an accumulator of its own, x1 w2, x2 w1, x2 w2,
@@ -12,7 +12,7 @@
 //   * the accumulator of x1 w1 is read, and begun anew, every 32 columns of K, and its values are added up in registers,
 //     rounded to nearest.  Left in tensor memory over all of K the cut-off bits add up: 8.6e-7 off 64 bits (2-norm) at K = 896
 //     where FFMA is 8.4e-8 off; the corrections are 2^-9 of the sum and may stay.
-// What does not fit that form (an infinity, a NaN, values that round to infinity in bf16) shows as a sum that is no finite
+// What does not fit that form (an infinity, a NaN, operands beyond 2^104, sums beyond 2^80) shows as a sum that is no finite
 // number; a block that sees one does its tile again with FFMA, so such inputs give what float arithmetic gives.
 //
 // A block makes a tile of 128 features (the MMA's 128 rows) x up to 160 tokens.  Sixteen warps fetch weights (two slices of 32
@@ -70,6 +70,11 @@ __device__ __forceinline__ uint64_t desc_kmajor64(uint32_t addr) {
     return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) | ((uint64_t)1 << 46) |
            ((uint64_t)4 << 61);
 }
+// Operands are split at 2^24 times their size and the sums taken back: every float is a whole multiple of 2^-149, so that a part is zero or
+// at least 2^-125, within what bf16 holds without losing bits (split as it is, a float below 2^-109 loses the third part, below 2^-117
+// the second: 2.7e-4 off at 1e-37).  Powers of two leave all other roundings as they are.
+constexpr float UP = 16777216.0f, DOWN = 1.0f / (UP * UP);
+__device__ __forceinline__ float4 scaled_up(const float4& v) { return make_float4(v.x * UP, v.y * UP, v.z * UP, v.w * UP); }
 // Two floats as three pairs of bf16 that add up to them.
 __device__ __forceinline__ void split2(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
     h = pack_bf16(x, y);
@@ -104,8 +109,8 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
     const int m = (int)(i / per_row), k = (int)(i - (long long)m * per_row) * 8;
     const float* src = A + (size_t)m * K + k;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 a = k < K ? *reinterpret_cast<const float4*>(src) : zero;
-    const float4 b = k + 4 < K ? *reinterpret_cast<const float4*>(src + 4) : zero;
+    const float4 a = scaled_up(k < K ? *reinterpret_cast<const float4*>(src) : zero);
+    const float4 b = scaled_up(k + 4 < K ? *reinterpret_cast<const float4*>(src + 4) : zero);
     uint4 h, m4, l;
     split2(a.x, a.y, h.x, m4.x, l.x);
     split2(a.z, a.w, h.y, m4.y, l.y);
@@ -284,7 +289,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const __gr
                 const int i = i0 + u;
                 if (i < slices) {
                     // (the stage is free: this thread has waited for the products of slice i - 4)
-                    if (ok) store_split(at + (i % STAGES) * STAGE_BYTES, w[u][0], w[u][1]);
+                    if (ok) store_split(at + (i % STAGES) * STAGE_BYTES, scaled_up(w[u][0]), scaled_up(w[u][1]));
                     fetch(i + 2, u);
                     fence_async_smem();
                     __syncwarp();
@@ -324,7 +329,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const __gr
         } else {
 #pragma unroll
             for (int j = 0; j < WARP_TOKENS; ++j)
-                if (t0 + j < rows) sums[(t0 + j) * FEATURES + feature] = acc[j];
+                if (t0 + j < rows) sums[(t0 + j) * FEATURES + feature] = acc[j] * DOWN;
         }
     }
     namespace cg = cooperative_groups;

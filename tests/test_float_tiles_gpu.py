@@ -51,7 +51,7 @@ def test_float_contraction_of_what_bf16_does_not_hold(ops, M, N, K):  # noqa: F8
     ops.gemm_simt(a, w, None, ops.EPI_STORE, out)
     want, got = (a.double() @ w.double().t()).cpu(), out.double().cpu()
     size = (a.abs().double() @ w.abs().double().t()).cpu()
-    bound = (K + 4) * 2.0 ** -24 * size + K * 2.0 ** -133          # (a third part below bf16's smallest number is lost)
+    bound = (K + 4) * 2.0 ** -24 * size
     safe = torch.isfinite(want) & (size < 3.0e38)                  # (no order of the sum passes the largest float)
     assert bool(((got - want).abs()[safe] <= bound[safe]).all()) and int(safe.sum()) >= (M - 6) * N
     assert bool((got[:2] == want[:2]).all()) and bool(torch.isnan(got[2]).all()) and bool(torch.isnan(got[3, 9]))
@@ -59,6 +59,24 @@ def test_float_contraction_of_what_bf16_does_not_hold(ops, M, N, K):  # noqa: F8
     assert bool((got[3][same_sign] == want[3][same_sign]).all())
     beyond = torch.isfinite(want[6]) & (want[6].abs() < 3.0e38) | torch.isnan(got[6]) | torch.isinf(got[6])
     assert bool(beyond.all())          # sums that pass the largest float on the way are infinite or NaN, as with FFMA
+
+
+@pytest.mark.parametrize("M,N,K", [(161, 1030, 516), (40, 128, 10240)])
+@pytest.mark.parametrize("small", [1e-32, 1e-34, 1e-36, 1e-38, 1e-40])
+@pytest.mark.parametrize("which", ["tokens", "weights"])
+def test_float_contraction_of_numbers_below_what_three_bf16_hold(ops, M, N, K, small, which):  # noqa: F811
+    """Operands down to the subnormal floats keep all the bits that they have; the other operand is large, so that the sums are ordinary."""
+    assert ops.lib().llb_gemm_simt_scratch_bytes(0, 0, M, N, K) > 0
+    a, w = rnd((M, K), torch.float32, 21), rnd((N, K), torch.float32, 22)
+    if which == "tokens":
+        a, w = (a.double() * small).float(), w * 1e9
+    else:
+        a, w = a * 1e9, (w.double() * small).float()
+    out = torch.full((M, N), float("nan"), device=dev())
+    ops.gemm_simt(a, w, None, ops.EPI_STORE, out)
+    want = a.double() @ w.double().t()
+    # as for ordinary numbers: 1.4e-7 at the longest K (FFMA 2.7e-7 to 4e-7)
+    assert float((out.double() - want).norm() / want.norm()) < 3e-7
 
 
 @pytest.mark.parametrize("Hq,Hkv,hd", [(14, 2, 64), (3, 3, 128), (12, 2, 128)])
