@@ -174,6 +174,82 @@ __device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, float (&r)[8]) {
                  : "memory");
 }
 
+// A tile's sums in float arithmetic, by the worker warps: for a tile with a sum that is no finite number.  Slices of K go through shared
+// memory (columns first, the next slice on its way in registers), and a thread adds 10 (few rows: 4) tokens x 4 features up in the
+// order of K.  A call of its own, so that its registers are not the kernel's.  Measured, ms, every thread from memory by itself -> here
+// (FFMA throughout): 389 x 9,728 x 896 with one NaN 14.7 -> 0.25, with one in every row 27.9 -> 0.43 (0.23); 389 x 151,936 x 896 114 -> 2.5
+// and 284 -> 5.2 (3.2); 389 x 896 x 4,864 17.1 -> 0.30 (0.16); 24 x 9,728 x 896 1.49 -> 0.10 (0.035).
+// Floats of a column: even, and four columns 8 banks on, so that the eight pieces of four rows that a warp stores meet two by two.
+constexpr int REDO_X = MAX_TOKENS + 2, REDO_W = FEATURES + 2;
+static_assert(REDO_X * 4 % 32 == 8 && REDO_W * 4 % 32 == 8, "see above");
+constexpr int REDO_AT = MAX_TOKENS * FEATURES * 4;                     // behind the sums
+static_assert(REDO_AT + SLICE * (REDO_X + REDO_W) * 4 <= STAGES * STAGE_BYTES, "a slice of floats beside the sums");
+__device__ __forceinline__ void workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory"); }
+template <int RT>          // tokens of a thread; 16 times as many of the tile
+__device__ __noinline__ void redo_tile(const float* __restrict__ A, const float* __restrict__ W, int K, int rows, int features, int k_lo,
+                                       int k_hi, uint8_t* smem) {
+    float* xs = reinterpret_cast<float*>(smem + REDO_AT);          // [SLICE][REDO_X]
+    float* ws = xs + SLICE * REDO_X;                               // [SLICE][REDO_W]
+    constexpr int RF = 4;                                          // a warp: 4 x RT tokens, 8 x 4 features
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int f0 = (warp & 3) * 32 + (lane & 7) * RF, t0 = ((warp >> 2) * 4 + (lane >> 3)) * RT;
+    constexpr int PIECES = SLICE / 4;                              // of four columns of a row, neighbouring threads'
+    constexpr int XN = (16 * RT * PIECES + WORKERS - 1) / WORKERS, WN = FEATURES * PIECES / WORKERS;
+    const int row = tid / PIECES, c = tid % PIECES * 4;
+    constexpr int STRIDE = WORKERS / PIECES;                       // rows on, the thread's next piece
+    float4 x[XN], w[WN];
+    auto fetch = [&](int k) {
+#pragma unroll
+        for (int u = 0; u < XN; ++u)
+            x[u] = row + u * STRIDE < rows && k < k_hi ? __ldg(reinterpret_cast<const float4*>(A + (size_t)(row + u * STRIDE) * K + k))
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < WN; ++u)
+            w[u] = row + u * STRIDE < features && k < k_hi ? __ldg(reinterpret_cast<const float4*>(W + (size_t)(row + u * STRIDE) * K + k))
+                                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto store = [](float* at, int column, const float4& v) {
+        at[0] = v.x; at[column] = v.y; at[2 * column] = v.z; at[3 * column] = v.w;
+    };
+    float acc[RT][RF];
+#pragma unroll
+    for (int j = 0; j < RT; ++j)
+#pragma unroll
+        for (int f = 0; f < RF; ++f) acc[j][f] = 0.0f;
+    fetch(k_lo + c);
+    for (int k0 = k_lo; k0 < k_hi; k0 += SLICE) {
+        workers_sync();          // the slice before has been read
+#pragma unroll
+        for (int u = 0; u < XN; ++u)
+            if (row + u * STRIDE < 16 * RT) store(xs + c * REDO_X + row + u * STRIDE, REDO_X, x[u]);
+#pragma unroll
+        for (int u = 0; u < WN; ++u) store(ws + c * REDO_W + row + u * STRIDE, REDO_W, w[u]);
+        workers_sync();
+        fetch(k0 + SLICE + c);       // (nothing beyond the last column)
+        const int columns = (warp >> 2) * 4 * RT < rows ? min(SLICE, k_hi - k0) : 0;
+#pragma unroll 4
+        for (int k = 0; k < columns; ++k) {
+            const float2 v0 = *reinterpret_cast<const float2*>(ws + k * REDO_W + f0), v1 = *reinterpret_cast<const float2*>(ws + k * REDO_W + f0 + 2);
+#pragma unroll
+            for (int j = 0; j < RT; j += 2) {
+                const float2 t = *reinterpret_cast<const float2*>(xs + k * REDO_X + t0 + j);
+                acc[j][0] = fmaf(t.x, v0.x, acc[j][0]);
+                acc[j][1] = fmaf(t.x, v0.y, acc[j][1]);
+                acc[j][2] = fmaf(t.x, v1.x, acc[j][2]);
+                acc[j][3] = fmaf(t.x, v1.y, acc[j][3]);
+                acc[j + 1][0] = fmaf(t.y, v0.x, acc[j + 1][0]);
+                acc[j + 1][1] = fmaf(t.y, v0.y, acc[j + 1][1]);
+                acc[j + 1][2] = fmaf(t.y, v1.x, acc[j + 1][2]);
+                acc[j + 1][3] = fmaf(t.y, v1.y, acc[j + 1][3]);
+            }
+        }
+    }
+    float* sums = reinterpret_cast<float*>(smem);
+#pragma unroll
+    for (int j = 0; j < RT; ++j)
+        if (t0 + j < rows) *reinterpret_cast<float4*>(sums + (t0 + j) * FEATURES + f0) = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+}
+
 template <int EPI>
 __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const F32Params p) {
     __shared__ __align__(8) uint64_t full[STAGES];      // the slice's operands are there (every worker warp, and the tokens' copies)
@@ -319,13 +395,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const __gr
     float* sums = reinterpret_cast<float*>(smem);
     if (warp < MMA_WARP) {
         if (bad) {
-            const int n = n0 + feature;
-            for (int t = t0; t < min(rows, t0 + WARP_TOKENS); ++t) {
-                float s = 0.0f;
-                if (n < p.N)
-                    for (int k = k_lo; k < k_hi; ++k) s = fmaf(p.A[(size_t)(m0 + t) * p.K + k], p.W[(size_t)n * p.K + k], s);
-                sums[t * FEATURES + feature] = s;
-            }
+            if (rows > 64) redo_tile<10>(p.A + (size_t)m0 * p.K, p.W + (size_t)n0 * p.K, p.K, rows, p.N - n0, k_lo, k_hi, smem);
+            else redo_tile<4>(p.A + (size_t)m0 * p.K, p.W + (size_t)n0 * p.K, p.K, rows, p.N - n0, k_lo, k_hi, smem);
         } else {
 #pragma unroll
             for (int j = 0; j < WARP_TOKENS; ++j)

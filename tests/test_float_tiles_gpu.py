@@ -37,7 +37,8 @@ def test_float_contraction(ops, M, N, K, epi):  # noqa: F811
     assert bool(((got - want).abs() <= bound).all())
 
 
-@pytest.mark.parametrize("M,N,K", [(161, 1030, 516), (40, 128, 10240)])          # a tile's K in one block, and cut among eight
+# a tile's K in one block, cut among eight and among four; tiles of 96, 48 and 160 tokens, the last feature tile ragged
+@pytest.mark.parametrize("M,N,K", [(161, 1030, 516), (40, 128, 10240), (320, 1299, 2020)])
 def test_float_contraction_of_what_bf16_does_not_hold(ops, M, N, K):  # noqa: F811
     """Infinities, NaN, values that round to infinity in bf16 and sums beyond the floats, among ordinary rows, on the tensor cores."""
     assert ops.lib().llb_gemm_simt_scratch_bytes(0, 0, M, N, K) > 0
@@ -59,6 +60,27 @@ def test_float_contraction_of_what_bf16_does_not_hold(ops, M, N, K):  # noqa: F8
     assert bool((got[3][same_sign] == want[3][same_sign]).all())
     beyond = torch.isfinite(want[6]) & (want[6].abs() < 3.0e38) | torch.isnan(got[6]) | torch.isinf(got[6])
     assert bool(beyond.all())          # sums that pass the largest float on the way are infinite or NaN, as with FFMA
+
+
+def test_a_nan_does_not_make_a_float_contraction_slow(ops):  # noqa: F811
+    """The tiles whose sums are no finite number are done again in float arithmetic: 7 times the time of finite ones here, where FFMA
+    throughout is 4 (every thread from memory by itself: 450)."""
+    a, w, out = rnd((389, 896), torch.float32, 23), rnd((9728, 896), torch.float32, 24, 0.02), torch.empty((389, 9728), device=dev())
+
+    def best():
+        times = []
+        for _ in range(5):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            for _ in range(4):
+                ops.gemm_simt(a, w, None, ops.EPI_STORE, out)
+            end.record()
+            end.synchronize()
+            times.append(begin.elapsed_time(end))
+        return min(times)
+    finite = best()
+    a[:, 5] = float("nan")
+    assert best() < 10 * finite and bool(torch.isnan(out).all())
 
 
 @pytest.mark.parametrize("M,N,K", [(161, 1030, 516), (40, 128, 10240)])
