@@ -260,9 +260,38 @@ def test_gemm_decode_clusters(ops, M, N, K, epi, split_k):
     assert bool(((got.double().cpu() - want).abs() <= bound).all())
 
 
+# more tiles of features than half the multiprocessors: two blocks a tile, with the rings of 16, 32 and 64 rows; 75 tiles (the last
+# ragged), 148, and one more than that; three blocks of 64 along K stay with one block
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("N,K", [(9500, 256), (18944, 328), (18946, 256), (9600, 192)])
+@pytest.mark.parametrize("epi", ["store", "relu", "residual", "swiglu"])
+def test_gemm_decode_two_blocks_a_tile(ops, M, N, K, epi):
+    w, bias, a = rnd((N, K), torch.bfloat16, 77, 0.2), rnd((N,), torch.float32, 78), rnd((M, K), torch.bfloat16, 79, 2.0)
+    y = a.double() @ w.double().t() + bias.double()
+    if epi == "residual":
+        res = rnd((M, N), torch.float32, 73)
+        got = res.clone()
+        ops.gemm_decode(w, ops.DEPI_RESIDUAL, M, a=a, bias=bias, residual=got, split_k=0)
+        want = y + res.double()
+    elif epi == "swiglu":
+        got = torch.full((M, N // 2), float("nan"), dtype=torch.bfloat16, device=dev())
+        ops.gemm_decode_glu(w, a, bias, got, 0, None)
+        want = y[:, 0::2] * torch.sigmoid(y[:, 0::2]) * y[:, 1::2]
+    else:
+        got = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=dev())
+        ops.gemm_decode_store(w, a, bias, got, (ops.ACT_SQUARED_RELU, 0.0, 0.0, 0.0) if epi == "relu" else None, 0)
+        want = y.clamp(min=0.0) ** 2 if epi == "relu" else y
+    ops.check_async_errors(dev())
+    # float sums (errors as in test_gemm_decode_clusters, taken at their largest), then bf16 but for the residual
+    size = float((a.double().abs() @ w.double().abs().t()).max()) + float(bias.abs().max()) + 4.0
+    error = (K + 8) * 2.0 ** -24 * size * {"store": 1.0, "residual": 1.0}.get(epi, 3.0 * size)
+    assert bool(((got.double() - want).abs() <= error + (0.0 if epi == "residual" else 2.0 ** -8) * want.abs()).all())
+
+
 @pytest.mark.parametrize("M", [2, 17, 64])
 @pytest.mark.parametrize("split_k", [0, 3, 8])
-@pytest.mark.parametrize("hd,rd,inter,Hq,Hkv,K", [(64, 64, False, 14, 2, 896), (128, 128, False, 4, 1, 520), (32, 16, True, 6, 3, 136)])
+@pytest.mark.parametrize("hd,rd,inter,Hq,Hkv,K", [(64, 64, False, 14, 2, 896), (128, 128, False, 4, 1, 520), (32, 16, True, 6, 3, 136),
+                                                  (128, 128, False, 65, 5, 264)])          # 75 tiles of features: two blocks each
 def test_gemm_decode_rope_clusters(ops, M, split_k, hd, rd, inter, Hq, Hkv, K):
     """The rotary epilogue behind parts of K: the same as from one block alone, up to the order of the sums."""
     N = (Hq + 2 * Hkv) * hd
