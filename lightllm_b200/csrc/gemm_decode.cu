@@ -510,6 +510,12 @@ int cached_map(const void* ptr, long long rows, long long cols, int box, CUtenso
 // Operand tiles, and behind them room for what a cluster's blocks send (a block alone uses the ring, which is idle by then).
 size_t tile_bytes(int BN, int stages, int b_tiles) { return (size_t)stages * A_BYTES + (size_t)b_tiles * BN * TILE_K * 2; }
 size_t recv_bytes(int BN, int cluster) { return cluster > 1 ? (size_t)cluster * llb_ceil_div(BN, cluster) * TILE_M * 4 : 0; }
+// The most that any cluster takes: not always the largest (16 tokens: three slots in each of 7 blocks, two in each of 8).
+size_t recv_bytes_most(int BN) {
+    size_t most = 0;
+    for (int c = 2; c <= MAX_CLUSTER; ++c) most = recv_bytes(BN, c) > most ? recv_bytes(BN, c) : most;
+    return most;
+}
 constexpr size_t SMEM_LIMIT = 224 * 1024;
 
 // How many clusters of `size` blocks of this kernel the device holds at once (asked once a kernel, size and device).
@@ -613,7 +619,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const DecodeGemmParams&
         const int most = split_k > 0 ? split_k : tiles < sms ? sms / tiles : 1;
         cluster = even(most < p.num_kb ? most : p.num_kb);
         if (cluster > MAX_CLUSTER) cluster = even(MAX_CLUSTER);
-        const size_t room = tile_bytes(BN, RING, NORM ? p.num_kb : RING) + recv_bytes(BN, MAX_CLUSTER) + 1024;
+        const size_t room = tile_bytes(BN, RING, NORM ? p.num_kb : RING) + recv_bytes_most(BN) + 1024;
         if (cluster > 1 && room > SMEM_LIMIT) cluster = 1;          // (a normed operand that is resident over a long K)
         if (cluster > 1) {
             const int rc = configure<BN, EPI, NORM, RING>(room);

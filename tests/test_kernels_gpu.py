@@ -288,6 +288,21 @@ def test_gemm_decode_two_blocks_a_tile(ops, M, N, K, epi):
     assert bool(((got.double() - want).abs() <= error + (0.0 if epi == "residual" else 2.0 ** -8) * want.abs()).all())
 
 
+# the longest K whose normed operand lies in shared memory beside the sums of a cluster of 8, and the next, at 16, 32 and 64 rows
+@pytest.mark.parametrize("M,K", [(16, 2752), (16, 2816), (32, 1216), (32, 1280), (64, 640), (64, 704)])
+@pytest.mark.parametrize("split_k", [5, 6, 7, 8])
+def test_gemm_decode_normed_over_the_longest_k(ops, M, K, split_k):
+    N = 256
+    w, x, nw = rnd((N, K), torch.bfloat16, 74, 0.2), rnd((M, K), torch.float32, 75, 2.0), 1 + 0.1 * rnd((K,), torch.float32, 76)
+    assert ops.gemm_decode_supports(M, N, K, True, ops.DEPI_SWIGLU)
+    out = torch.full((M, N // 2), float("nan"), dtype=torch.bfloat16, device=dev())
+    ops.gemm_decode(w, ops.DEPI_SWIGLU, M, x=x, norm_weight=nw, eps=1e-5, out=out, split_k=split_k)
+    ops.check_async_errors(dev())
+    ref = gemm_reference(plain_rmsnorm(x.cpu(), nw.cpu(), 1e-5).to(torch.bfloat16), w, None, 3, None)
+    # (the operand's bf16 may be rounded the other way: 2^-9 of a product each, as in test_gemm_decode)
+    assert torch.allclose(out.double().cpu(), ref, atol=2e-2 * max(1.0, float(ref.abs().max())), rtol=0)
+
+
 @pytest.mark.parametrize("M", [2, 17, 64])
 @pytest.mark.parametrize("split_k", [0, 3, 8])
 @pytest.mark.parametrize("hd,rd,inter,Hq,Hkv,K", [(64, 64, False, 14, 2, 896), (128, 128, False, 4, 1, 520), (32, 16, True, 6, 3, 136),
