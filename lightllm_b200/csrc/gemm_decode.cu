@@ -546,16 +546,19 @@ int clusters_at_once(int size, size_t smem) {
     return n;
 }
 
+// The kernel's limit on shared memory, one figure whatever a launch takes: threads that come here at the same time set the same, and
+// none lowers what another's launch needs.
 template <int BN, int EPI, bool NORM, int STAGES>
-int configure(size_t smem) {
-    static std::atomic<size_t> configured[64] = {};
+int configure() {
+    static std::atomic<bool> configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     const bool cached = dev >= 0 && dev < 64;
-    if (cached && configured[dev].load() >= smem) return 0;
-    const cudaError_t e = cudaFuncSetAttribute(gemm_decode_kernel<BN, EPI, NORM, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return llb_fail("gemm_decode: cannot opt in to %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    if (cached) configured[dev].store(smem);
+    if (cached && configured[dev].load()) return 0;
+    const size_t room = tile_bytes(BN, STAGES, STAGES) + recv_bytes_most(BN) + 1024, most = NORM || room > SMEM_LIMIT ? SMEM_LIMIT : room;
+    const cudaError_t e = cudaFuncSetAttribute(gemm_decode_kernel<BN, EPI, NORM, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e != cudaSuccess) return llb_fail("gemm_decode: cannot opt in to %zu bytes of shared memory: %s", most, cudaGetErrorString(e));
+    if (cached) configured[dev].store(true);
     return 0;
 }
 
@@ -564,7 +567,7 @@ int launch_stages(const CUtensorMap& mw, const CUtensorMap& mx, DecodeGemmParams
     const int b_tiles = NORM ? p.num_kb : STAGES;
     const size_t tiles = tile_bytes(BN, STAGES, b_tiles), smem = tiles + recv_bytes(BN, cluster) + 1024;
     LLB_REQUIRE(smem <= SMEM_LIMIT, "gemm_decode: K=%d with %d rows needs %zu bytes of shared memory", p.K, BN, smem);
-    int rc = configure<BN, EPI, NORM, STAGES>(smem);
+    int rc = configure<BN, EPI, NORM, STAGES>();
     if (rc) return rc;
     p.kb_per_split = llb_ceil_div(p.num_kb, cluster * pieces);
     p.cluster = cluster;
@@ -622,7 +625,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const DecodeGemmParams&
         const size_t room = tile_bytes(BN, RING, NORM ? p.num_kb : RING) + recv_bytes_most(BN) + 1024;
         if (cluster > 1 && room > SMEM_LIMIT) cluster = 1;          // (a normed operand that is resident over a long K)
         if (cluster > 1) {
-            const int rc = configure<BN, EPI, NORM, RING>(room);
+            const int rc = configure<BN, EPI, NORM, RING>();
             if (rc) return rc;
             while (split_k == 0 && cluster > 1 && clusters_at_once<BN, EPI, NORM, RING>(cluster, room) < tiles) cluster = even(cluster - 1);
             // several clusters along K add into the residual
@@ -636,12 +639,8 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const DecodeGemmParams&
     if constexpr (!NORM && EPI != DEPI_STORE_F32) {
         // more tiles than half the multiprocessors: two blocks a tile, and two of them on a multiprocessor
         constexpr int PAIR = BN == 16 ? 5 : BN == 32 ? 4 : 3;
-        constexpr size_t room = (size_t)PAIR * (A_BYTES + BN * TILE_K * 2) + BN * TILE_M * 4 + 1024;
-        if (split_k == 0 && may_cut && pieces == 1 && tiles <= sms && p.num_kb >= 4) {
-            const int rc = configure<BN, EPI, NORM, PAIR>(room);
-            if (rc) return rc;
+        if (split_k == 0 && may_cut && pieces == 1 && tiles <= sms && p.num_kb >= 4)
             return launch_stages<BN, EPI, NORM, PAIR>(mw, mx, p, 2, 1, stream);
-        }
     }
     // the float-store epilogue is the head's: a vocabulary's worth of blocks
     if constexpr (EPI == DEPI_STORE_F32 && !NORM)

@@ -1,6 +1,9 @@
 """Each kernel alone against a plain PyTorch float32 reference of the same op, at sizes other
 than the engine's."""
 import math
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -301,6 +304,41 @@ def test_gemm_decode_normed_over_the_longest_k(ops, M, K, split_k):
     ref = gemm_reference(plain_rmsnorm(x.cpu(), nw.cpu(), 1e-5).to(torch.bfloat16), w, None, 3, None)
     # (the operand's bf16 may be rounded the other way: 2^-9 of a product each, as in test_gemm_decode)
     assert torch.allclose(out.double().cpu(), ref, atol=2e-2 * max(1.0, float(ref.abs().max())), rtol=0)
+
+
+def test_gemm_decode_first_called_by_many_threads_at_once():
+    """Threads that are the first to call a kernel, some with more shared memory than others (blocks alone, clusters of each size)."""
+    code = """
+import threading, torch
+from lightllm_b200.csrc import ops
+torch.cuda.set_device(0)
+dev = torch.device("cuda:0")
+ops.lib(), ops.async_error_flag(dev)
+w = [(torch.arange(256 * 512, device=dev).reshape(256, 512) % 7 - 3).to(torch.bfloat16) for _ in range(8)]
+a = [(torch.arange(m * 512, device=dev).reshape(m, 512) % 5 - 2).to(torch.bfloat16) for m in (16, 32, 64)]
+want = [x.double() @ w[0].double().t() for x in a]
+torch.cuda.synchronize()
+start, bad = threading.Barrier(8), []
+def work(i):
+    try:
+        torch.cuda.set_device(0)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for x, y in zip(a, want):
+                out = torch.empty(x.shape[0], 256, dtype=torch.bfloat16, device=dev)
+                start.wait()
+                ops.gemm_decode_store(w[i], x, None, out, None, i + 1)
+                torch.cuda.current_stream().synchronize()
+                if not torch.equal(out, y.to(torch.bfloat16)): bad.append((i, x.shape[0]))
+    except BaseException as e:
+        bad.append((i, repr(e))); start.abort()
+threads = [threading.Thread(target=work, args=(i,)) for i in range(8)]
+[t.start() for t in threads]; [t.join() for t in threads]
+ops.check_async_errors(dev)
+assert not bad, bad
+"""
+    for _ in range(3):
+        done = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=120)
+        assert done.returncode == 0, done.stderr[-2000:]
 
 
 @pytest.mark.parametrize("M", [2, 17, 64])
