@@ -163,6 +163,7 @@ class StepContext:
         self.page_size = 0
         self.decode_only = False
         self.fresh_positions = 0                # of a row: the last positions that this step may write (0: not known)
+        self.captured = False                   # the step's launches are recorded into a graph, not run one by one
         self.rowwise = False                    # a mixed step described row by row: several spans may be one request's
         self.select_rows: Optional[torch.Tensor] = None   # row by row: the wanted rows, picked from the logits of all rows
         self.rows_given = 0                     # the tokens that the entries brought (T counts a row-by-row step's padding)

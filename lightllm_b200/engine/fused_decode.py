@@ -23,14 +23,24 @@ from ..parts.norm import RMSNorm
 from ..parts.rotary import NoPositionEncoding, RotaryEmbedding
 
 MAX_ROWS = 64          # what the kernel takes
-# Where the persistent kernel is faster than the layers launched kernel by kernel (each kernel set up while the one before it runs):
-# layers of a few megabytes of weights, of which nothing but the chain of stages is left, under two rows and more.  Measured on
-# B200, ms a step of 24 layers, persistent / kernel by kernel: width 256 (2 MB a layer) 0.56 / 0.50 at one row, 0.55 / 0.61 at four,
-# 0.69 / 0.81 at 32; width 512 (6 MB) 0.61 / 0.55, 0.58 / 0.58, 0.72 / 0.74; width 768 (15 MB) 0.64 / 0.59, 0.62 / 0.67, 0.88 / 0.85, eight
-# rows 0.71 / 0.68; the 0.5B sizes (30 MB) 0.73 / 0.67, 0.73 / 0.72, 0.97 / 0.95; the 1.5B sizes (93 MB, 28 layers) 1.36 / 1.20, 1.38 / 1.23, 2.10 / 1.56.
+# Where the persistent kernel is faster than the layers launched kernel by kernel (each kernel set up while the one before it runs).
+# Measured on B200 over contexts of 1,024, us a step of 24 layers (the last: 28), persistent / kernel by kernel; MB: weights of a layer.
+#   replayed from a graph                       1 row        2            4            8            16           32
+#     width 256 (2.6 MB)                     564 / 515    546 / 531    541 / 545    559 / 558    617 / 613    701 / 772
+#     width 384 (5.5 MB)                     587 / 508    566 / 522    558 / 539    576 / 567    641 / 637    726 / 739
+#     width 512 (10 MB)                      613 / 526    589 / 550    589 / 568    611 / 600    678 / 631    773 / 773
+#     width 768 (22 MB)                      657 / 595    646 / 616    650 / 631    673 / 644    747 / 689    883 / 833
+#   launched one by one, the host's time
+#     width 256                              709 / 694    700 / 721    697 / 751    722 / 790    794 / 845    910 / 1,076
+#     width 768                              801 / 818    799 / 855    806 / 869    835 / 908    953 / 957  1,100 / 1,137
+#     0.5B sizes (30 MB)                     836 / 833    835 / 856    842 / 875    874 / 917    971 / 984  1,160 / 1,191
+#     1.5B sizes (93 MB)                   1,464 / 1,305  1,453 / 1,345  1,450 / 1,361  1,522 / 1,423  1,751 / 1,519  2,217 / 1,782
+# A step of a shape that comes for the first time is launched one by one, and there five launches are less for the host than 170, until
+# the layers' bytes count.
 DEFAULT_ROWS = 32
-MIN_ROWS = 2
-MAX_LAYER_BYTES = 8 << 20
+GRAPH_MIN_ROWS = 2
+GRAPH_LAYER_BYTES = 8 << 20
+MAX_LAYER_BYTES = 32 << 20
 
 
 def _layer_facts(block, view):
@@ -73,6 +83,7 @@ class Segment:
         self.position = position
         self.descriptors = ops.decode_layers_descriptors(layers, self.D, self.Hq, self.Hkv, self.hd, self.I, device)
         self.keep = layers                   # the descriptors hold addresses of these tensors
+        self.layer_bytes = max(FusedDecode._layer_bytes(t) for t in layers)
         self.counters = ops.decode_layers_counters(device)
         self.scratch: Optional[torch.Tensor] = None
 
@@ -125,8 +136,10 @@ class FusedDecode:
     def takes(self, ctx) -> bool:
         # (one row a request: the kernel's attention stage makes a row's new key and value itself, beside the rows that
         # read the cache, so the rows of a step described row by row, which share requests, go kernel by kernel)
-        return (self.enabled and ctx.decode_only and not ctx.rowwise and MIN_ROWS <= ctx.T <= self.max_rows
-                and len(ctx.block_tables) <= ops.MAX_FUSED_GROUPS)
+        return (self.enabled and ctx.decode_only and not ctx.rowwise and ctx.T <= self.max_rows
+                and (not ctx.captured or ctx.T >= GRAPH_MIN_ROWS) and len(ctx.block_tables) <= ops.MAX_FUSED_GROUPS)
 
-    def segment_at(self, run_index: int) -> Optional[Segment]:
-        return self.segments[run_index]
+    def segment_at(self, run_index: int, captured: bool = False) -> Optional[Segment]:
+        """The segment that begins at this run entry, if the kernel is to run it in such a step (``captured``: recorded into a graph)."""
+        segment = self.segments[run_index]
+        return None if segment is None or (captured and segment.layer_bytes > GRAPH_LAYER_BYTES) else segment

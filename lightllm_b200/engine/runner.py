@@ -316,7 +316,7 @@ class ModelRunner:
         while i < len(m.run):
             if enters[i] is not None:          # a part that rewrites the stream before this run of the layer
                 enters[i].forward(residual, ctx)
-            segment = fused.segment_at(i) if fused is not None else None
+            segment = fused.segment_at(i, ctx.captured) if fused is not None else None
             if self._nvtx:
                 torch.cuda.nvtx.range_push(f"run{i}:" + (f"fused to {segment.end}" if segment else f"layer{m.run[i].layer}"))
             if segment is not None:
@@ -326,7 +326,7 @@ class ModelRunner:
                 j = self.native.stretch(i)
                 j = next((k for k in range(i + 1, j) if enters[k] is not None), j)
                 if fused is not None:           # up to where the next fused segment begins
-                    j = next((k for k in range(i + 1, j) if fused.segment_at(k) is not None), j)
+                    j = next((k for k in range(i + 1, j) if fused.segment_at(k, ctx.captured) is not None), j)
                 self.native.run(residual, ctx, i, j)
                 i = j
             else:
@@ -365,6 +365,7 @@ class ModelRunner:
         cached block of device and pinned memory, about 6 ms, after which the next allocations go to the driver again):
         a server captures dozens of shapes while it runs, and none of them needs the memory that those give back."""
         graph = torch.cuda.CUDAGraph()
+        ctx.captured = True
         current = ops.torch_stream()
         if self._capture_stream is None:
             self._capture_stream = torch.cuda.Stream(self.device)

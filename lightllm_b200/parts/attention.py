@@ -279,16 +279,18 @@ class AttentionMixer(Mixer):
         if n < 2 or n > ops.DECODE_EVEN_MAX:
             return nsplit
         window = self.kernel_window()
-        starts = np.fromiter((ctx.spans[i].start for i in which), dtype=np.int64, count=n)
-        keys = starts + 1
+        keep = self.keep_first
+        # (plain numbers: arrays of a few requests cost the host more than the sums)
         if window > 0:
-            keys = np.minimum(keys, window + self.keep_first)
+            keys = [min(ctx.spans[i].start + 1, window + keep) for i in which]
         elif window < 0:
-            keys = np.minimum(keys, starts % -window + 1 + self.keep_first)
+            keys = [min(ctx.spans[i].start + 1, ctx.spans[i].start % -window + 1 + keep) for i in which]
+        else:
+            keys = [ctx.spans[i].start + 1 for i in which]
         resident = ops.decode_mma_resident(self.head_dim) * L.num_sms(ctx.device) // (self.num_kv_heads * self.value_cross)
         pieces = max(n, min(resident, n + 128))
-        even = max(64, -(-int(keys.sum()) // pieces))
-        if -(-int(keys.max()) // nsplit) < even + EVEN_GAIN_KEYS[self.head_dim]:
+        even = max(64, -(-sum(keys) // pieces))
+        if -(-max(keys) // nsplit) < even + EVEN_GAIN_KEYS[self.head_dim]:
             return nsplit
         ctx.shape_key.append(("even", pieces))
         return -pieces

@@ -453,6 +453,34 @@ def test_small_mixed_steps_described_row_by_row(tmp_path, monkeypatch, name, dty
     assert worst <= tol, worst
 
 
+@pytest.mark.parametrize("limit,rows,want", [(0, 4, [True, False, False]), (1 << 30, 4, [True, True, False])])
+def test_new_shapes_take_the_persistent_kernel_and_graphs_what_is_faster(tmp_path, monkeypatch, limit, rows, want):
+    """A decode shape's first step is launched one by one, through the persistent kernel; its graph holds it for small layers
+    only; a replay launches nothing.  All of them follow the plain implementation."""
+    from lightllm_b200.engine import fused_decode
+    monkeypatch.setattr(fused_decode, "GRAPH_LAYER_BYTES", limit, raising=False)
+    d = model_dir(tmp_path, "E", seed=35, store="bfloat16", edit=sharpen(3.0))
+    cfg, w = P.read_model_dir(d)
+    rng = random.Random(36)
+    seqs = {i: [rng.randrange(cfg["vocab_size"]) for _ in range(50)] for i in range(rows)}
+    ref = {i: P.plain_forward(cfg, w, s) for i, s in seqs.items()}
+    core = core_for(d, "bfloat16", pages=32)
+    ran, run = [], fused_decode.Segment.run
+    monkeypatch.setattr(fused_decode.Segment, "run", lambda self, residual, ctx: (ran.append(1), run(self, residual, ctx))[1])
+    for i in seqs:
+        core.open(i)
+    core.step([StepEntry(i, s[:40], []) for i, s in seqs.items()])
+    seen, worst = [], 0.0
+    for k in range(40, 44):
+        ran.clear()
+        out = core.step([StepEntry(i, [s[k]], [0]) for i, s in seqs.items()])
+        seen.append(bool(ran))
+        worst = max(worst, max(float((out[i].float().cpu() - ref[i][k]).abs().max()) for i in seqs))
+    core.runner.check_device_errors()
+    assert seen == want + [False]
+    assert worst <= atol_for("E sharp", "bfloat16", ref), worst
+
+
 @pytest.mark.parametrize("fused", ["0", "1"])
 @pytest.mark.parametrize("name", ["D", "E"])
 def test_a_step_row_by_row_after_decoding_batches_of_as_many_rows(tmp_path, monkeypatch, name, fused):
