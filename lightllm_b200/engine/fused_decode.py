@@ -35,11 +35,12 @@ MAX_ROWS = 64          # what the kernel takes
 #     width 768                              801 / 818    799 / 855    806 / 869    835 / 908    953 / 957  1,100 / 1,137
 #     0.5B sizes (30 MB)                     836 / 833    835 / 856    842 / 875    874 / 917    971 / 984  1,160 / 1,191
 #     1.5B sizes (93 MB)                   1,464 / 1,305  1,453 / 1,345  1,450 / 1,361  1,522 / 1,423  1,751 / 1,519  2,217 / 1,782
-# A step of a shape that comes for the first time is launched one by one, and there five launches are less for the host than 170, until
-# the layers' bytes count.
+# From a graph what is left is the chain of stages, where the persistent kernel is ahead for the smallest layers only (12 rows 574 / 604, 24
+# 655 / 702 at width 256; 688 / 672 at 384).  A step of a shape that comes for the first time is launched one by one, and there five
+# launches are less for the host than 170, until the layers' bytes count.
 DEFAULT_ROWS = 32
-GRAPH_MIN_ROWS = 2
-GRAPH_LAYER_BYTES = 8 << 20
+GRAPH_MIN_ROWS = 3
+GRAPH_LAYER_BYTES = 4 << 20
 MAX_LAYER_BYTES = 32 << 20
 
 

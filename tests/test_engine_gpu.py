@@ -453,10 +453,11 @@ def test_small_mixed_steps_described_row_by_row(tmp_path, monkeypatch, name, dty
     assert worst <= tol, worst
 
 
-@pytest.mark.parametrize("limit,rows,want", [(0, 4, [True, False, False]), (1 << 30, 4, [True, True, False])])
+@pytest.mark.parametrize("limit,rows,want", [(0, 4, [True, False, False]), (0, 2, [True, False, False]), (1 << 30, 4, [True, True, False]),
+                                             (1 << 30, 2, [True, False, False])])
 def test_new_shapes_take_the_persistent_kernel_and_graphs_what_is_faster(tmp_path, monkeypatch, limit, rows, want):
-    """A decode shape's first step is launched one by one, through the persistent kernel; its graph holds it for small layers
-    only; a replay launches nothing.  All of them follow the plain implementation."""
+    """A decode shape's first step is launched one by one, through the persistent kernel; its graph holds it for small layers and from
+    three rows on only; a replay launches nothing.  All of them follow the plain implementation."""
     from lightllm_b200.engine import fused_decode
     monkeypatch.setattr(fused_decode, "GRAPH_LAYER_BYTES", limit, raising=False)
     d = model_dir(tmp_path, "E", seed=35, store="bfloat16", edit=sharpen(3.0))
