@@ -56,7 +56,7 @@ namespace {
 
 constexpr int F32 = 0, BF16 = 1;                 // the library's dtype codes
 constexpr int PAGE = 16;                         // tokens of a cache page
-constexpr int EXPECTED_ABI = 25;
+constexpr int EXPECTED_ABI = 26;
 constexpr int CLUSTER_MERGE_MAX_KEYS = 8192;     // up to here the decode attention merges its pieces inside a cluster
 
 [[noreturn]] void die(const std::string& what) {
