@@ -1,6 +1,7 @@
 // Error reporting shared by every exported function of the library.
 #include "common.cuh"
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 
@@ -13,6 +14,18 @@ int llb_fail(const char* fmt, ...) {
     vsnprintf(g_last_error, sizeof(g_last_error), fmt, ap);
     va_end(ap);
     return -1;
+}
+
+int llb_device_sms() {
+    static std::atomic<int> known[64] = {};
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64) sms = known[dev].load();
+    if (sms == 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return 1;
+        if (dev >= 0 && dev < 64) known[dev].store(sms);
+    }
+    return sms;
 }
 
 int llb_check_launch(const char* what) {

@@ -24,6 +24,7 @@ enum LlbEpilogue {
 
 int llb_fail(const char* fmt, ...);          // stores the message, returns -1
 int llb_check_launch(const char* what);      // cudaGetLastError() -> 0 or llb_fail
+int llb_device_sms();                        // multiprocessors of the current device (asked once a device; 1 if it does not say)
 
 #define LLB_REQUIRE(cond, ...)                 \
     do {                                       \

@@ -591,18 +591,6 @@ int launch_stages(const CUtensorMap& mw, const CUtensorMap& mx, DecodeGemmParams
     return llb_check_launch("gemm_decode");
 }
 
-int device_sms() {
-    static std::atomic<int> known[64] = {};
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64) sms = known[dev].load();
-    if (sms == 0) {
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return 1;
-        if (dev >= 0 && dev < 64) known[dev].store(sms);
-    }
-    return sms;
-}
-
 // K in `pieces` x `cluster` parts.  Asked for a number of parts: clusters of up to 8 of them.  Asked to choose (split_k = 0): the tiles
 // of features alone leave most multiprocessors idle where there are few of them, and a block's part of K then is its time, so the
 // largest clusters that all find a place at once; tiles that fill more than half of the multiprocessors get two blocks each with short
@@ -612,7 +600,7 @@ int device_sms() {
 template <int BN, int EPI, bool NORM>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const DecodeGemmParams& p, int split_k, cudaStream_t stream) {
     constexpr int RING = BN == 64 ? MIDDLE : DEEP;          // beside the received sums
-    const int tiles = llb_ceil_div(p.N, TILE_M), sms = device_sms();
+    const int tiles = llb_ceil_div(p.N, TILE_M), sms = llb_device_sms();
     const bool may_cut = EPI != DEPI_STORE_F32 && !(EPI == DEPI_SWIGLU && p.N % 2);
     int cluster = 1, pieces = 1;
     auto even = [&](int parts) { return llb_ceil_div(p.num_kb, llb_ceil_div(p.num_kb, parts)); };          // without empty parts

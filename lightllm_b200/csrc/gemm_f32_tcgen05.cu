@@ -434,18 +434,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const __gr
     }
 }
 
-int device_sms() {
-    static std::atomic<int> known[64] = {};
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64) sms = known[dev].load();
-    if (sms == 0) {
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return 1;
-        if (dev >= 0 && dev < 64) known[dev].store(sms);
-    }
-    return sms;
-}
-
 // A map over the planes [rows, cols] of bf16 with boxes of box_rows x 32 and the 64-byte swizzle.
 int make_planes_map(const void* ptr, long long rows, long long cols, int box_rows, CUtensorMap* out) {
     EncodeTiledFn fn = encode_tiled_fn();
@@ -479,7 +467,7 @@ int launch(const F32Params& p0, __nv_bfloat16* planes, cudaStream_t stream) {
     p.tokens = llb_ceil_div(even, 16) * 16;
     const int mt = llb_ceil_div(p.M, p.tokens), nt = llb_ceil_div(p.N, FEATURES), slices = llb_ceil_div(p.K, SLICE);
     int split = 1;
-    while (split < 8 && (long long)mt * nt * split * 2 <= device_sms() * (split < 4 ? 9 : 8) / 10 && slices >= split * 6) split *= 2;
+    while (split < 8 && (long long)mt * nt * split * 2 <= llb_device_sms() * (split < 4 ? 9 : 8) / 10 && slices >= split * 6) split *= 2;
     const int per = llb_ceil_div(slices, split);
     split = llb_ceil_div(slices, per);
     p.k_part = per * SLICE;

@@ -324,23 +324,10 @@ __global__ void __launch_bounds__(F_THREADS, 2) gemm_f32_kernel(const float* __r
     if (parts > 1) cg::this_cluster().sync();          // the others may still read this block's sums
 }
 
-// Multiprocessors of the current device.
-int device_sms() {
-    static std::atomic<int> known[64] = {};
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64) sms = known[dev].load();
-    if (sms == 0) {
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return 1;
-        if (dev >= 0 && dev < 64) known[dev].store(sms);
-    }
-    return sms;
-}
-
 // Into how many pieces K is cut: two blocks are resident on a multiprocessor, and the tiles shall fill them once; no piece
 // below four slices.  The order of a row's sum depends on it, and so its last bits depend on how many rows are beside it.
 int f32_split(int tiles, int slices) {
-    int split = 2 * device_sms() / tiles;
+    int split = 2 * llb_device_sms() / tiles;
     split = split > slices / 4 ? slices / 4 : split;
     return split < 1 ? 1 : split > F_MAX_SPLIT ? F_MAX_SPLIT : split;
 }
@@ -352,7 +339,7 @@ int f32_split(int tiles, int slices) {
 // 256 5.0 us, streaming 3.9 to 5.0; 2,048 x 128 4.1 / 3.3 to 4.1; 4,096 x 256 at five rows 5.2 / 4.7), and a longer K that is not cut
 // because every multiprocessor has a tile but few have two (9,728 x 896 23.6 / 17 to 21 at up to seven rows, 10,624 x 4,096 98 / 70 to 83).
 bool f32_streamed(int M, int N, int K) {
-    const int nt = llb_ceil_div(N, F_BN), slices = llb_ceil_div(K, F_BK), sms = device_sms();
+    const int nt = llb_ceil_div(N, F_BN), slices = llb_ceil_div(K, F_BK), sms = llb_device_sms();
     if (M <= 4 || M > 8) return M <= 4;
     if (slices <= 8) return slices >= 3 && (long long)nt * M <= 320;
     return slices >= 16 && nt > sms && nt <= sms * 6 / 5 && nt * M <= 8 * sms;

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(512) rmsnorm_block_kernel(const float* __restr
 // A warp per row leaves most multiprocessors without a row until there are about as many rows as multiprocessors; beyond, both are alike.
 // us a launch in a chain of them, warps / block: 896 wide 27 rows 1.66 / 1.31, 100 1.74 / 1.42, 148 1.75 / 1.75; 1,536 wide 27 rows 2.14 /
 // 1.35, 148 2.24 / 2.23.  Wider rows always take a block (3,584 wide, single floats a thread before: 8 rows 2.24 -> 1.55, 2,048 9.6 -> 7.5).
-static bool norm_by_warps(int R, int D) { return D <= 128 * 16 && R >= 148; }
+static bool norm_by_warps(int R, int D) { return D <= 128 * 16 && R >= llb_device_sms(); }
 
 template <typename TI, typename TW, typename TO>
 static int launch_rmsnorm(const void* x, const void* w, void* out, const int* rows, int R, int D, float eps,
