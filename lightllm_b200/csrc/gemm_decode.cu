@@ -195,8 +195,6 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* a_tiles = smem;                             // STAGES weight tiles
     uint8_t* b_tiles = smem + STAGES * A_BYTES;          // NORM: num_kb resident tiles; else STAGES tiles
-    const int b_count = NORM ? p.num_kb : STAGES;
-    (void)b_count;
     float* recv = (float*)(smem + p.recv_offset);        // [cluster][slots][128]: this block's tokens' sums, from every block
     volatile int* abort_flag = &abort_s;
 

@@ -1108,28 +1108,6 @@ def rope_table(positions: torch.Tensor, inv_freq: torch.Tensor, transposed: bool
     return out
 
 
-_splitk = {}
-_splitk_retired = []     # meeting places that a larger one replaced: CUDA graphs captured earlier still use them
-
-
-def reserve_splitk_scratch(device: torch.device, floats: int, tiles: int) -> None:
-    """A zeroed place of ``floats`` floats and ``tiles`` counters on the device (a larger one replaces a smaller, which is kept
-    alive).  The contractions of this library need none: their parts along K meet in shared memory."""
-    key = torch.device(device).index or 0
-    have = _splitk.get(key)
-    if have is None or have[0].numel() < floats or have[1].numel() < tiles:
-        floats = max(floats, have[0].numel() if have else 0)
-        tiles = max(tiles, have[1].numel() if have else 0)
-        if have is not None:
-            _splitk_retired.append(have)
-        _splitk[key] = (torch.zeros(floats, dtype=torch.float32, device=device),
-                        torch.zeros(tiles, dtype=torch.int32, device=device))
-
-
-def splitk_scratch(device: torch.device):
-    return _splitk.get(torch.device(device).index or 0)
-
-
 def gemm_decode_supports(M: int, N: int, K: int, norm: bool, epilogue: int, head_dim: int = 0) -> bool:
     return bool(lib().llb_gemm_decode_supports(M, N, K, 1 if norm else 0, epilogue, head_dim))
 
