@@ -37,6 +37,28 @@ def test_float_contraction(ops, M, N, K, epi):  # noqa: F811
     assert bool(((got - want).abs() <= bound).all())
 
 
+def on_ffma(ops, a, w):  # noqa: F811
+    """The same contraction on CUDA cores: without scratch for the split tokens it stays there."""
+    (M, K), N, out = a.shape, w.shape[0], torch.empty((a.shape[0], w.shape[0]), device=dev())
+    ops._check(ops.lib().llb_gemm_simt(a.data_ptr(), 0, w.data_ptr(), 0, 0, out.data_ptr(), 0, ops.EPI_STORE, M, N, K, 0, 0,
+                                       ops.async_error_flag(dev()).data_ptr(), ops.current_stream()))
+    return out
+
+
+@pytest.mark.parametrize("M,N,K", [s for s in SHAPES if s[0] > 16] + [(389, 9728, 896), (24, 9728, 896), (17, 6200, 4864), (40, 6200, 512), (389, 1500, 8960)])
+def test_float_contraction_is_no_further_off_than_ffma(ops, M, N, K):  # noqa: F811
+    """The relative 2-norm error against 64 bits, on the tensor cores beside FFMA (which is 1.1 to 3.6 times as far off).  Two parts an
+    operand instead of three, a plane in another's place or a product left out are 2.4e-6 and more off at every K, and one accumulation in
+    tensor memory over K = 896 8.6e-7."""
+    if ops.lib().llb_gemm_simt_scratch_bytes(0, 0, M, N, K) == 0:
+        pytest.skip("these sizes stay on CUDA cores")
+    a, w, out = rnd((M, K), torch.float32, 11), rnd((N, K), torch.float32, 12), torch.empty((M, N), device=dev())
+    ops.gemm_simt(a, w, None, ops.EPI_STORE, out)
+    want = a.double() @ w.double().t()
+    error, ffma = (float((x.double() - want).norm() / want.norm()) for x in (out, on_ffma(ops, a, w)))
+    assert error <= ffma and error < 3e-7, (error, ffma)
+
+
 # a tile's K in one block, cut among eight and among four; tiles of 96, 48 and 160 tokens, the last feature tile ragged
 @pytest.mark.parametrize("M,N,K", [(161, 1030, 516), (40, 128, 10240), (320, 1299, 2020)])
 def test_float_contraction_of_what_bf16_does_not_hold(ops, M, N, K):  # noqa: F811
