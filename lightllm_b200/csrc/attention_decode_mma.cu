@@ -230,7 +230,9 @@ __global__ void __launch_bounds__(NWARPS * 32) paged_decode_mma_kernel(DecodePar
         cp_async_commit();
     };
 
-    // Only the last positions are written in this step: tiles of keys from earlier steps are asked for before the kernel before has completed
+    // Only the last positions are written in this step: tiles of keys from earlier steps are asked for before the kernel before has completed.
+    // That earlier steps are complete when this block runs rests on the step's first launch, which waits before it signals (see
+    // LlbStepArgs::fresh)
     // (8 requests of 2,048 keys of 64, us a layer, with the merge by sending: 8.2 -> 7.4; 64 requests 18.0 -> 16.3).
     int early = 0;
 #pragma unroll

@@ -10,7 +10,7 @@ template <typename TW, typename TC>
 __global__ void embedding_kernel(const int* __restrict__ ids, const TW* __restrict__ table,
                                  float* __restrict__ out, int D, int V, int* __restrict__ err, float scale,
                                  TC* __restrict__ copy) {
-    llb_after_previous();
+    llb_after_previous();          // (a step's first launch: it has to wait before it signals, see LlbStepArgs::fresh)
     const int t = blockIdx.x;
     const int id = ids[t];
     const bool ok = id >= 0 && id < V;

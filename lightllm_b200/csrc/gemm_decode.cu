@@ -516,7 +516,8 @@ size_t recv_bytes_most(int BN) {
 }
 constexpr size_t SMEM_LIMIT = 224 * 1024;
 
-// How many clusters of `size` blocks of this kernel the device holds at once (asked once a kernel, size and device).
+// How many clusters of `size` blocks of this kernel the device holds at once (asked once a kernel, size and device: a normed operand's
+// shared memory grows with K, but with rings of six and eight stages a multiprocessor holds one block whatever K is).
 template <int BN, int EPI, bool NORM, int STAGES>
 int clusters_at_once(int size, size_t smem) {
     static std::atomic<int> known[64][MAX_CLUSTER + 1] = {};

@@ -2,7 +2,8 @@
 //
 // C[M,N] = A[M,K] * W[N,K]^T, W stored [out, in] as in the checkpoint (src/engine/engine_server.cpp:1542-1544; the reference
 // calls cublasSgemm, src/ops/gemm.cu:92-97).  The tensor cores multiply bf16 exactly but take no floats, and they cut off what
-// does not fit a float after every instruction instead of rounding it.  So
+// does not fit a float after every instruction instead of rounding it.  So (the splitting is a published method: G. Henry, P. T. P. Tang
+// and A. Heinecke, Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations, 2019)
 //   * every operand is the sum of three bf16 numbers, x = x1 + x2 + x3 (each rounded to nearest from what is left, which is
 //     exact for a float's 24 bits, see UP).  The weights are split on the way into shared memory, so no copy of them is kept; the
 //     tokens, which every tile of features reads, by a kernel before this one (split in every block they took most of its
@@ -11,7 +12,7 @@
 //     x1 w3, x3 w1 into a second one (the other three are below 2^-25 of the product);
 //   * the accumulator of x1 w1 is read, and begun anew, every 32 columns of K, and its values are added up in registers,
 //     rounded to nearest.  Left in tensor memory over all of K the cut-off bits add up: 8.6e-7 off 64 bits (2-norm) at K = 896
-//     where FFMA is 8.4e-8 off; the corrections are 2^-9 of the sum and may stay.
+//     where FFMA is 2.7e-7 off; the corrections are 2^-9 of the sum and may stay.
 // What does not fit that form (an infinity, a NaN, operands beyond 2^104, sums beyond 2^80) shows as a sum that is no finite
 // number; a block that sees one does its tile again with FFMA, so such inputs give what float arithmetic gives.
 //
@@ -21,9 +22,11 @@
 // meet in shared memory in the order of K.  Waits are bounded as in the other tensor-core kernels.
 //
 // Measured (us, FFMA tiles of csrc/gemm_simt.cu -> here, the split of the tokens included): 389 rows x 9,728 features x 896
-// 227 -> 58 (116 TFLOP/s), 389 x 896 x 4,864 158 -> 41, 389 x 151,936 x 896 3,110 -> 703 (150), 389 x 37,888 x 3,584 2,976 -> 611
-// (173), 160 x 9,728 x 896 115 -> 30.  2-norm error against 64 bits there 2.7e-7 -> 1.1e-7, 3.7e-7 -> 1.3e-7, 2.7e-7 -> 1.1e-7,
-// 5.4e-7 -> 2.1e-7, 2.7e-7 -> 1.1e-7.  What bounds it: a slice takes about 1,300 cycles at 32 tokens (each warp's chain of split, fence
+// 228 -> 60 (113 TFLOP/s), 389 x 896 x 4,864 160 -> 42, 389 x 151,936 x 896 3,230 -> 730 (145), 160 x 9,728 x 896 119 -> 31.  2-norm error
+// against 64 bits at 389 x 1,500 x K, FFMA -> here: K = 4 4.0e-8 -> 2.7e-8, 64 8.4e-8 -> 5.4e-8, 256 1.5e-7 -> 6.7e-8, 896 2.7e-7 -> 9.1e-8,
+// 4,864 6.3e-7 -> 1.7e-7; 17 x 6,200 x 896 1.7e-7 -> 9.1e-8.  Sums of numbers of one sign, whose result's own rounding is 2.5e-8, are
+// about even: K = 64 5.0e-8 -> 5.7e-8, 128 5.7e-8 -> 5.9e-8, 256 6.9e-8 -> 6.4e-8, 896 1.1e-7 -> 8.5e-8; 64 rows, K = 512 5.2e-8 -> 5.9e-8.
+// What bounds it: a slice takes about 1,300 cycles at 32 tokens (each warp's chain of split, fence
 // and drain) and 1,500 at 144, of which 12 products are 860 and their operands' reads from shared memory as many.
 #include <cooperative_groups.h>
 

@@ -745,6 +745,8 @@ int main(int argc, char** argv) {
         }
 
         // ---- the attention plan (parts/attention.py: AttentionMixer._plan) ------------------------------------------
+        // (The same but for requests of very different lengths: the engine cuts their keys together, AttentionMixer._even_pieces, and
+        // here every request is cut by itself, which leaves a step's attention to the longest one.)
         LlbAttentionPlan plan{};
         auto decode_splits = [&](int nspans) {
             const int bound = P * PAGE;

@@ -111,7 +111,11 @@ typedef struct {
     int max_pages, page_size;
     int num_plans;
     int first_layer, last_layer;   // run entries [first, last)
-    int fresh;                     // a row's last positions that this step may write (see llb_paged_decode_mma_biased)
+    // A row's last positions that this step may write (see llb_paged_decode_mma_biased; 0: not known).  Keys at the others are read before
+    // the kernel before has completed, and most kernels of a step give their early word before they wait.  So what ran before the
+    // step must have completed before any of them starts: the step's first launch waits first and signals then (the embedding
+    // does), or follows a copy in the stream.
+    int fresh;
 } LlbStepArgs;
 
 // Runs the run entries [first_layer, last_layer) over the step.  0, or a negative code with llb_last_error().

@@ -268,8 +268,10 @@ class ModelRunner:
         ctx.max_pages, ctx.page_size = P, ps
         ctx.decode_only = all(s.length == 1 for s in spans)
         ctx.rowwise = rowwise
-        # the last positions of a row that attends alone which this step itself may write: its own, or in a step described row by
-        # row those of its whole portion
+        # The last positions of a row that attends alone which this step itself may write: its own, or in a step described row by
+        # row those of its whole portion.  Decode attention reads the others early, while the kernels before it still run: that what
+        # earlier steps wrote is there by then rests on the step's first launch, the embedding, which waits for all before it (the copy
+        # of the metadata, the last step) before it lets the next kernel be set up.
         ctx.fresh_positions = self.ROWWISE_MAX_ROWS if rowwise else 1
         ctx.max_context = max_context
         ctx.dtype, ctx.device = self.model.dtype, self.device
