@@ -77,7 +77,15 @@ __device__ __forceinline__ uint64_t desc_kmajor64(uint32_t addr) {
 // at least 2^-125, within what bf16 holds without losing bits (split as it is, a float below 2^-109 loses the third part, below 2^-117
 // the second: 2.7e-4 off at 1e-37).  Powers of two leave all other roundings as they are.
 constexpr float UP = 16777216.0f, DOWN = 1.0f / (UP * UP);
-__device__ __forceinline__ float4 scaled_up(const float4& v) { return make_float4(v.x * UP, v.y * UP, v.z * UP, v.w * UP); }
+__device__ __forceinline__ float2 scaled_up2(float x, float y) {          // two products an instruction
+    float2 r;
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tmul.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}" : "=f"(r.x), "=f"(r.y) : "f"(x), "f"(y), "f"(UP));
+    return r;
+}
+__device__ __forceinline__ float4 scaled_up(const float4& v) {
+    const float2 a = scaled_up2(v.x, v.y), b = scaled_up2(v.z, v.w);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
 // Two floats as three pairs of bf16 that add up to them.
 __device__ __forceinline__ void split2(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
     h = pack_bf16(x, y);
