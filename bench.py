@@ -56,6 +56,12 @@ def peaks():
     return {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "source": "fallback"}
 
 
+def newest_graph(runner):
+    """The graph of the step that ran last: the only one that the step metadata on the device fits (the runner keeps the most recently
+    used graph last).  Replayed over another step's metadata, a graph would take its counts for page and token numbers."""
+    return next(reversed(runner._graphs.values()))[0]
+
+
 class ClockSampler:
     """Samples SM clocks and throttle reasons with nvidia-smi while the timed region runs."""
 
@@ -595,7 +601,7 @@ def main() -> int:
             r = core.runner
             extra = {"graph_replays": r.graph_replays, "graphs": len(r._graphs)}
             if r._graphs:      # the same captured step replayed back to back: device time without any host work
-                g = next(iter(r._graphs.values()))[0]
+                g = newest_graph(r)
                 torch.cuda.synchronize()
                 e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 e0.record()

@@ -176,3 +176,16 @@ def test_a_decoding_batch_and_a_step_row_by_row_share_no_graph():
     for rowwise in (False, False, True, True, False, True):
         step(rowwise)
     assert captured == [False, True, False, True]          # each from its second sight on, from a graph of its own kind
+
+
+def test_the_benchmark_replays_the_graph_of_the_last_step():
+    """A prompt's graph, captured before the decoding steps' one, may not be replayed over a decoding step's metadata."""
+    import importlib.util
+    import os
+    from types import SimpleNamespace
+    path = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "bench.py")
+    spec = importlib.util.spec_from_file_location("bench_under_test", path)
+    bench = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(bench)
+    graphs = {("prompt",): ("graph of the prompts", None, 1), ("decode",): ("graph of the decoding steps", None, 1)}
+    assert bench.newest_graph(SimpleNamespace(_graphs=graphs)) == "graph of the decoding steps"
